@@ -20,6 +20,7 @@
 #include "gsdr_testing.h"
 #include "job.h"
 #include "lcs_band.cuh"
+#include "lcs_seg.cuh"
 
 namespace gsdr {
 
@@ -406,11 +407,14 @@ int Job::init(const gsdr_reads* reads, const gsdr_opts* opts_in, cudaStream_t s,
         if (const char* bs = std::getenv("GSDR_BAND_SERIAL")) R_.band_serial = std::atoll(bs);
     R_.align_blocks = opts.align_blocks;
     R_.filter_blocks = opts.filter_blocks;
-    R_.group_max_w = opts.group_words > 0 ? std::min(opts.group_words, kGroupMaxWords)
-                                          : opts.group_words < 0 ? 0 : kGroupMaxWords;
+    R_.group_max_w = opts.group_words > 0   ? std::min(opts.group_words, kSegMaxWords)
+                     : opts.group_words < 0 ? 0
+                                            : kSegMaxWords;
     if (opts.group_words == 0)
         if (const char* gw = std::getenv("GSDR_GROUP_MAXW"))
-            R_.group_max_w = std::min(std::max(std::atoi(gw), 0), kGroupMaxWords);
+            R_.group_max_w = std::min(std::max(std::atoi(gw), 0), kSegMaxWords);
+    // a window holds at most the longest read's rows
+    R_.wide = (P.max_len + 31) / 32 > R_.group_max_w ? 1 : 0;
     refoff16_.swap(P.refoff16);
     pack_off_.swap(P.pack_off);
     kmer_off_.swap(P.kmer_off);
@@ -872,20 +876,23 @@ int Job::lcs_pairs(const int32_t* pat, const int32_t* txt, int n_pairs, int mapp
         seen[pat[k]] = 1;
         int c = align_class_host((gf[pat[k]] + 31) >> 5);
         if (mapping == 2) {
-            // the banded kernel where the band fits 32 words (as batched passes do)
+            // the lane-banded kernel where the band fits 8 words (its widest
+            // window), else the segment kernel
             const int T = gf[txt[k]], q = gf[pat[k]], cb = cut[pat[k]];
             // (the serial-work limit of the passes is not applied: tests reach
             // every window class with any length)
             if (T > 0 && cb > 0 && q >= cb && T >= cb) {
                 const int bw = band_words(T, q, cb);
-                if (bw <= 32) c = kSysClasses + (bw <= 4 ? 0 : bw <= 8 ? 1 : bw <= 16 ? 2 : 3);
+                const int sw = seg_words(T, q, cb, kSegSteps32);
+                if (bw <= kBandMaxWords) c = kSysClasses + (bw <= 4 ? 0 : 1);
+                else if (bw <= 32 && sw <= kSegMaxWords) c = seg_class(sw);
             }
         } else if (mapping == 3) {
-            // the group-banded kernel where the band fits 128 words
+            // the segment kernel where the window fits
             const int T = gf[txt[k]], q = gf[pat[k]], cb = cut[pat[k]];
             if (T > 0 && cb > 0 && q >= cb && T >= cb) {
-                const int bw = band_words(T, q, cb);
-                if (bw <= kGroupMaxWords) c = group_class(bw);
+                const int sw = seg_words(T, q, cb, kSegSteps32);
+                if (sw <= kSegMaxWords) c = seg_class(sw);
             }
         }
         cls[c].push_back(Pair{txt[k], pat[k]});
@@ -906,6 +913,7 @@ int Job::lcs_pairs(const int32_t* pat, const int32_t* txt, int n_pairs, int mapp
     JCUDA(cudaMemsetAsync(B_.cluster, 0xff, sizeof(int32_t) * n, stream));
     JCUDA(cudaMemsetAsync(B_.tidx, 0xff, sizeof(uint32_t) * n, stream));
     JCUDA(cudaEventRecord(ev_[2], stream));
+    R_.wide = 1;  // the queues above fill the systolic classes too
     launch_align_stage(R_, B_, mapping >= 1, greedy != 0, stream);
     JCUDA(cudaGetLastError());
     JCUDA(cudaEventRecord(ev_[3], stream));

@@ -24,16 +24,14 @@ constexpr int kMaxPatternWords = 2048;  // 8 warps x 32 lanes x 8 words: 65536 g
 constexpr int kSysClasses = 8;          // pattern length classes of the systolic alignment kernels
 constexpr int kLongClass = kSysClasses - 1;  // patterns above kMaxPatternWords: in chunks
 constexpr int64_t kMaxReadBases = 1ll << 24;  // longest read (raw bases) a job takes
-constexpr int kBandClasses = 4;         // window classes (4, 8, 16, 32 words) of the banded kernel
-constexpr int kGroupClasses = 5;        // group-banded classes: 2, 4, 8, 16, 32 lanes x 4 words
-constexpr int kGroupMaxWords = 128;     // widest window of the group-banded kernel
-constexpr int kAlignClasses = kSysClasses + kBandClasses + kGroupClasses;  // alignment queues
+constexpr int kBandClasses = 2;         // window classes (4, 8 words) of the lane-banded kernel
+constexpr int kSegClasses = 5;          // window classes of the segment kernel (seg_class)
+constexpr int kAlignClasses = kSysClasses + kBandClasses + kSegClasses;  // alignment queues
 constexpr int kSingleWorkSlot = kAlignClasses;  // work counter of the merged single-warp systolic classes
 
-// Group-banded class of a window of bw <= kGroupMaxWords words: the fewest
-// lanes (2, 4, .. 32) whose 4 words each hold it.
-__host__ __device__ __forceinline__ int group_class(int bw) {
-    const int g = bw <= 8 ? 0 : bw <= 16 ? 1 : bw <= 32 ? 2 : bw <= 64 ? 3 : 4;
+// Segment-kernel class of a window of at most kSegMaxWords words.
+__host__ __device__ __forceinline__ int seg_class(int words) {
+    const int g = words <= 32 ? 0 : words <= 64 ? 1 : words <= 128 ? 2 : words <= 256 ? 3 : 4;
     return kSysClasses + kBandClasses + g;
 }
 constexpr int kMaxBatch = 1024;         // tentative representatives per batched pass
@@ -106,9 +104,12 @@ struct DevReads {
     // word-filter kernels are launched with (0: as many as fit)
     int32_t align_blocks;
     int32_t filter_blocks;
-    // widest window (words) given to the group-banded kernel (kGroupMaxWords;
-    // 0: none, those pairs go to the systolic kernels)
+    // widest window (words) given to the segment kernel (kSegMaxWords; 0:
+    // none, those pairs go to the systolic kernels)
     int32_t group_max_w;
+    // 1: some pair may need a wider window than that, so passes also launch
+    // the systolic kernels
+    int32_t wide;
     // semantics (gsdr_opts::variant): 1 = the SYCL program's.  brk (variant 1
     // with filters, null otherwise): bit g of read i (word pack_off[i] + g/32)
     // is set when a non-ACGT byte stands right before gap-free base g in the

@@ -28,6 +28,8 @@
 
 namespace gsdr {
 
+constexpr int kBandMaxWords = 8;  // widest window of the lane-banded kernel
+
 // Words a lane's window needs for a pair: 32W must exceed the band's height
 // plus one block of 32 bases of slide plus word alignment.
 __host__ __device__ __forceinline__ int band_words(int T, int q, int c) {

@@ -10,9 +10,11 @@
 //                 composition bound first, then the candidate's (k-mer, count)
 //                 entries streamed with 16-byte loads against the
 //                 representative's table staged in shared memory.  Survivors
-//                 are queued for alignment in six length classes.
-//   k_align       kernel_align (func.cu:828-999): bit-parallel LCS on a group
-//                 of G warps with W pattern words per lane (lcs_sys.cuh).
+//                 are queued for alignment by the size of their window.
+//   k_seg         kernel_align (func.cu:828-999): bit-parallel LCS on the text
+//                 rows a long enough common subsequence can still use
+//                 (lcs_seg.cuh); k_align (lcs_sys.cuh) takes the pairs whose
+//                 window is wider than that kernel holds.
 //   k_compact     updataRemain (func.cu:689-699): drops clustered reads from
 //                 the remain list and finds the smallest unclustered index.
 //   k_advance     updateRepresentative (func.cu:677-687).
@@ -31,7 +33,8 @@
 //                 k-mer count bitmaps or per-k-mer tentative masks (the last
 //                 two with exact sums for the pairs their bounds leave open);
 //                 k_bprefilter in drop mode
-//   k_align       as above, accepted pairs listed instead of applied
+//   k_band, k_seg, k_align  as above, accepted pairs listed instead of applied
+//                 (k_band: a lane per pair, short reads with narrow bands)
 //   k_bsurvive    survival of the tentatives in order (one warp)
 //   k_bclaim      first surviving tentative per candidate (keyed atomicMax)
 //   k_bapply      writes the winners into cluster[]
@@ -44,7 +47,7 @@
 
 #include "gsdr_device.cuh"
 #include "lcs_band.cuh"
-#include "lcs_bandg.cuh"
+#include "lcs_seg.cuh"
 #include "lcs_sys.cuh"
 
 namespace gsdr {
@@ -56,10 +59,10 @@ constexpr int kFilterThreads = 256;
 constexpr int kAlignThreads = 256;  // 8 warps: 8/G groups of G warps
 constexpr int kAbsorbHigh = 64;     // absorbed reads per representative that shrink R
 constexpr int kFewPairs = 16384;    // queued pairs below which R grows 8x, not 2x
-// Largest band window (words) sent to the banded kernel: batched passes, plain
-// rounds.  A plain round waits for its slowest pair, and a lane works through
-// its pair alone, so the plain form keeps long pairs on the systolic kernels.
-constexpr int kBandMaxW = 32;
+// Widest band window (words) sent to the lane-banded kernel: batched passes,
+// plain rounds.  A plain round waits for its slowest pair, and a lane works
+// through its pair alone, so the plain form keeps to the segment kernel.
+constexpr int kBandMaxW = kBandMaxWords;
 constexpr int kPlainBandMaxW = 0;
 
 __device__ __forceinline__ bool prefilter_pass(const int4 a, const int4 b, int cut) {
@@ -83,23 +86,24 @@ __device__ __forceinline__ int align_class(int words) {
                          : words <= kMaxPatternWords ? 6 : kLongClass;
 }
 
-// Queue of a pair: a band class (kSysClasses + 0..3 for windows of 4, 8, 16,
-// 32 words) when its band fits a window of at most band_max_w words, else the
+// Queue of a pair: a band class (windows of 4 and 8 words) when its band fits
+// and its serial work (text bases x window words: a lane works through its
+// pair alone, and a longer one would hold up its pass) stays below
+// band_serial; else the segment kernel's class of its widest window; else the
 // systolic length class of its pattern.  Pairs decided without alignment
-// (trivial_decision) stay in the systolic classes, which decide them.
-// A lane works through its pair alone, so only pairs whose serial work (text
-// bases x window words) stays below R.band_serial go to the banded kernel; a
-// longer one would hold up its pass.
+// (trivial_decision) go to whichever of the last two the job launches.
 __device__ __forceinline__ int pair_class(int T, int q, int c, int band_max_w,
-                                          long long band_serial, int group_max_w) {
-    if (band_max_w > 0 && T > 0 && c > 0 && q >= c && T >= c) {
+                                          long long band_serial, int seg_max_w) {
+    if (T > 0 && c > 0 && q >= c && T >= c) {
         const int bw = band_words(T, q, c);
         if (bw <= band_max_w) {
-            const int w = bw <= 4 ? 4 : bw <= 8 ? 8 : bw <= 16 ? 16 : 32;
-            if ((long long)T * w <= band_serial)
-                return kSysClasses + (w == 4 ? 0 : w == 8 ? 1 : w == 16 ? 2 : 3);
+            const int w = bw <= 4 ? 4 : 8;
+            if ((long long)T * w <= band_serial) return kSysClasses + (w == 4 ? 0 : 1);
         }
-        if (bw <= group_max_w) return group_class(bw);
+        const int sw = seg_words(T, q, c, kSegSteps32);
+        if (sw <= seg_max_w) return seg_class(sw);
+    } else if (seg_max_w > 0) {
+        return seg_class(1);
     }
     return align_class((q + 31) >> 5);
 }
@@ -733,86 +737,117 @@ __global__ void __launch_bounds__(kAlignThreads) k_band(DevReads R, RoundState* 
     if (done) atomicAdd(&st->cells_done, (unsigned long long)done * (32ull * 32 * W));
 }
 
-// Banded alignment (lcs_bandg.cuh) of the pairs of group class cls: one pair
-// per group of G lanes (window of 4G words); a group whose pair is decided
-// takes the next one from the class queue at the next block of 32 text bases.
-template <int G, bool BATCH>
-__global__ void __launch_bounds__(kAlignThreads) k_bandg(DevReads R, RoundState* st, AlignArgs A,
-                                                         int cls) {
+// The pairs of the segment classes (lcs_seg.cuh) in one launch: each warp
+// takes pairs from the classes' queues, widest windows (longest work) first.
+// G lanes per pair: 8 for windows of up to 128 words (fewest instructions per
+// cell: a step costs 3 W + 3 integer ops for W words, and a segment G steps to
+// fill and drain), 16 and 32 for the wider ones.  A stage with fewer pairs
+// than half the grid's warps is bound by its longest pair instead, and every
+// pair gets a whole warp (fewest words per lane, the shortest step).
+//
+// Bound by the ALU pipe like the systolic kernels it replaces for these pairs;
+// it wins by the cells it does not step.  Alignment stage, systolic and
+// group-banded kernels before -> this one: 200k reads of 300-10,000 bp at
+// t = 0.95 40.6 -> 20.9 ms (3.36e12 -> 1.67e12 cells), 3k reads of 2-30 kbp at
+// t = 0.80 420 -> 199 ms, 30k reads of 150-5,000 bp at t = 0.90 60 -> 34 ms
+// (most of its passes hold few pairs: latency), 1k such reads at t = 0.95
+// 2.66 -> 1.44 ms.
+template <bool BATCH>
+__global__ void __launch_bounds__(kAlignThreads, 2) k_seg(DevReads R, RoundState* st,
+                                                          AlignArgs A) {
+    extern __shared__ __align__(16) uint32_t seg_sm[];  // kSegWarpWords per warp
     if (st->done) return;
     if (BATCH && (st->pair_overflow || st->n_tent == 0)) return;
-    const int np = min(st->n_pairs[cls], A.seg_cap);
-    if (np <= 0) return;
+    constexpr int c0 = kSysClasses + kBandClasses;
+    int total = 0;
+#pragma unroll
+    for (int c = 0; c < kSegClasses; c++) total += min(st->n_pairs[c0 + c], A.seg_cap);
+    if (total <= 0) return;
+    const bool alone = total <= (int)gridDim.x * (kAlignThreads / 64);
     const int pass = BATCH ? st->pass : 0;
     const int lane = threadIdx.x & 31;
-    const bool leader = (lane & (G - 1)) == 0;
     const unsigned lt_mask = (1u << lane) - 1u;
-    const Pair* list = A.pairs + (size_t)cls * A.seg_cap;
-    int* work = A.work + cls;
-    __shared__ uint4 btab[kAlignThreads / 32][4 * 32];  // match masks, per warp
-    __shared__ unsigned s_done[kAlignThreads / 32];  // blocks of 32 bases run by busy groups
-    if (lane == 0) s_done[threadIdx.x >> 5] = 0;
-    BandGroup<G> L;
-    L.init_lane(lane, btab[threadIdx.x >> 5]);
-    L.clear();
-    Pair p{-1, -1};
-    bool busy = false, more = true;
-    unsigned long long cells = 0;
+    uint32_t* peq = seg_sm + (threadIdx.x >> 5) * kSegWarpWords;
+    for (int i = lane; i < kSegMaxW * 32; i += 32) peq[kSegNoBase + i] = 0u;
+    unsigned long long cells = 0, done = 0;
     unsigned acc = 0;
-    while (true) {
-        // idle groups take the next pairs (one atomic per warp, by the leaders)
-        unsigned need = __ballot_sync(kFull, leader && !busy);
-        while (need && more) {
-            int base = 0;
-            if (lane == 0) base = atomicAdd(work, __popc(need));
-            base = __shfl_sync(kFull, base, 0);
-            const int mine = base + __popc(need & lt_mask);  // meaningful in idle leaders
-            const int i = __shfl_sync(kFull, mine, 0, G);
-            if (!busy && i < np) {
-                const Pair pp = list[i];
-                if (pp.rep >= 0) {  // not already accepted by k_greedy
-                    p = pp;
-                    L.start(R.packed + R.pack_off[pp.cand], R.len_gf[pp.cand],
-                            R.packed + R.pack_off[pp.rep], R.len_gf[pp.rep], R.cut_base[pp.cand]);
-                    busy = true;
+    for (int cls = kSegClasses - 1; cls >= 0; cls--) {
+        const int np = min(st->n_pairs[c0 + cls], A.seg_cap);
+        if (np <= 0) continue;
+        const int G = alone || cls == 4 ? 32 : cls == 3 ? 16 : 8;
+        const int S = G == 32 ? kSegSteps32 : kSegSteps8;
+        const int g = lane / G;
+        const bool leader = (lane & (G - 1)) == 0;
+        uint32_t* vb = peq + kSegPeqWords + g * (G * kSegMaxW + G);
+        uint16_t* codes = reinterpret_cast<uint16_t*>(peq + kSegPeqWords + kSegVWords);
+        __syncwarp();
+        for (int i = lane; i < kSegCodes; i += 32) codes[i] = kSegNoBase;
+        codes += g * (S + 2 * G);
+        const Pair* list = A.pairs + (size_t)(c0 + cls) * A.seg_cap;
+        int* work = A.work + c0 + cls;
+        SegPair P = {};
+        Pair p{-1, -1};
+        bool more = true;
+        while (true) {
+            // idle groups take the next pairs (one atomic per warp)
+            unsigned need = __ballot_sync(kFull, leader && !P.busy);
+            while (need && more) {
+                int base = 0;
+                if (lane == 0) base = atomicAdd(work, __popc(need));
+                base = __shfl_sync(kFull, base, 0);
+                const int mine = base + __popc(need & lt_mask);  // meaningful in idle leaders
+                const int i = __shfl_sync(kFull, mine, 0, G);
+                if (!P.busy && i < np) {
+                    p = list[i];
+                    if (p.rep >= 0) {  // not already accepted by k_greedy
+                        const int64_t po = R.pack_off[p.rep];
+                        P.T = R.len_gf[p.rep];
+                        P.q = R.len_gf[p.cand];
+                        P.c = R.cut_base[p.cand];
+                        const int trivial = trivial_decision(P.T, P.q, P.c);
+                        if (trivial < 0) {
+                            P.stride = (int)((R.pack_off[p.rep + 1] - po) >> 1);
+                            P.planes = R.bm + 2 * po;
+                            P.pq = R.packed + R.pack_off[p.cand];
+                            P.slope = (float)P.T / (float)P.q;
+                            P.busy = true;
+                            seg_start(P, S, false);
+                        } else if (leader) {
+                            cells += (unsigned long long)P.T * (unsigned long long)P.q;
+                            if (trivial) {
+                                acc++;
+                                on_accept<BATCH>(st, A, p, pass);
+                            }
+                        }
+                        if (trivial >= 0) P.T = P.q = P.c = 0;
+                    }
                 }
+                if (base + __popc(need) >= np) more = false;
+                need = __ballot_sync(kFull, leader && !P.busy);
             }
-            if (base + __popc(need) >= np) more = false;
-            need = __ballot_sync(kFull, leader && !busy);
-        }
-        if (!__any_sync(kFull, busy)) break;
-        uint32_t tw0 = 0, tw1 = 0;
-        if (busy) {
-            if (L.x0 < L.T) tw0 = __ldg(L.pt + (L.x0 >> 4));
-            if (L.x0 + 16 < L.T) tw1 = __ldg(L.pt + (L.x0 >> 4) + 1);
-        }
-        // a block inside every busy group's text takes the table path
-        if (__all_sync(kFull, !busy || L.x0 + 32 <= L.T)) L.block_full(tw0, tw1);
-        else L.block(tw0, tw1);
-        const int d = L.finish_block(busy);
-        {
-            const unsigned ran = __ballot_sync(kFull, busy && leader);
-            if (lane == 0) s_done[threadIdx.x >> 5] += __popc(ran);
-        }
-        if (busy && d >= 0) {
-            if (leader) {
-                cells += (unsigned long long)L.T * (unsigned long long)L.q;
-                if (d) {
-                    acc++;
-                    on_accept<BATCH>(st, A, p, pass);
+            if (!__any_sync(kFull, P.busy)) break;
+            const int wl =
+                __reduce_max_sync(kFull, P.busy ? (P.n_words + G - 1) / G : 1);
+            int steps = 0;
+            const int d = seg_dispatch(P, wl, peq, vb, codes, G, S, lane, steps);
+            if (P.busy && leader) done += (unsigned long long)steps * (32 * G * seg_tile(wl));
+            if (P.busy && d >= 0) {
+                if (leader) {
+                    cells += (unsigned long long)P.T * (unsigned long long)P.q;
+                    if (d) {
+                        acc++;
+                        on_accept<BATCH>(st, A, p, pass);
+                    }
                 }
+                P = SegPair{};
             }
-            busy = false;
-            L.clear();
         }
     }
     acc = (unsigned)warp_sum_i((int)acc);
     if (!BATCH && lane == 0 && acc) atomicAdd(&st->cnt_accepted, (unsigned long long)acc);
     if (cells) atomicAdd(&st->cells, cells);
-    // cells: 32 bases x the window's 4G words x 32 bits per block
-    if (lane == 0 && s_done[threadIdx.x >> 5])
-        atomicAdd(&st->cells_done,
-                  (unsigned long long)s_done[threadIdx.x >> 5] * (32ull * 32 * 4 * G));
+    // cells: steps x the window's words x 32 bits
+    if (done) atomicAdd(&st->cells_done, done);
 }
 
 // Pairs whose pattern has more rows than one group of 8 warps x 32 lanes x 8
@@ -2744,11 +2779,15 @@ void launch_align_t(const DevReads& R, RoundBuffers& B, int cls, cudaStream_t s)
     k_align<G, W, BATCH><<<shaped(grid, R.align_blocks), kAlignThreads, smem, s>>>(R, B.st, align_args(B), cls);
 }
 
-template <int G, bool BATCH>
-void launch_bandg_t(const DevReads& R, RoundBuffers& B, int cls, cudaStream_t s) {
+template <bool BATCH>
+void launch_seg_t(const DevReads& R, RoundBuffers& B, cudaStream_t s) {
+    constexpr int smem = (kAlignThreads / 32) * kSegWarpWords * 4;
     static int grid = 0;
-    if (!grid) grid = grid_for(k_bandg<G, BATCH>, kAlignThreads, 0, 8);
-    k_bandg<G, BATCH><<<shaped(grid, R.align_blocks), kAlignThreads, 0, s>>>(R, B.st, align_args(B), cls);
+    if (!grid) {
+        cudaFuncSetAttribute(k_seg<BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        grid = grid_for(k_seg<BATCH>, kAlignThreads, smem, 8);
+    }
+    k_seg<BATCH><<<shaped(grid, R.align_blocks), kAlignThreads, smem, s>>>(R, B.st, align_args(B));
 }
 
 template <int W, bool BATCH>
@@ -2773,26 +2812,20 @@ void launch_align_long_t(const DevReads& R, RoundBuffers& B, cudaStream_t s) {
 
 // Kernels launch_align_classes launches (after the greedy bound).
 template <bool BATCH>
-int align_launches(const RoundBuffers& B) {
-    return kSysClasses - 1 - (BATCH ? 3 : 0) + (B.long_carry ? 1 : 0) +
-           (BATCH || kPlainBandMaxW > 0 ? kBandClasses + kGroupClasses : 0);
+int align_launches(const DevReads& R, const RoundBuffers& B) {
+    return (BATCH ? kBandClasses : 0) + (R.group_max_w > 0 ? 1 : 0) +
+           (R.wide ? (BATCH ? 4 : 7) + (B.long_carry ? 1 : 0) : 0);
 }
 
 template <bool BATCH>
 void launch_align_classes(const DevReads& R, RoundBuffers& B, cudaStream_t s, bool greedy = true) {
     if (greedy) k_greedy<BATCH><<<num_sms() * 8, 256, 0, s>>>(R, B.st, align_args(B));
-    if (BATCH || kPlainBandMaxW > 0) {
+    if constexpr (BATCH) {
         launch_band_t<4, BATCH>(R, B, kSysClasses + 0, s);
         launch_band_t<8, BATCH>(R, B, kSysClasses + 1, s);
-        launch_band_t<16, BATCH>(R, B, kSysClasses + 2, s);
-        launch_band_t<32, BATCH>(R, B, kSysClasses + 3, s);
-        constexpr int g0 = kSysClasses + kBandClasses;
-        launch_bandg_t<32, BATCH>(R, B, g0 + 4, s);  // widest windows (longest work) first
-        launch_bandg_t<16, BATCH>(R, B, g0 + 3, s);
-        launch_bandg_t<8, BATCH>(R, B, g0 + 2, s);
-        launch_bandg_t<4, BATCH>(R, B, g0 + 1, s);
-        launch_bandg_t<2, BATCH>(R, B, g0 + 0, s);
     }
+    if (R.group_max_w > 0) launch_seg_t<BATCH>(R, B, s);
+    if (!R.wide) return;
     if constexpr (!BATCH) {
         launch_align_t<1, 1, BATCH>(R, B, 0, s);
         launch_align_t<1, 2, BATCH>(R, B, 1, s);
@@ -2864,7 +2897,7 @@ void launch_plain_round(const DevReads& R, RoundBuffers& B, int drop, int parity
     k_advance<<<1, 1, 0, s>>>(B.st, B.cluster, align_work_of(B.st));
     if (ev4) cudaEventRecordWithFlags(ev4[3], s, cudaEventRecordExternal);
     if (count)
-        *count += 4 + align_launches<false>(B) + (R.pig_q && !drop ? 1 : 0) +
+        *count += 4 + align_launches<false>(R, B) + (R.pig_q && !drop ? 1 : 0) +
                   (!drop && R.k >= kWideK ? 2 : 0);
 }
 
@@ -2901,7 +2934,7 @@ void launch_batch_pass(const DevReads& R, RoundBuffers& B, int drop, int parity,
                                B.amb_cap, drop);
     if (ev4) cudaEventRecordWithFlags(ev4[3], s, cudaEventRecordExternal);
     if (count)
-        *count += 8 + align_launches<true>(B) + (!drop ? 1 : 0) +
+        *count += 8 + align_launches<true>(R, B) + (!drop ? 1 : 0) +
                   (R.pig_q && !drop ? 1 : 0) + (B.amb && !drop ? 4 : 0);
     // (a word-filter form launches two kernels, six with the open-pair
     // queue: the bitmap form k_filter, k_bfilter_bits, the mask form k_bmask,

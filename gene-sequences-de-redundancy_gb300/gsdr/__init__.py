@@ -45,7 +45,7 @@ class Opts(C.Structure):
         ("word_filter", C.c_int32),
         ("variant", C.c_int32),  # 0 cuda-version semantics, 1 the SYCL program's
         ("band_serial", C.c_int32),  # lane-banded kernel's limit; 0 automatic, -1 none
-        ("group_words", C.c_int32),  # group-banded kernel's widest window; 0 automatic, -1 none
+        ("group_words", C.c_int32),  # segment kernel's widest window; 0 automatic, -1 none
         ("align_blocks", C.c_int32),  # block shape: CTAs per SM of the alignment kernels
         ("filter_blocks", C.c_int32),  # the same for the word-filter kernels
         ("graph_steps", C.c_int32),  # staging depth: rounds / passes per graph launch

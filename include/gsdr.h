@@ -65,9 +65,10 @@ typedef struct {
                              largest serial work (text bases x window words) of a pair it
                              takes; 0 = automatic (16,384), -1 = none (those pairs go to
                              the other alignment kernels); the result is the same */
-    int32_t group_words;  /* band tile of the group-banded alignment kernel: the widest
-                             band window (32-bit words, 1..128) it takes; 0 = automatic
-                             (128), -1 = none; the result is the same */
+    int32_t group_words;  /* window of the segment alignment kernel (a group of lanes per
+                             pair): the widest (32-bit words, 1..128) it takes; 0 =
+                             automatic (512), -1 = none (those pairs go to the systolic
+                             kernels); the result is the same */
     int32_t align_blocks; /* block shape: resident CTAs per SM the alignment kernels are
                              launched with (1..8, capped by what fits; 0 = automatic: as
                              many as fit); the result is the same */
