@@ -895,6 +895,13 @@ int Job::lcs_pairs(const int32_t* pat, const int32_t* txt, int n_pairs, int mapp
                 if (sw <= kSegMaxWords) c = seg_class(sw);
             }
         }
+        if (greedy) {
+            // a narrow run first where the passes would take one
+            const int T = gf[txt[k]], q = gf[pat[k]], cb = cut[pat[k]];
+            if (T > 0 && cb > 0 && q >= cb && T >= cb &&
+                seg_narrow(T, q, cb, seg_words(T, q, cb, kSegSteps32)))
+                c = kNarrowClass;
+        }
         cls[c].push_back(Pair{txt[k], pat[k]});
     }
     RoundState st{};
@@ -914,7 +921,7 @@ int Job::lcs_pairs(const int32_t* pat, const int32_t* txt, int n_pairs, int mapp
     JCUDA(cudaMemsetAsync(B_.tidx, 0xff, sizeof(uint32_t) * n, stream));
     JCUDA(cudaEventRecord(ev_[2], stream));
     R_.wide = 1;  // the queues above fill the systolic classes too
-    launch_align_stage(R_, B_, mapping >= 1, greedy != 0, stream);
+    launch_align_stage(R_, B_, mapping >= 1, stream);
     JCUDA(cudaGetLastError());
     JCUDA(cudaEventRecord(ev_[3], stream));
     JCUDA(cudaMemcpyAsync(h_state_, B_.st, sizeof(RoundState), cudaMemcpyDeviceToHost, stream));

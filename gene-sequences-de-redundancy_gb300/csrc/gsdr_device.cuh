@@ -26,7 +26,8 @@ constexpr int kLongClass = kSysClasses - 1;  // patterns above kMaxPatternWords:
 constexpr int64_t kMaxReadBases = 1ll << 24;  // longest read (raw bases) a job takes
 constexpr int kBandClasses = 2;         // window classes (4, 8 words) of the lane-banded kernel
 constexpr int kSegClasses = 5;          // window classes of the segment kernel (seg_class)
-constexpr int kAlignClasses = kSysClasses + kBandClasses + kSegClasses;  // alignment queues
+constexpr int kNarrowClass = kSysClasses + kBandClasses + kSegClasses;  // its narrow runs
+constexpr int kAlignClasses = kNarrowClass + 1;  // alignment queues
 constexpr int kSingleWorkSlot = kAlignClasses;  // work counter of the merged single-warp systolic classes
 
 // Segment-kernel class of a window of at most kSegMaxWords words.
@@ -240,9 +241,8 @@ void resume_rounds(const DevReads& R, RoundBuffers& B, int batched, int r_max, c
 void launch_plain_round(const DevReads& R, RoundBuffers& B, int drop, int parity,
                         cudaStream_t s, long long* count, cudaEvent_t* ev4);
 // Only the alignment stage over the queued pairs (st->n_pairs), with the
-// plain or the batched warp grouping, optionally after the greedy bound.
-void launch_align_stage(const DevReads& R, RoundBuffers& B, bool batched_mapping, bool greedy,
-                        cudaStream_t s);
+// plain or the batched warp grouping.
+void launch_align_stage(const DevReads& R, RoundBuffers& B, bool batched_mapping, cudaStream_t s);
 int align_class_host(int words);
 bool index_in_smem(int k, int r_max, int64_t cap, int smem_optin);
 // One batched pass (select, filter, align, resolve, compact, advance).

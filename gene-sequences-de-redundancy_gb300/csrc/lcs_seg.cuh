@@ -36,11 +36,10 @@
 // moves and W becomes the smallest that holds it.  A warp runs 32 / G pairs
 // side by side at the W of its widest.
 //
-// Narrow runs (seg_next with narrow set) also cut the window to a strip along
-// the line x = i * T / q.  That only drops cells, so L' is still a lower bound
-// of the LCS: an accept is final, anything else is run again without the
-// strip.  Used where the text is so much longer than the pattern that nearly
-// every pair is accepted.
+// Narrow runs also cut the window to a strip along a line x = slope * i.  That
+// only drops cells, so L' is still a lower bound of the LCS: an accept is
+// final, anything else is run again without the strip.  Used where the text is
+// so much longer than the pattern that nearly every pair is accepted.
 #pragma once
 #include <stdint.h>
 
@@ -67,8 +66,29 @@ __host__ __device__ __forceinline__ int seg_words(int T, int q, int c, int S) {
     return w < nw ? w : nw;
 }
 
-// Half the strip of a narrow run, in rows.
-constexpr int kSegStrip = 192;
+// Narrow runs: rows on either side of the line, and the slope beyond which
+// more text per pattern base is not needed (above the ratio of seg_narrow).
+constexpr int kSegStrip = 96;
+constexpr float kSegSlopeMore = 0.6f;
+
+// T / q at which unrelated bases start to reach c nearly always, read off the
+// decisions of the named workloads (1.55 at c/q = 0.80, 1.8 at 0.85, 2.2 at
+// 0.90, 2.7 at 0.95): close to linear in log2(q / (q - c)).
+__host__ __device__ __forceinline__ float seg_accept_ratio(int q, int c) {
+    return 0.23f + 0.57f * log2f((float)q / (float)(q - c));
+}
+__host__ __device__ __forceinline__ float seg_narrow_slope(int T, int q, int c) {
+    return fminf((float)T / (float)q, seg_accept_ratio(q, c) + kSegSlopeMore);
+}
+// Whether a narrow run comes first (`words`: the full window): from that ratio
+// on, and where the strip is at most half the full window's words.  A wrong
+// guess costs the strip's run and changes no decision.
+__host__ __device__ __forceinline__ bool seg_narrow(int T, int q, int c, int words) {
+    if (c >= q || T <= q) return false;
+    const float s = seg_narrow_slope(T, q, c);
+    if ((float)T < seg_accept_ratio(q, c) * (float)q) return false;
+    return words >= 2 * ((int)(kSegSteps8 * s + 2 * kSegStrip) / 32 + 2);
+}
 
 __device__ __forceinline__ int seg_vidx(int k) { return k + (k >> 4); }
 
@@ -95,7 +115,7 @@ struct SegPair {
     const uint32_t* planes;  // text bit planes: plane c at planes + c * stride
     const uint32_t* pq;      // pattern, packed
     int stride;
-    float slope;             // T / q
+    float slope;             // narrow runs: rows per step
     int q, T, c;
     int i0;                  // pattern bases applied
     int w_lo;                // first word of the window

@@ -184,7 +184,7 @@ extern "C" int gsdr_lcs_decide_noalloc(const uint32_t* d_packed, const int64_t* 
                                                            d_len_raw, n_seq, t);
     k_na_bucket<<<(n_pairs + threads - 1) / threads, threads, 0, s>>>(
         B.st, B.pairs, B.cluster, d_len_gf, d_pat, d_txt, n_pairs, n_seq);
-    launch_align_stage(R, B, false, false, s);
+    launch_align_stage(R, B, false, s);
     k_na_finish<<<(n_pairs + threads - 1) / threads, threads, 0, s>>>(B.cluster, d_pat, d_txt,
                                                                       n_pairs, n_seq, d_accept);
     e = cudaGetLastError();

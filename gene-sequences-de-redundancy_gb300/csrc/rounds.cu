@@ -101,6 +101,7 @@ __device__ __forceinline__ int pair_class(int T, int q, int c, int band_max_w,
             if ((long long)T * w <= band_serial) return kSysClasses + (w == 4 ? 0 : 1);
         }
         const int sw = seg_words(T, q, c, kSegSteps32);
+        if (seg_max_w > 0 && seg_narrow(T, q, c, sw)) return kNarrowClass;
         if (sw <= seg_max_w) return seg_class(sw);
     } else if (seg_max_w > 0) {
         return seg_class(1);
@@ -429,90 +430,6 @@ __device__ __forceinline__ void on_accept(RoundState* st, const AlignArgs& A, co
     }
 }
 
-// Greedy embedding in front of the alignment, one thread per queued pair:
-// walking the candidate base by base and taking, for each, the next
-// occurrence in the representative after the previous match builds a common
-// subsequence, so its length is a lower bound of the LCS.  When it reaches the
-// cutoff the pair is accepted without the bit-parallel alignment and removed
-// from its queue (rep = -1).  Any other pair is left to k_align.  Next
-// occurrences come from the representative's base bit-planes.
-template <bool BATCH>
-__global__ void __launch_bounds__(256) k_greedy(DevReads R, RoundState* st, AlignArgs A) {
-    if (st->done) return;
-    if (BATCH && (st->pair_overflow || st->n_tent == 0)) return;
-    const int pass = BATCH ? st->pass : 0;
-    int counts[kAlignClasses], total = 0;
-    for (int c = 0; c < kAlignClasses; c++) {
-        counts[c] = min(st->n_pairs[c], A.seg_cap);
-        total += counts[c];
-    }
-    unsigned acc = 0;
-    unsigned long long cells = 0;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < total; k += gridDim.x * blockDim.x) {
-        int cls = 0, kk = k;
-        while (kk >= counts[cls]) kk -= counts[cls++];
-        Pair* slot = const_cast<Pair*>(A.pairs) + (size_t)cls * A.seg_cap + kk;
-        const Pair p = *slot;
-        const int T = R.len_gf[p.rep], q = R.len_gf[p.cand], c = R.cut_base[p.cand];
-        if (T == 0 || c <= 0 || q < c || T < c) continue;  // trivial: k_align decides
-        // The walk is sequential, and the longest walk of a pass delays the
-        // whole pass: long candidates go to the (lane-parallel) alignment
-        // unless the representative is long enough for an embedding.
-        if (q > 4096 || (q > 2048 && T < 3 * c)) continue;
-        const int64_t po = R.pack_off[p.rep];
-        const int stride = (int)((R.pack_off[p.rep + 1] - po) >> 1);
-        const uint32_t* planes = R.bm + 2 * po;
-        const int nw = (T + 31) >> 5;
-        const uint32_t* pq = R.packed + R.pack_off[p.cand];
-        // The four plane words of the current 32-base text word stay in
-        // registers; a new word is loaded only when the match position
-        // crosses into it.  The walk also stops when reaching the cutoff has
-        // become impossible (too little text or candidate left) or, after
-        // 256 matches, when the text used per match so far projects well
-        // past the end: stopping only hands the pair to the alignment.
-        int pos = 0, g = 0, wcur = -1;
-        uint32_t p0 = 0, p1 = 0, p2 = 0, p3 = 0;
-        uint32_t qw = 0;
-        for (int i = 0; i < q; i++) {
-            if ((i & 15) == 0) qw = __ldg(pq + (i >> 4));
-            const uint32_t ch = (qw >> (30 - 2 * (i & 15))) & 3u;
-            uint32_t m = 0;
-            int w = pos >> 5;
-            while (w < nw) {
-                if (w != wcur) {
-                    p0 = __ldg(planes + w);
-                    p1 = __ldg(planes + stride + w);
-                    p2 = __ldg(planes + 2 * stride + w);
-                    p3 = __ldg(planes + 3 * stride + w);
-                    wcur = w;
-                }
-                m = ch == 0 ? p0 : ch == 1 ? p1 : ch == 2 ? p2 : p3;
-                if (32 * w < pos) m &= 0xffffffffu << (pos & 31);
-                if (m) break;
-                w++;
-            }
-            if (!m) break;
-            pos = 32 * w + __ffs(m);  // one past the match
-            if (++g >= c) break;
-            const int need = c - g;
-            if (g + (q - 1 - i) < c || T - pos < need) break;
-            if (g >= 256 && (long long)pos * need > 5ll * (T - pos) * g / 4) break;
-        }
-        if (g >= c) {
-            on_accept<BATCH>(st, A, p, pass);
-            slot->rep = -1;
-            acc++;
-            cells += (unsigned long long)T * (unsigned long long)q;
-        }
-    }
-    acc = warp_sum_i((int)acc);
-    if ((threadIdx.x & 31) == 0 && acc) {
-        if (!BATCH) atomicAdd(&st->cnt_accepted, (unsigned long long)acc);
-    }
-    // per-thread cell counts: one atomic per non-zero thread is rare enough
-    if (cells) atomicAdd(&st->cells, cells);
-}
-
 template <int G, int W, bool BATCH>
 __global__ void __launch_bounds__(kAlignThreads, 3) k_align(DevReads R, RoundState* st, AlignArgs A,
                                                          int cls) {
@@ -545,10 +462,6 @@ __global__ void __launch_bounds__(kAlignThreads, 3) k_align(DevReads R, RoundSta
         const int i = *(volatile int*)&S.idx;
         if (i >= np) break;
         const Pair p = list[i];
-        if (p.rep < 0) {  // already accepted by k_greedy
-            group_bar(bar_id, bar_n);
-            continue;
-        }
         const int T = R.len_gf[p.rep], q = R.len_gf[p.cand], c = R.cut_base[p.cand];
         const int trivial = trivial_decision(T, q, c);
         if (trivial < 0) {
@@ -616,7 +529,6 @@ __global__ void __launch_bounds__(kAlignThreads, 3) k_align_single(DevReads R, R
         while (i >= cnt[q4]) i -= cnt[q4++];
         const int cls = 3 - q4;
         const Pair p = A.pairs[(size_t)cls * A.seg_cap + i];
-        if (p.rep < 0) continue;  // already accepted by k_greedy
         const int T = R.len_gf[p.rep], q = R.len_gf[p.cand], c = R.cut_base[p.cand];
         int ok = trivial_decision(T, q, c);
         if (ok < 0) {
@@ -694,14 +606,11 @@ __global__ void __launch_bounds__(kAlignThreads) k_band(DevReads R, RoundState* 
             if (!busy) {
                 const int i = base + __popc(need & lt_mask);
                 if (i < np) {
-                    const Pair pp = list[i];
-                    if (pp.rep >= 0) {  // not already accepted by k_greedy
-                        p = pp;
-                        L.start(R.packed + R.pack_off[pp.cand], R.len_gf[pp.cand],
-                                R.packed + R.pack_off[pp.rep], R.len_gf[pp.rep],
-                                R.cut_base[pp.cand]);
-                        busy = true;
-                    }
+                    p = list[i];
+                    L.start(R.packed + R.pack_off[p.cand], R.len_gf[p.cand],
+                            R.packed + R.pack_off[p.rep], R.len_gf[p.rep],
+                            R.cut_base[p.cand]);
+                    busy = true;
                 }
             }
             if (base + __popc(need) >= np) more = false;
@@ -752,16 +661,26 @@ __global__ void __launch_bounds__(kAlignThreads) k_band(DevReads R, RoundState* 
 // t = 0.80 420 -> 199 ms, 30k reads of 150-5,000 bp at t = 0.90 60 -> 34 ms
 // (most of its passes hold few pairs: latency), 1k such reads at t = 0.95
 // 2.66 -> 1.44 ms.
-template <bool BATCH>
+//
+// NARROW: the pairs of the narrow class on their strip (8 lanes a pair, or a
+// warp), launched first; a pair it does not accept goes to the queue of its
+// full window behind it.  It took the place of a greedy walk with one thread
+// per pair, whose longest walk (up to 4,096 dependent steps) held up every
+// pass and which needed T/q > 3.6 at t = 0.95 where the strip accepts from 2.7
+// on: alignment stage 20.9 -> 18.2 ms (200k reads of 300-10,000 bp), 34 -> 16.7
+// ms (30k reads of 150-5,000 bp, t = 0.90, 92 passes), 29.6 -> 15.0 ms (100k
+// such reads, t = 0.95, 103 passes), 2.9 -> 1.05 ms (10k reads, 14 passes).
+template <bool BATCH, bool NARROW>
 __global__ void __launch_bounds__(kAlignThreads, 2) k_seg(DevReads R, RoundState* st,
                                                           AlignArgs A) {
     extern __shared__ __align__(16) uint32_t seg_sm[];  // kSegWarpWords per warp
     if (st->done) return;
     if (BATCH && (st->pair_overflow || st->n_tent == 0)) return;
-    constexpr int c0 = kSysClasses + kBandClasses;
+    constexpr int c0 = NARROW ? kNarrowClass : kSysClasses + kBandClasses;
+    constexpr int nc = NARROW ? 1 : kSegClasses;
     int total = 0;
 #pragma unroll
-    for (int c = 0; c < kSegClasses; c++) total += min(st->n_pairs[c0 + c], A.seg_cap);
+    for (int c = 0; c < nc; c++) total += min(st->n_pairs[c0 + c], A.seg_cap);
     if (total <= 0) return;
     const bool alone = total <= (int)gridDim.x * (kAlignThreads / 64);
     const int pass = BATCH ? st->pass : 0;
@@ -771,11 +690,11 @@ __global__ void __launch_bounds__(kAlignThreads, 2) k_seg(DevReads R, RoundState
     for (int i = lane; i < kSegMaxW * 32; i += 32) peq[kSegNoBase + i] = 0u;
     unsigned long long cells = 0, done = 0;
     unsigned acc = 0;
-    for (int cls = kSegClasses - 1; cls >= 0; cls--) {
+    for (int cls = nc - 1; cls >= 0; cls--) {
         const int np = min(st->n_pairs[c0 + cls], A.seg_cap);
         if (np <= 0) continue;
         const int G = alone || cls == 4 ? 32 : cls == 3 ? 16 : 8;
-        const int S = G == 32 ? kSegSteps32 : kSegSteps8;
+        const int S = G == 32 && !NARROW ? kSegSteps32 : kSegSteps8;
         const int g = lane / G;
         const bool leader = (lane & (G - 1)) == 0;
         uint32_t* vb = peq + kSegPeqWords + g * (G * kSegMaxW + G);
@@ -799,27 +718,25 @@ __global__ void __launch_bounds__(kAlignThreads, 2) k_seg(DevReads R, RoundState
                 const int i = __shfl_sync(kFull, mine, 0, G);
                 if (!P.busy && i < np) {
                     p = list[i];
-                    if (p.rep >= 0) {  // not already accepted by k_greedy
+                    const int T = R.len_gf[p.rep], q = R.len_gf[p.cand], c = R.cut_base[p.cand];
+                    const int trivial = trivial_decision(T, q, c);
+                    if (trivial < 0) {
                         const int64_t po = R.pack_off[p.rep];
-                        P.T = R.len_gf[p.rep];
-                        P.q = R.len_gf[p.cand];
-                        P.c = R.cut_base[p.cand];
-                        const int trivial = trivial_decision(P.T, P.q, P.c);
-                        if (trivial < 0) {
-                            P.stride = (int)((R.pack_off[p.rep + 1] - po) >> 1);
-                            P.planes = R.bm + 2 * po;
-                            P.pq = R.packed + R.pack_off[p.cand];
-                            P.slope = (float)P.T / (float)P.q;
-                            P.busy = true;
-                            seg_start(P, S, false);
-                        } else if (leader) {
-                            cells += (unsigned long long)P.T * (unsigned long long)P.q;
-                            if (trivial) {
-                                acc++;
-                                on_accept<BATCH>(st, A, p, pass);
-                            }
+                        P.T = T;
+                        P.q = q;
+                        P.c = c;
+                        P.stride = (int)((R.pack_off[p.rep + 1] - po) >> 1);
+                        P.planes = R.bm + 2 * po;
+                        P.pq = R.packed + R.pack_off[p.cand];
+                        P.slope = NARROW ? seg_narrow_slope(T, q, c) : 0.0f;
+                        P.busy = true;
+                        seg_start(P, S, NARROW);
+                    } else if (leader) {
+                        cells += (unsigned long long)T * (unsigned long long)q;
+                        if (trivial) {
+                            acc++;
+                            on_accept<BATCH>(st, A, p, pass);
                         }
-                        if (trivial >= 0) P.T = P.q = P.c = 0;
                     }
                 }
                 if (base + __popc(need) >= np) more = false;
@@ -830,17 +747,28 @@ __global__ void __launch_bounds__(kAlignThreads, 2) k_seg(DevReads R, RoundState
                 __reduce_max_sync(kFull, P.busy ? (P.n_words + G - 1) / G : 1);
             int steps = 0;
             const int d = seg_dispatch(P, wl, peq, vb, codes, G, S, lane, steps);
-            if (P.busy && leader) done += (unsigned long long)steps * (32 * G * seg_tile(wl));
-            if (P.busy && d >= 0) {
-                if (leader) {
+            if (!P.busy) continue;
+            if (leader) done += (unsigned long long)steps * (32 * G * seg_tile(wl));
+            if (d < 0) continue;
+            if (leader) {
+                if (NARROW && d == 0) {
+                    const int sw = seg_words(P.T, P.q, P.c, kSegSteps32);
+                    const int to = sw <= R.group_max_w ? seg_class(sw)
+                                                       : align_class((P.q + 31) >> 5);
+                    const int slot = atomicAdd(&st->n_pairs[to], 1);
+                    if (slot < A.seg_cap)
+                        const_cast<Pair*>(A.pairs)[(size_t)to * A.seg_cap + slot] = p;
+                    else
+                        st->pair_overflow = 1;
+                } else {
                     cells += (unsigned long long)P.T * (unsigned long long)P.q;
                     if (d) {
                         acc++;
                         on_accept<BATCH>(st, A, p, pass);
                     }
                 }
-                P = SegPair{};
             }
+            P = SegPair{};
         }
     }
     acc = (unsigned)warp_sum_i((int)acc);
@@ -880,7 +808,6 @@ __global__ void __launch_bounds__(kAlignThreads, 1) k_align_long(DevReads R, Rou
         __syncthreads();
         if (i >= np) break;
         const Pair p = A.pairs[(size_t)kLongClass * A.seg_cap + i];
-        if (p.rep < 0) continue;  // already accepted by k_greedy
         const int T = R.len_gf[p.rep], q = R.len_gf[p.cand], c = R.cut_base[p.cand];
         int ok = trivial_decision(T, q, c);
         if (ok < 0) {
@@ -2779,15 +2706,17 @@ void launch_align_t(const DevReads& R, RoundBuffers& B, int cls, cudaStream_t s)
     k_align<G, W, BATCH><<<shaped(grid, R.align_blocks), kAlignThreads, smem, s>>>(R, B.st, align_args(B), cls);
 }
 
-template <bool BATCH>
+template <bool BATCH, bool NARROW>
 void launch_seg_t(const DevReads& R, RoundBuffers& B, cudaStream_t s) {
     constexpr int smem = (kAlignThreads / 32) * kSegWarpWords * 4;
     static int grid = 0;
     if (!grid) {
-        cudaFuncSetAttribute(k_seg<BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        grid = grid_for(k_seg<BATCH>, kAlignThreads, smem, 8);
+        cudaFuncSetAttribute(k_seg<BATCH, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             smem);
+        grid = grid_for(k_seg<BATCH, NARROW>, kAlignThreads, smem, 8);
     }
-    k_seg<BATCH><<<shaped(grid, R.align_blocks), kAlignThreads, smem, s>>>(R, B.st, align_args(B));
+    k_seg<BATCH, NARROW><<<shaped(grid, R.align_blocks), kAlignThreads, smem, s>>>(R, B.st,
+                                                                             align_args(B));
 }
 
 template <int W, bool BATCH>
@@ -2810,21 +2739,23 @@ void launch_align_long_t(const DevReads& R, RoundBuffers& B, cudaStream_t s) {
                                                                B.long_carry, B.long_words);
 }
 
-// Kernels launch_align_classes launches (after the greedy bound).
+// Kernels launch_align_classes launches.
 template <bool BATCH>
 int align_launches(const DevReads& R, const RoundBuffers& B) {
-    return (BATCH ? kBandClasses : 0) + (R.group_max_w > 0 ? 1 : 0) +
+    return (BATCH ? kBandClasses : 0) + (R.group_max_w > 0 ? 2 : 0) +
            (R.wide ? (BATCH ? 4 : 7) + (B.long_carry ? 1 : 0) : 0);
 }
 
 template <bool BATCH>
-void launch_align_classes(const DevReads& R, RoundBuffers& B, cudaStream_t s, bool greedy = true) {
-    if (greedy) k_greedy<BATCH><<<num_sms() * 8, 256, 0, s>>>(R, B.st, align_args(B));
+void launch_align_classes(const DevReads& R, RoundBuffers& B, cudaStream_t s) {
     if constexpr (BATCH) {
         launch_band_t<4, BATCH>(R, B, kSysClasses + 0, s);
         launch_band_t<8, BATCH>(R, B, kSysClasses + 1, s);
     }
-    if (R.group_max_w > 0) launch_seg_t<BATCH>(R, B, s);
+    if (R.group_max_w > 0) {
+        launch_seg_t<BATCH, true>(R, B, s);
+        launch_seg_t<BATCH, false>(R, B, s);
+    }
     if (!R.wide) return;
     if constexpr (!BATCH) {
         launch_align_t<1, 1, BATCH>(R, B, 0, s);
@@ -2897,14 +2828,14 @@ void launch_plain_round(const DevReads& R, RoundBuffers& B, int drop, int parity
     k_advance<<<1, 1, 0, s>>>(B.st, B.cluster, align_work_of(B.st));
     if (ev4) cudaEventRecordWithFlags(ev4[3], s, cudaEventRecordExternal);
     if (count)
-        *count += 4 + align_launches<false>(R, B) + (R.pig_q && !drop ? 1 : 0) +
+        *count += 3 + align_launches<false>(R, B) + (R.pig_q && !drop ? 1 : 0) +
                   (!drop && R.k >= kWideK ? 2 : 0);
 }
 
-void launch_align_stage(const DevReads& R, RoundBuffers& B, bool batched_mapping, bool greedy,
+void launch_align_stage(const DevReads& R, RoundBuffers& B, bool batched_mapping,
                         cudaStream_t s) {
-    if (batched_mapping) launch_align_classes<true>(R, B, s, greedy);
-    else launch_align_classes<false>(R, B, s, greedy);
+    if (batched_mapping) launch_align_classes<true>(R, B, s);
+    else launch_align_classes<false>(R, B, s);
 }
 
 int align_class_host(int words) {
@@ -2934,7 +2865,7 @@ void launch_batch_pass(const DevReads& R, RoundBuffers& B, int drop, int parity,
                                B.amb_cap, drop);
     if (ev4) cudaEventRecordWithFlags(ev4[3], s, cudaEventRecordExternal);
     if (count)
-        *count += 8 + align_launches<true>(R, B) + (!drop ? 1 : 0) +
+        *count += 7 + align_launches<true>(R, B) + (!drop ? 1 : 0) +
                   (R.pig_q && !drop ? 1 : 0) + (B.amb && !drop ? 4 : 0);
     // (a word-filter form launches two kernels, six with the open-pair
     // queue: the bitmap form k_filter, k_bfilter_bits, the mask form k_bmask,

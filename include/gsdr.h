@@ -121,7 +121,7 @@ typedef struct {
     double cells_computed;    /* DP cells the alignment kernels actually stepped: per block
                                  of 32 text bases, the 32-bit pattern or band-window words
                                  a warp or lane held x 32 bits x 32 bases (early exits,
-                                 bands and the greedy bound make it smaller than cells) */
+                                 windows and narrow runs make it smaller than cells) */
     int32_t tuned;            /* 1: an automatic job (batch 0) took its knobs from the
                                  tuning cache written by gsdr_autotune */
 } gsdr_stats;

@@ -22,7 +22,8 @@ extern "C" {
  * form's, 2 = the batched form's with the banded one-pair-per-lane kernel for
  * every pair whose band fits its 8 words and the segment kernel up to 32,
  * 3 = the batched form's with the segment kernel (one pair per 8..32 lanes)
- * for every pair whose window fits its 512 words; greedy: 1 = try the greedy-embedding lower bound first.
+ * for every pair whose window fits its 512 words; greedy: 1 = a
+ * narrow run (a lower bound of the LCS) first where a pass would take one.
  * accept[k] receives 0/1; *ms the device time of the alignment stage. */
 int gsdr_lcs_decide(const char* bytes, int64_t n_bytes, const int64_t* off, const int32_t* len,
                     int32_t n_seq, const int32_t* pat, const int32_t* txt, int32_t n_pairs,
