@@ -167,13 +167,11 @@ int make_plan(const gsdr_reads* reads, const gsdr_opts& o, Plan& P, PlanPreset* 
         if (masks) index = false;
         P.bits = bits;
         P.masks = masks;
-        // automatic R with the table and bitmap forms: the largest R for
-        // k <= 6 (the table form measured 22.6 us per representative at
-        // R_max 1024 against 25.5 at 256 on the 200k-read workload), 256 for
-        // k = 7, whose tables and bitmaps are four times larger (200k reads of
-        // 150-5,000 bp at t = 0.90: bitmaps 1.19 s at 256 against 1.72 s at
-        // 1024, tables 3.7 against 4.4 s)
-        if (o.batch == 0 && !index) P.r_max = k >= 7 && !masks ? 256 : kMaxBatch;
+        // automatic R: the largest, except for the table form at k = 7, whose
+        // tables hold only 4 tentatives per CTA (200k reads of 150-5,000 bp at
+        // t = 0.90: 3.7 s at 256 against 4.4 s at 1024; the bitmap form, on
+        // the tensor cores, reads a candidate once per 240 tentatives)
+        if (o.batch == 0 && !index) P.r_max = k >= 7 && !masks && !bits ? 256 : kMaxBatch;
         if (index) {
             // a pass indexes at most R_max tentatives: for length-sorted reads
             // those hold at most the first R_max reads' entries

@@ -49,6 +49,7 @@
 #include "lcs_band.cuh"
 #include "lcs_seg.cuh"
 #include "lcs_sys.cuh"
+#include "tc05.cuh"
 
 namespace gsdr {
 
@@ -1184,7 +1185,7 @@ __global__ void __launch_bounds__(kFilterThreads) k_bprefilter(DevReads R, Round
     }
 }
 
-// ---- word filter by two-level k-mer count bitmaps (k <= kMaxBitsK) --------
+// ---- word filter by two-level k-mer count bitmaps (k <= kMaxBits2K) -------
 //
 // Per read two 4^k-bit bitmaps: level 1 holds the k-mers with a stored count
 // of at least one, level 2 those with at least two; E3 is the excess above
@@ -1192,172 +1193,310 @@ __global__ void __launch_bounds__(kFilterThreads) k_bprefilter(DevReads R, Round
 // (func.cu:803-826) is S = sum over k-mers of min(c_t, c_q), and since
 // min(c_t, c_q) = [both >= 1] + [both >= 2] + max(min(c_t, c_q) - 2, 0),
 //     lo = D1 + D2 <= S <= lo + min(E3_t, E3_q),
-// with D1, D2 the popcounts of the two levels' intersections.  k_bfilter_bits
-// forms lo with 2 x 4^k / 32 AND + POPC per pair (lane = tentative, no table
-// lookups, no bank conflicts) and decides every pair outside the gap; the few
-// pairs inside it go to k_bexact_t, which forms S itself.  The second level
-// keeps the gap small where one level leaves it wide (reads holding a large
-// share of the k-mer space, whose counts are mostly 1 or 2).
+// with D1, D2 the popcounts of the two levels' intersections.  The second
+// level keeps the gap small where one level leaves it wide (reads holding a
+// large share of the k-mer space, whose counts are mostly 1 or 2).  lo decides
+// every pair outside the gap; the few pairs inside it go to k_bexact_t, which
+// forms S itself.
+//
+// lo is an entry of a matrix product: the candidates' bitmaps (both levels end
+// to end, 0/1) times the tentatives' transposed.  k_bfilter_bits forms it on
+// the tensor cores: tiles of 128 candidates x up to 240 tentatives, the
+// bitmaps spread to 4-bit values on their way into shared memory (any fixed
+// order of a read's k-mers gives the same sum, so the spread is three shifts
+// and four masks per 32 k-mers), accumulators in tensor memory.
+//
+// A CTA per SM: one warp issues the MMAs, 23 warps load and spread the
+// bitmaps into a ring of four stages (256 k-mers of every row), and four warps
+// read the finished tile's sums, apply the composition bound and queue the
+// pairs while the next tile is summed in the other accumulator.  A producer
+// lane loads 16 bytes of a row, eight lanes 128 contiguous bytes, and word w of
+// its 16 bytes goes to the w-th of four stages: full lines from L2 and whole
+// rows of shared memory per store.
+//
+// 84,800 candidates x 1,024 tentatives, k = 6: 0.42 ms (2.1e11 pairs/s), ALU
+// pipe 71% (the spread and the composition bound), shared-memory pipe 64%,
+// tensor pipe 35%; the AND + POPC kernel before it took about 3 ms.  Filter stage: 149 -> 27 ms (100k reads of 150-5,000 bp, t = 0.95),
+// 42 -> 8.1 ms (30k, t = 0.90, k = 7, with R_max 1024 instead of 256, which the
+// lanes' form could not stage), 2.36 -> 0.91 ms (10k reads of 200-1,000 bp).
+// On the way there: eight producer loads of 32 bytes of a row each (shared
+// pipe 71%, 0.49 ms); 12 producers (0.53 ms: every warp takes part in every
+// stage, so a stage lasts as long as one warp's share of it); the MMAs issued
+// by a producer (0.73 ms); branches per column in the epilogue (0.63 ms).
+constexpr int kBitsProducers = 23;  // 4 rows per 8 lanes, 28 warps: 72 registers each
+constexpr int kBitsEpilogue = 4;
+constexpr int kBitsThreads = 32 * (1 + kBitsEpilogue + kBitsProducers);
+constexpr int kBitsStages = 4;
+constexpr int kBitsStageBytes = (128 + kTcMaxN) * kTcRowBytes;
+constexpr int kTentPad = kMaxBatch + 16;  // a tile's columns are read sixteen at a time
+constexpr int kBitsSmem = 1024 + kBitsStages * kBitsStageBytes + kTentPad * (16 + 8);
+static_assert(128 % 8 == 0 && kTcMaxN % 16 == 0, "whole groups of eight rows");
+constexpr int kBitsRows = (128 + kTcMaxN + 4 * kBitsProducers - 1) / (4 * kBitsProducers);
+
+template <int K>
+__global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
+    DevReads R, RoundState* st, const int32_t* __restrict__ remain,
+    const int32_t* __restrict__ tent, Pair* pairs, int seg_cap, Pair* amb, int amb_cap) {
+    constexpr int NQ = (1 << (2 * K)) / 128;        // 16-byte words of one bitmap
+    constexpr int GL = NQ >= 8 ? NQ / 8 : 1;        // groups of four stages per level
+    constexpr int CH = 4 * (K == 4 ? 1 : 2 * GL);   // stages per tile (k = 4: half of them zeros)
+    extern __shared__ __align__(1024) uint8_t bsm_raw[];
+    __shared__ uint64_t full[kBitsStages], empty[kBitsStages], tfull[2], tempty[2], drain;
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_quit;
+    if (st->done) return;
+    const int nt = st->n_tent;
+    if (nt <= 1) return;  // a single tentative's pass runs k_filter instead
+    const int n = st->n_remain;
+    const int tiles_n = (nt + kTcMaxN - 1) / kTcMaxN;
+    const int N = (((nt + tiles_n - 1) / tiles_n) + 15) & ~15;  // tentatives per tile
+    const int tiles = ((n + 127) >> 7) * tiles_n;
+    if ((int)blockIdx.x >= tiles) return;
+    uint8_t* stage0 = reinterpret_cast<uint8_t*>(
+        (reinterpret_cast<uintptr_t>(bsm_raw) + 1023) & ~(uintptr_t)1023);
+    int4* tcomp = reinterpret_cast<int4*>(stage0 + kBitsStages * kBitsStageBytes);
+    int2* tte = reinterpret_cast<int2*>(tcomp + kTentPad);  // tentative and its excess
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kBitsStages; i++) {
+            mbar_init(&full[i], kBitsProducers);
+            mbar_init(&empty[i], 1);
+        }
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&tfull[i], 1);
+            mbar_init(&tempty[i], kBitsEpilogue);
+        }
+        mbar_init(&drain, 1);
+        s_quit = 0;
+        mbar_init_fence();
+    }
+    if (warp == 0) tmem_alloc_all(&s_tmem);
+    for (int t = threadIdx.x; t < nt; t += blockDim.x) {
+        const int rep = tent[t];
+        tcomp[t] = R.comp[rep];
+        tte[t] = make_int2(rep, R.kextra3[rep]);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = s_tmem;
+    if (warp >= 1 && warp <= 4) tc_fill_scales(tmem, warp);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const int limit = max(c_spin_limit, 1);
+    bool ok = true;  // this warp's waits all ended
+    if (warp == 0) {
+        if (lane == 0) {
+            const uint32_t idesc = tc_idesc_fp4(N);
+            int s = 0, it = 0;
+            uint32_t ph = 0;
+            for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x, it++) {
+                const int buf = it & 1;
+                // (the first use of each accumulator passes at once)
+                ok = mbar_wait(&tempty[buf], ((it >> 1) & 1) ^ 1, limit, &s_quit);
+                tc_fence_after();
+                for (int c = 0; ok && c < CH; c++) {
+                    ok = mbar_wait(&full[s], ph, limit, &s_quit);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t a = smem_u32(stage0 + s * kBitsStageBytes);
+                    tc_mma_stage(tmem + buf * kTcMaxN, tmem, a, a + 128 * kTcRowBytes, idesc,
+                                 c == 0);
+                    tc_commit(&empty[s]);
+                    if (++s == kBitsStages) s = 0, ph ^= 1;
+                }
+                if (ok) tc_commit(&tfull[buf]);
+            }
+        }
+    } else if (warp <= kBitsEpilogue) {
+        const int row = (warp & 3) * 32 + lane;
+        unsigned n_wf = 0, n_al = 0;
+        unsigned long long n_pf = 0, bytes = 0;
+        int it = 0;
+        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, it++) {
+            const int m = tile / tiles_n, t0 = (tile - m * tiles_n) * N;
+            const int t1 = min(nt, t0 + N);
+            const int idx = m * 128 + row;
+            int q = -1, cw = 0, exq = 0, cbq = 0;
+            int4 cq = make_int4(0, 0, 0, 0);
+            if (idx < n) {
+                q = remain[idx];
+                cw = R.cut_word[q];
+                exq = R.kextra3[q];
+                cq = R.comp[q];
+                cbq = R.cut_base[q] - R.strict;
+                if (t0 == 0) bytes += kCandFixedBytes + 2ull * 16 * NQ;  // once per launch
+            }
+            const int buf = it & 1;
+            ok = mbar_wait(&tfull[buf], (it >> 1) & 1, limit, &s_quit);
+            if (!__all_sync(kFull, ok)) {
+                ok = false;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t addr = tmem + ((uint32_t)(warp & 3) << 21) + buf * kTcMaxN;
+            for (int c0 = t0; c0 < t1; c0 += 16) {
+                float v[16];
+                tc_load16(v, addr + (c0 - t0));
+                // sixteen independent chains with no branch: which tentatives
+                // come before q and pass kernel_preFilter (func.cu:738-754),
+                // and which of those the bound does not reject
+                const int ncol = t1 - c0;
+                uint32_t before = 0, pre = 0, hit = 0;
+#pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    const int t = c0 + j;  // (entries past nt: any values, masked below)
+                    const int2 te = tte[t];
+                    before |= te.x < q ? 1u << j : 0u;
+                    pre |= prefilter_pass(tcomp[t], cq, cbq) ? 1u << j : 0u;
+                    hit |= (int)(4.0f * v[j]) + min(te.y, exq) >= cw ? 1u << j : 0u;
+                }
+                before &= ncol >= 16 ? 0xffffu : (1u << ncol) - 1u;
+                pre &= before;
+                hit &= pre;
+                n_pf += __popc(before);
+                n_wf += __popc(pre);
+                while (hit) {
+                    const int j = __ffs(hit) - 1;
+                    hit &= hit - 1;
+                    float vj = v[0];
+#pragma unroll
+                    for (int i = 1; i < 16; i++) vj = j == i ? v[i] : vj;
+                    const int rep = tte[c0 + j].x;
+                    if ((int)(4.0f * vj) >= cw) {
+                        push_pair(st, pairs, seg_cap, R, rep, q, kBandMaxW);
+                        n_al++;
+                    } else {
+                        const int slot = atomicAdd(&st->n_amb, 1);
+                        if (slot < amb_cap) amb[slot] = Pair{rep, q};
+                        else st->pair_overflow = 1;
+                    }
+                }
+                __syncwarp();
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tempty[buf]);
+        }
+        n_wf = (unsigned)warp_sum_i((int)n_wf);
+        n_al = (unsigned)warp_sum_i((int)n_al);
+        n_pf = warp_sum_ull(n_pf);
+        bytes = warp_sum_ull(bytes);
+        if (lane == 0) {
+            if (n_pf) atomicAdd(&st->cnt_prefilter, n_pf);
+            if (n_wf) atomicAdd(&st->cnt_word, (unsigned long long)n_wf);
+            if (n_al) atomicAdd(&st->cnt_aligned, (unsigned long long)n_al);
+            if (bytes) atomicAdd(&st->filter_bytes, bytes);
+        }
+    } else {
+        // producers: lane piece p = lane % 8 (16 bytes of 128) of rows r0 +
+        // 92 j (rows 0..127: the tile's candidates, then its tentatives)
+        const int tid = threadIdx.x - 32 * (1 + kBitsEpilogue);
+        const uint4* kb1 = reinterpret_cast<const uint4*>(R.kbits);
+        const uint4* kb2 = reinterpret_cast<const uint4*>(R.kbits2);
+        const int p = tid & 7, r0 = tid >> 3;
+        constexpr int RS = 4 * kBitsProducers;  // rows per sweep
+        static_assert(RS % 8 == 4 && RS * kBitsRows == 128 + kTcMaxN, "row layout");
+        const int off0 = r0 * kTcRowBytes + ((p ^ (r0 & 7)) << 4);
+        const int odd = ((p ^ ((r0 + 4) & 7)) << 4) - ((p ^ (r0 & 7)) << 4);
+        const int rows = (128 + N - r0 + RS - 1) / RS;
+        // (rows past the last candidate or tentative hold read 0: their sums
+        // are not looked at)
+        auto read_of = [&](int tile, int r) -> int {
+            if (tile >= tiles) return 0;
+            const int m = tile / tiles_n, t0 = (tile - m * tiles_n) * N;
+            if (r < 128) return m * 128 + r < n ? remain[m * 128 + r] : 0;
+            r -= 128;
+            return r < N && t0 + r < nt ? tent[t0 + r] : 0;
+        };
+        int ft = blockIdx.x, fg = 0;  // the next group to load
+        int cur[kBitsRows], nxt[kBitsRows];
+#pragma unroll
+        for (int j = 0; j < kBitsRows; j++) {
+            cur[j] = read_of(ft, r0 + RS * j);
+            nxt[j] = read_of(ft + gridDim.x, r0 + RS * j);
+        }
+        auto load = [&](uint4 (&v)[kBitsRows]) {
+#pragma unroll
+            for (int j = 0; j < kBitsRows; j++) {
+                if constexpr (K == 4) {
+                    v[j] = make_uint4(0u, 0u, 0u, 0u);
+                    if (p < 4) v[j] = __ldg((p < 2 ? kb1 : kb2) + (size_t)cur[j] * NQ + (p & 1));
+                } else {
+                    v[j] = __ldg((fg < GL ? kb1 : kb2) + (size_t)cur[j] * NQ +
+                                 8 * (fg & (GL - 1)) + p);
+                }
+            }
+            if (++fg == CH / 4) {
+                fg = 0;
+                ft += gridDim.x;
+#pragma unroll
+                for (int j = 0; j < kBitsRows; j++) {
+                    cur[j] = nxt[j];
+                    nxt[j] = read_of(ft + gridDim.x, r0 + RS * j);
+                }
+            }
+        };
+        int s = 0;
+        uint32_t ph = 1;  // the first round of stages is free
+        // the four stages of one group
+        auto store = [&](const uint4 (&v)[kBitsRows]) {
+#pragma unroll
+            for (int w = 0; w < 4; w++) {
+                ok = __all_sync(kFull, mbar_wait(&empty[s], ph, limit, &s_quit));
+                if (!ok) return;
+                uint8_t* base = stage0 + s * kBitsStageBytes + off0;
+#pragma unroll
+                for (int j = 0; j < kBitsRows; j++) {
+                    // (row r0 + RS j: RS is 4 mod 8, so the swizzle alternates)
+                    if (j < rows)
+                        *reinterpret_cast<uint4*>(base + j * RS * kTcRowBytes +
+                                                  (j & 1 ? odd : 0)) =
+                            tc_spread(w == 0 ? v[j].x : w == 1 ? v[j].y : w == 2 ? v[j].z : v[j].w);
+                }
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[s]);
+                if (++s == kBitsStages) s = 0, ph ^= 1;
+            }
+        };
+        const int mine =
+            (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * (CH / 4);
+        uint4 va[kBitsRows], vb[kBitsRows];
+        load(va);
+        for (int i = 0; ok && i < mine; i += 2) {
+            load(vb);
+            store(va);
+            if (!ok || i + 1 >= mine) break;
+            load(va);
+            store(vb);
+        }
+    }
+    if (!ok) {
+        // a wait gave up: the others stop at their next poll
+        s_quit = 1;
+        st->error = 1;
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        if (s_quit && lane == 0) {
+            // the MMAs in flight, before the accumulators are given back
+            const int none = 0;
+            tc_commit(&drain);
+            mbar_wait(&drain, 0, kSpinLimit, &none);
+        }
+        __syncwarp();
+        tmem_free_all(tmem);
+    }
+}
 
 // Carry-save adder: a + b + c = s + 2 * carry, bit by bit (two LOP3s).
 __device__ __forceinline__ void csa(uint32_t& s, uint32_t& carry, uint32_t a, uint32_t b,
                                     uint32_t c) {
     s = a ^ b ^ c;
     carry = (a & b) | (c & (a ^ b));
-}
-
-// The summed population count of eight words with four POPCs (the POPC pipe
-// bounds the bitmap filter): a tree of carry-save adders (Harley and Seal)
-// reduces them to words of weight 1, 1, 2 and 4 first.
-__device__ __forceinline__ int popc8(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3,
-                                     uint32_t w4, uint32_t w5, uint32_t w6, uint32_t w7) {
-    uint32_t s1, c1, s2, c2, s3, c3, t2, f4;
-    csa(s1, c1, w0, w1, w2);
-    csa(s2, c2, w3, w4, w5);
-    csa(s3, c3, s1, s2, w6);
-    csa(t2, f4, c1, c2, c3);
-    return __popc(s3) + __popc(w7) + 2 * __popc(t2) + 4 * __popc(f4);
-}
-
-// Shared memory of k_bfilter_bits: the group's two bitmap levels as
-// [level][quad][tentative] (lane t reads consecutive 16 bytes: conflict-free),
-// each warp's candidate bitmaps, and the group's tentatives, compositions and
-// excesses.  k <= 6: 128 tentatives per CTA of 32 warps (163 KB); k = 7, whose
-// bitmaps are four times larger: 32 tentatives per CTA of 16 warps (193 KB).
-template <int K>
-struct BitsSmem {
-    static constexpr int NQ = (1 << (2 * K)) / 128;  // 16-byte words of one bitmap
-    static constexpr int RG = K <= 6 ? 128 : 32;     // tentatives staged per CTA
-    static constexpr int THREADS = K <= 6 ? 1024 : 512;
-    static constexpr int WARPS = THREADS / 32;
-    static constexpr size_t tb_quads = 2 * (size_t)NQ * RG;
-    static constexpr size_t cb_quads = (size_t)WARPS * 2 * NQ;
-    static constexpr size_t bytes = 16 * (tb_quads + cb_quads) + RG * (16 + 4 + 4);
-};
-
-template <int K>
-__global__ void __launch_bounds__(BitsSmem<K>::THREADS, 1) k_bfilter_bits(DevReads R, RoundState* st,
-                                                                  const int32_t* __restrict__ remain,
-                                                                  const int32_t* __restrict__ tent,
-                                                                  Pair* pairs, int seg_cap, Pair* amb,
-                                                                  int amb_cap) {
-    using L = BitsSmem<K>;
-    constexpr int NQ = L::NQ;
-    constexpr int RG = L::RG;
-    constexpr int WARPS = L::WARPS;
-    extern __shared__ __align__(16) uint4 bsm[];
-    uint4* tb = bsm;                                  // tb[(level * NQ + w) * RG + t]
-    uint4* cball = bsm + L::tb_quads;                 // cb[(warp * 2 + level) * NQ + w]
-    int4* tcomp = reinterpret_cast<int4*>(cball + L::cb_quads);
-    int* ttent = reinterpret_cast<int*>(tcomp + RG);
-    int* textra = ttent + RG;
-    if (st->done) return;
-    const int nt = st->n_tent;
-    if (nt <= 1) return;  // a single tentative's pass runs k_filter instead
-    const int n = st->n_remain;
-    const int ngroups = (nt + RG - 1) / RG;
-    const int parts = max(1, (int)gridDim.x / ngroups);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint4* cb = cball + warp * 2 * NQ;
-    const uint4* kb1 = reinterpret_cast<const uint4*>(R.kbits);
-    const uint4* kb2 = reinterpret_cast<const uint4*>(R.kbits2);
-    unsigned n_pf = 0, n_wf = 0, n_al = 0;
-    unsigned long long bytes = 0;
-    int cur_group = -1;
-    for (int item = blockIdx.x; item < ngroups * parts; item += gridDim.x) {
-        const int g = item % ngroups, part = item / ngroups;
-        const int t0 = g * RG;
-        const int ng = min(RG, nt - t0);
-        if (g != cur_group) {
-            __syncthreads();
-            if (threadIdx.x < RG) {
-                const bool in = (int)threadIdx.x < ng;
-                const int rep = in ? tent[t0 + threadIdx.x] : 0;
-                ttent[threadIdx.x] = in ? rep : 0x7fffffff;
-                tcomp[threadIdx.x] = in ? R.comp[rep] : make_int4(0, 0, 0, 0);
-                textra[threadIdx.x] = in ? R.kextra3[rep] : 0;
-            }
-            for (int i = threadIdx.x; i < 2 * NQ * RG; i += L::THREADS) {
-                const int t = i % RG, lw = i / RG, lv = lw / NQ, w = lw % NQ;
-                uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                if (t < ng) v = __ldg((lv ? kb2 : kb1) + (size_t)tent[t0 + t] * NQ + w);
-                tb[i] = v;
-            }
-            __syncthreads();
-            cur_group = g;
-        }
-        const int per = (n + parts - 1) / parts;
-        const int lo = part * per, hi = min(n, lo + per);
-        for (int idx = lo + warp; idx < hi; idx += WARPS) {
-            const int q = remain[idx];
-            if (g == 0) bytes += kCandFixedBytes + 2ull * 16 * NQ;  // once per launch
-            const int4 cq = R.comp[q];
-            const int cbq = R.cut_base[q] - R.strict;  // the prefilter's cutoff
-            unsigned ok_bits[RG / 32];
-            bool any = false;
-#pragma unroll
-            for (int h = 0; h < RG / 32; h++) {
-                const int t = 32 * h + lane;
-                const bool before = t < ng && ttent[t] < q;
-                n_pf += before;
-                // kernel_preFilter (func.cu:738-754) first
-                const bool ok = before && prefilter_pass(tcomp[t], cq, cbq);
-                ok_bits[h] = __ballot_sync(kFull, ok);
-                any |= ok_bits[h] != 0;
-            }
-            if (!any) continue;
-            for (int i = lane; i < 2 * NQ; i += 32)
-                cb[i] = __ldcs((i < NQ ? kb1 : kb2) + (size_t)q * NQ + (i % NQ));
-            __syncwarp();
-            const int cw = R.cut_word[q];
-            const int exq = R.kextra3[q];
-            // word by word: the candidate's two quads load once and serve every
-            // chunk of 32 tentatives with a pair left (fewer shared loads: the
-            // kernel is bound by their issue queue and the POPC pipe)
-            int dsum[RG / 32];
-#pragma unroll
-            for (int h = 0; h < RG / 32; h++) dsum[h] = 0;
-#pragma unroll 1
-            for (int w = 0; w < NQ; w++) {
-                const uint4 a1 = cb[w], a2 = cb[NQ + w];
-#pragma unroll
-                for (int h = 0; h < RG / 32; h++) {
-                    if (!ok_bits[h]) continue;
-                    const int t = 32 * h + lane;
-                    const uint4 b1 = tb[w * RG + t], b2 = tb[(NQ + w) * RG + t];
-                    dsum[h] += popc8(a1.x & b1.x, a1.y & b1.y, a1.z & b1.z, a1.w & b1.w,
-                                     a2.x & b2.x, a2.y & b2.y, a2.z & b2.z, a2.w & b2.w);
-                }
-            }
-#pragma unroll
-            for (int h = 0; h < RG / 32; h++) {
-                if (!ok_bits[h]) continue;
-                const int t = 32 * h + lane;
-                const int d = dsum[h];
-                if ((ok_bits[h] >> lane) & 1u) {
-                    n_wf++;
-                    if (d >= cw) {
-                        push_pair(st, pairs, seg_cap, R, ttent[t], q, kBandMaxW);
-                        n_al++;
-                    } else if (d + min(textra[t], exq) >= cw) {
-                        const int slot = atomicAdd(&st->n_amb, 1);
-                        if (slot < amb_cap) amb[slot] = Pair{ttent[t], q};
-                        else st->pair_overflow = 1;
-                    }
-                }
-            }
-            __syncwarp();
-        }
-    }
-    n_pf = (unsigned)warp_sum_i((int)n_pf);
-    n_wf = (unsigned)warp_sum_i((int)n_wf);
-    n_al = (unsigned)warp_sum_i((int)n_al);
-    if (lane == 0) {
-        if (n_pf) atomicAdd(&st->cnt_prefilter, (unsigned long long)n_pf);
-        if (n_wf) atomicAdd(&st->cnt_word, (unsigned long long)n_wf);
-        if (n_al) atomicAdd(&st->cnt_aligned, (unsigned long long)n_al);
-        if (bytes) atomicAdd(&st->filter_bytes, bytes);
-    }
 }
 
 // The open pairs grouped by tentative.  In the early passes of long-read
@@ -2581,16 +2720,14 @@ void launch_bfilter_bits_t(const DevReads& R, RoundBuffers& B, const int32_t* re
     // passes with one tentative (the first passes of adaptive R) go to the
     // plain kernel, which streams the candidates against one table
     launch_filter_t<K, false>(R, B, remain, s, B.tent);
-    constexpr int bsmem = (int)BitsSmem<K>::bytes;
-    constexpr int bthreads = BitsSmem<K>::THREADS;
     static int grid = 0;
     if (!grid) {
         cudaFuncSetAttribute(k_bfilter_bits<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             bsmem);
-        grid = grid_for(k_bfilter_bits<K>, bthreads, bsmem, 2);
+                             kBitsSmem);
+        grid = grid_for(k_bfilter_bits<K>, kBitsThreads, kBitsSmem, 1);
     }
-    k_bfilter_bits<K><<<shaped(grid, R.filter_blocks), bthreads, bsmem, s>>>(
-        R, B.st, remain, B.tent, B.pairs, B.seg_cap, B.amb, B.amb_cap);
+    k_bfilter_bits<K><<<grid, kBitsThreads, kBitsSmem, s>>>(R, B.st, remain, B.tent, B.pairs,
+                                                            B.seg_cap, B.amb, B.amb_cap);
     launch_exact_t<K>(R, B, s);
 }
 
