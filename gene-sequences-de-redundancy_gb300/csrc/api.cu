@@ -236,7 +236,6 @@ size_t carve_all(char* base, int n, int64_t n_bytes, const Plan& P, bool drop, i
     B.best = c.take<uint32_t>(n);
     B.tt = c.take<uint32_t>((size_t)kMaxBatch * kTTWords);
     B.ttrow = c.take<uint32_t>(kTTWords);
-    B.survive = c.take<uint32_t>(kTTWords);
     B.acc_cap = 2 * B.seg_cap;
     B.acc = c.take<Pair>((size_t)B.acc_cap);
     B.r_max = P.r_max;
@@ -411,6 +410,7 @@ int Job::init(const gsdr_reads* reads, const gsdr_opts* opts_in, cudaStream_t s,
     if (opts.group_words == 0)
         if (const char* gw = std::getenv("GSDR_GROUP_MAXW"))
             R_.group_max_w = std::min(std::max(std::atoi(gw), 0), kSegMaxWords);
+    R_.band_few = R_.group_max_w > 0 ? kBandFew : 0;
     // a window holds at most the longest read's rows
     R_.wide = (P.max_len + 31) / 32 > R_.group_max_w ? 1 : 0;
     refoff16_.swap(P.refoff16);
@@ -918,7 +918,8 @@ int Job::lcs_pairs(const int32_t* pat, const int32_t* txt, int n_pairs, int mapp
     JCUDA(cudaMemsetAsync(B_.cluster, 0xff, sizeof(int32_t) * n, stream));
     JCUDA(cudaMemsetAsync(B_.tidx, 0xff, sizeof(uint32_t) * n, stream));
     JCUDA(cudaEventRecord(ev_[2], stream));
-    R_.wide = 1;  // the queues above fill the systolic classes too
+    R_.wide = 1;      // the queues above fill the systolic classes too
+    R_.band_few = 0;  // and the lane-banded ones run on their own kernel
     launch_align_stage(R_, B_, mapping >= 1, stream);
     JCUDA(cudaGetLastError());
     JCUDA(cudaEventRecord(ev_[3], stream));

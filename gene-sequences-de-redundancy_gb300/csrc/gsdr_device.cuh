@@ -101,6 +101,8 @@ struct DevReads {
     // largest serial work (text bases x window words) of a pair given to the
     // lane-per-pair banded kernel; longer pairs go to the systolic kernels
     int64_t band_serial;
+    // lane-banded pairs of a stage up to which the segment kernel takes them
+    int32_t band_few;
     // block shape (gsdr_opts): resident CTAs per SM the alignment and the
     // word-filter kernels are launched with (0: as many as fit)
     int32_t align_blocks;
@@ -148,6 +150,7 @@ struct RoundState {
     int32_t absorbed;   // reads absorbed this pass
     int32_t n_amb;      // pairs the bitmap or mask bound left to the exact word filter
     int32_t n_pig;      // pairs queued for the pigeon filter
+    int32_t ticket;     // blocks of the compaction that have finished
     int32_t pass_limit; // > 0: stop after this many passes (timing runs; result unfinished)
     long long rounds;   // representatives taken so far
     long long passes;
@@ -169,6 +172,9 @@ int launch_kmers(const DevReads& R, int k, cudaStream_t s);
 // CTAs of the hash-based k-mer count (k >= 8): each owns R.khash_slots slots.
 constexpr int kHashCtas = 128;
 constexpr int kWideK = 8;  // word lengths from here on use the wide k-mer layout
+// DevReads::band_few of a job: about the pairs that k_seg's groups of eight
+// lanes hold at once (152 SMs x 16 warps x 4)
+constexpr int kBandFew = 8192;
 // Default of DevReads::band_serial (GSDR_BAND_SERIAL overrides it).
 constexpr long long kBandMaxSerial = 16384;
 // Base bit-planes of every read (after launch_pack).
@@ -192,9 +198,8 @@ struct RoundBuffers {
     int32_t* tent;       // kMaxBatch tentative read indices (ascending)
     uint32_t* tidx;      // n: (pass << 12) | tentative index, for reads that are tentatives
     uint32_t* best;      // n: (pass << 12) | (4095 - i) of the claiming tentative
-    uint32_t* tt;        // kMaxBatch x kTTWords: tentative h accepted tentative i
+    uint32_t* tt;        // kMaxBatch x kTTWords: row i, the tentatives that accepted tentative i
     uint32_t* ttrow;     // kTTWords: rows of tt with any bit
-    uint32_t* survive;   // kTTWords
     Pair* acc;           // accepted pairs of the pass
     int32_t acc_cap;
     // batched word filter by inverted index (sparse k-mer spaces; null = the

@@ -16,8 +16,9 @@
 //                 (lcs_seg.cuh); k_align (lcs_sys.cuh) takes the pairs whose
 //                 window is wider than that kernel holds.
 //   k_compact     updataRemain (func.cu:689-699): drops clustered reads from
-//                 the remain list and finds the smallest unclustered index.
-//   k_advance     updateRepresentative (func.cu:677-687).
+//                 the remain list and finds the smallest unclustered index;
+//                 its last block advances the round state
+//                 (updateRepresentative, func.cu:677-687).
 //
 // Batched form: every decision is a pure function of (representative,
 // candidate), so a pass takes the next R unclustered reads r_1 < ... < r_R as
@@ -35,10 +36,9 @@
 //                 k_bprefilter in drop mode
 //   k_band, k_seg, k_align  as above, accepted pairs listed instead of applied
 //                 (k_band: a lane per pair, short reads with narrow bands)
-//   k_bsurvive    survival of the tentatives in order (one warp)
-//   k_bclaim      first surviving tentative per candidate (keyed atomicMax)
-//   k_bapply      writes the winners into cluster[]
-//   k_compact, k_badvance
+//   k_bclaim      survival of the tentatives in order, then the first
+//                 surviving tentative per candidate (keyed atomicMax)
+//   k_compact     as above, and writes the winners into cluster[]
 // R adapts per pass: it halves after a pass in which representatives absorbed
 // many reads (tentatives there mostly repeat each other's work) and doubles
 // otherwise (8x after a pass too small to fill the device), up to the
@@ -146,6 +146,29 @@ constexpr unsigned long long kCandFixedBytes = 16 + 8 + 4;
 __device__ __forceinline__ unsigned long long cand_bytes(const DevReads& R, int q, bool drop) {
     // (k >= 8: 4-byte k-mer ids and 2-byte counts)
     return kCandFixedBytes + (drop ? 0ull : (R.kcnt ? 6ull : 4ull) * (unsigned)R.n_kmer[q]);
+}
+
+// Adds a kernel's counts to the round state, once per block.  Every thread of
+// the block calls it; the values are per warp, in lane 0.
+__device__ __forceinline__ void add_counts(RoundState* st, int lane, unsigned long long n_pf,
+                                           unsigned long long n_wf, unsigned long long n_al,
+                                           unsigned long long bytes) {
+    __shared__ unsigned long long s_cnt[4];
+    if (threadIdx.x < 4) s_cnt[threadIdx.x] = 0;
+    __syncthreads();
+    if (lane == 0) {
+        if (n_pf) atomicAdd(&s_cnt[0], n_pf);
+        if (n_wf) atomicAdd(&s_cnt[1], n_wf);
+        if (n_al) atomicAdd(&s_cnt[2], n_al);
+        if (bytes) atomicAdd(&s_cnt[3], bytes);
+    }
+    __syncthreads();
+    if (threadIdx.x < 4 && s_cnt[threadIdx.x])
+        atomicAdd(threadIdx.x == 0   ? &st->cnt_prefilter
+                  : threadIdx.x == 1 ? &st->cnt_word
+                  : threadIdx.x == 2 ? &st->cnt_aligned
+                                     : &st->filter_bytes,
+                  s_cnt[threadIdx.x]);
 }
 
 // ---------------------------------------------------------------- plain form
@@ -269,12 +292,9 @@ __global__ void __launch_bounds__(kFilterThreads, 6) k_filter(DevReads R, RoundS
         n_al++;
         if (lane == 0) push_pair(st, pairs, seg_cap, R, rep, q, band_w);
     }
-    if (lane == 0) {
-        if (n_pf) atomicAdd(&st->cnt_prefilter, (unsigned long long)n_pf);
-        if (n_wf) atomicAdd(&st->cnt_word, (unsigned long long)n_wf);
-        if (n_al) atomicAdd(&st->cnt_aligned, (unsigned long long)n_al);
-        if (bytes) atomicAdd(&st->filter_bytes, bytes);
-    }
+    // one addition per block and counter: the counters share a cache line, and
+    // one per warp (7,296 warps) took most of a 10k-candidate launch's 21.9 us
+    add_counts(st, lane, n_pf, n_wf, n_al, bytes);
 }
 
 // kernel_pigeon (cuda-version/func.cu:756-801) on the queued pairs, one warp
@@ -381,12 +401,7 @@ __global__ void __launch_bounds__(kFilterThreads) k_filter_g(DevReads R, RoundSt
         n_al++;
         if (lane == 0) push_pair(st, pairs, seg_cap, R, rep, q, kPlainBandMaxW);
     }
-    if (lane == 0) {
-        if (n_pf) atomicAdd(&st->cnt_prefilter, (unsigned long long)n_pf);
-        if (n_wf) atomicAdd(&st->cnt_word, (unsigned long long)n_wf);
-        if (n_al) atomicAdd(&st->cnt_aligned, (unsigned long long)n_al);
-        if (bytes) atomicAdd(&st->filter_bytes, bytes);
-    }
+    add_counts(st, lane, n_pf, n_wf, n_al, bytes);
 }
 
 // Decisions that need no alignment; -1 when the LCS must be computed.
@@ -426,8 +441,8 @@ __device__ __forceinline__ void on_accept(RoundState* st, const AlignArgs& A, co
     const uint32_t kc = A.tidx[p.cand];
     if ((int)(kc >> 12) == pass) {
         const int h = A.tidx[p.rep] & 0xfff, ci = kc & 0xfff;
-        atomicOr(&A.tt[h * kTTWords + (ci >> 5)], 1u << (ci & 31));
-        atomicOr(&A.ttrow[h >> 5], 1u << (h & 31));
+        atomicOr(&A.tt[ci * kTTWords + (h >> 5)], 1u << (h & 31));
+        atomicOr(&A.ttrow[ci >> 5], 1u << (ci & 31));
     }
 }
 
@@ -577,13 +592,26 @@ __global__ void __launch_bounds__(kAlignThreads, 3) k_align_single(DevReads R, R
 // fits a window of W words: one pair per lane.  All lanes of a warp run the
 // same blocks of 32 text bases, each on its own pair; a lane whose pair is
 // decided takes the next one from the class queue at the next block.
+//
+// A lane's pair takes a few hundred dependent steps per word, so a launch lasts
+// 20 us (150 bp) to 50 us (1,000 bp) however few its pairs are; a stage of at
+// most R.band_few leaves them to k_seg, whose groups of lanes finish a pair in
+// a fraction of that (14 passes of 10k reads of 200-1,000 bp: 70 -> 20 us).
+__device__ __forceinline__ int band_pairs(const RoundState* st) {
+    int n = 0;
+#pragma unroll
+    for (int c = 0; c < kBandClasses; c++) n += st->n_pairs[kSysClasses + c];
+    return n;
+}
+
 template <int W, bool BATCH>
 __global__ void __launch_bounds__(kAlignThreads) k_band(DevReads R, RoundState* st, AlignArgs A,
                                                         int cls) {
-    // text bases per unrolled group: fewer for wide windows (code size)
-    constexpr int G = W >= 16 ? 4 : 8;
+    // text bases per unrolled group
+    constexpr int G = 8;
     if (st->done) return;
     if (BATCH && (st->pair_overflow || st->n_tent == 0)) return;
+    if (band_pairs(st) <= R.band_few) return;  // k_seg's
     const int np = min(st->n_pairs[cls], A.seg_cap);
     if (np <= 0) return;
     const int pass = BATCH ? st->pass : 0;
@@ -679,9 +707,10 @@ __global__ void __launch_bounds__(kAlignThreads, 2) k_seg(DevReads R, RoundState
     if (BATCH && (st->pair_overflow || st->n_tent == 0)) return;
     constexpr int c0 = NARROW ? kNarrowClass : kSysClasses + kBandClasses;
     constexpr int nc = NARROW ? 1 : kSegClasses;
+    // the lane-banded classes' pairs too when they are few (k_band)
+    const int first = !NARROW && BATCH && band_pairs(st) <= R.band_few ? -kBandClasses : 0;
     int total = 0;
-#pragma unroll
-    for (int c = 0; c < nc; c++) total += min(st->n_pairs[c0 + c], A.seg_cap);
+    for (int c = first; c < nc; c++) total += min(st->n_pairs[c0 + c], A.seg_cap);
     if (total <= 0) return;
     const bool alone = total <= (int)gridDim.x * (kAlignThreads / 64);
     const int pass = BATCH ? st->pass : 0;
@@ -691,7 +720,7 @@ __global__ void __launch_bounds__(kAlignThreads, 2) k_seg(DevReads R, RoundState
     for (int i = lane; i < kSegMaxW * 32; i += 32) peq[kSegNoBase + i] = 0u;
     unsigned long long cells = 0, done = 0;
     unsigned acc = 0;
-    for (int cls = nc - 1; cls >= 0; cls--) {
+    for (int cls = nc - 1; cls >= first; cls--) {
         const int np = min(st->n_pairs[c0 + cls], A.seg_cap);
         if (np <= 0) continue;
         const int G = alone || cls == 4 ? 32 : cls == 3 ? 16 : 8;
@@ -772,11 +801,24 @@ __global__ void __launch_bounds__(kAlignThreads, 2) k_seg(DevReads R, RoundState
             P = SegPair{};
         }
     }
+    // (cells: steps x the window's words x 32 bits)
     acc = (unsigned)warp_sum_i((int)acc);
-    if (!BATCH && lane == 0 && acc) atomicAdd(&st->cnt_accepted, (unsigned long long)acc);
-    if (cells) atomicAdd(&st->cells, cells);
-    // cells: steps x the window's words x 32 bits
-    if (done) atomicAdd(&st->cells_done, done);
+    cells = warp_sum_ull(cells);
+    done = warp_sum_ull(done);
+    __shared__ unsigned long long s_sum[3];
+    if (threadIdx.x < 3) s_sum[threadIdx.x] = 0;
+    __syncthreads();
+    if (lane == 0) {
+        atomicAdd(&s_sum[0], cells);
+        atomicAdd(&s_sum[1], done);
+        atomicAdd(&s_sum[2], (unsigned long long)acc);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (s_sum[0]) atomicAdd(&st->cells, s_sum[0]);
+        if (s_sum[1]) atomicAdd(&st->cells_done, s_sum[1]);
+        if (!BATCH && s_sum[2]) atomicAdd(&st->cnt_accepted, s_sum[2]);
+    }
 }
 
 // Pairs whose pattern has more rows than one group of 8 warps x 32 lanes x 8
@@ -860,36 +902,7 @@ __global__ void __launch_bounds__(kAlignThreads, 1) k_align_long(DevReads R, Rou
     if (lane == 0 && done) atomicAdd(&st->cells_done, done);
 }
 
-__global__ void k_compact(RoundState* st, const int32_t* __restrict__ remain_in,
-                          int32_t* __restrict__ remain_out, const int32_t* __restrict__ cluster) {
-    if (st->done) return;
-    const int n = st->n_remain;
-    const int lane = threadIdx.x & 31;
-    int local_min = 0x7fffffff;
-    const int stride = gridDim.x * blockDim.x;
-    for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += stride) {
-        const int idx = base + lane;
-        int j = -1;
-        bool keep = false;
-        if (idx < n) {
-            j = remain_in[idx];
-            keep = cluster[j] == -1;
-        }
-        const unsigned m = __ballot_sync(kFull, keep);
-        if (!m) continue;
-        int pos = 0;
-        if (lane == 0) pos = atomicAdd(&st->n_next, __popc(m));
-        pos = __shfl_sync(kFull, pos, 0);
-        if (keep) {
-            remain_out[pos + __popc(m & ((1u << lane) - 1u))] = j;
-            local_min = min(local_min, j);
-        }
-    }
-    local_min = __reduce_min_sync(kFull, local_min);
-    if (lane == 0 && local_min != 0x7fffffff) atomicMin(&st->next_min, local_min);
-}
-
-__device__ void reset_align_counters(RoundState* st, int* align_work) {
+__device__ void reset_align_counters(volatile RoundState* st, int* align_work) {
     st->n_pig = 0;
     for (int c = 0; c < kAlignClasses; c++) {
         st->n_pairs[c] = 0;
@@ -898,10 +911,12 @@ __device__ void reset_align_counters(RoundState* st, int* align_work) {
     align_work[kSingleWorkSlot] = 0;  // k_align_single's shared queue
 }
 
-__global__ void k_advance(RoundState* st, int32_t* cluster, int* align_work) {
-    if (st->done) return;
-    st->rounds += 1;
-    st->passes += 1;
+// Next representative (plain form).  Runs in one thread of the last block of
+// k_compact; `st` is volatile so that the other blocks' additions are read
+// from L2.
+__device__ void advance_plain(volatile RoundState* st, int32_t* cluster, int* align_work) {
+    st->rounds = st->rounds + 1;
+    st->passes = st->passes + 1;
     if (st->error || st->pair_overflow) {
         st->done = 1;
         return;
@@ -927,14 +942,160 @@ __global__ void k_advance(RoundState* st, int32_t* cluster, int* align_work) {
     reset_align_counters(st, align_work);
 }
 
+// The batched form's state for the next pass (in the same place).
+__device__ void advance_batch(volatile RoundState* st, const int32_t* tent, int seg_cap,
+                              int acc_cap, int amb_cap, int drop) {
+    st->passes = st->passes + 1;
+    st->pass = st->pass + 1;
+    if (st->error) {
+        st->done = 1;
+        return;
+    }
+    if (st->pair_overflow || st->acc_overflow) {
+        // queues too small for this many tentatives: the pass changed nothing
+        // (the compaction copied the remain list unchanged); redo it with fewer
+        if (st->R == 1) {
+            st->error = 2;
+            st->done = 1;
+            return;
+        }
+        st->R = max(1, st->R / 8);
+        st->n_next = 0;
+        return;
+    }
+    const int nt = st->n_tent;
+    if (nt > 0) st->cursor = tent[nt - 1] + 1;
+    const int surv = max(1, st->survivors);
+    // a pass that queued fewer pairs than the device keeps in flight ran on
+    // the latency of its longest pairs: grow R faster, and also where its
+    // representatives absorbed many reads (the tentatives' repeated work is
+    // then free; 30k reads of 150-5,000 bp at t = 0.90 spent 18 of 43 passes
+    // at R = 1)
+    int queued = 0, fullest = 0;
+    for (int c = 0; c < kAlignClasses; c++) {
+        queued += st->n_pairs[c];
+        fullest = max(fullest, st->n_pairs[c]);
+    }
+    if (queued >= kFewPairs && st->absorbed > kAbsorbHigh * surv) {
+        st->R = max(1, st->R / 2);
+    } else {
+        // (drop mode has no filter pass to share between tentatives: R grows
+        // only while the passes are too small to fill the device, since every
+        // tentative that an earlier one absorbs wastes its alignments)
+        long long r = (long long)st->R * (queued < kFewPairs ? 8 : (drop ? 1 : 2));
+        // queue use grows with the tentatives: keep the fullest alignment
+        // queue and the accept list under 3/4 of their capacity (an overflow
+        // costs a redone pass; without the cap, drop mode, where every
+        // candidate pairs with every tentative, alternates between overflow
+        // and a small R)
+        if (nt > 0 && fullest > 0) r = min(r, (long long)nt * (3ll * seg_cap / 4) / fullest);
+        if (nt > 0 && st->n_acc > 0) r = min(r, (long long)nt * (3ll * acc_cap / 4) / st->n_acc);
+        // and the bitmap filter's queue of open pairs
+        if (nt > 0 && amb_cap > 0 && st->n_amb > 0)
+            r = min(r, (long long)nt * (3ll * amb_cap / 4) / st->n_amb);
+        st->R = (int)max(1ll, min((long long)st->R_max, r));
+    }
+    const int n = st->n_next;
+    st->n_next = 0;
+    st->next_min = 0x7fffffff;
+    if (n == 0) {
+        st->done = 1;
+        return;
+    }
+    st->n_remain = n;
+    if (st->pass_limit > 0 && st->passes >= st->pass_limit) st->done = 1;  // timing runs
+}
+
+struct CompactArgs {
+    int32_t* cluster;
+    int* align_work;
+    // batched form
+    const uint32_t* best;
+    const int32_t* tent;
+    int seg_cap, acc_cap, amb_cap, drop;
+};
+
+// Drops clustered reads from the remain list.  Batched: a candidate claimed in
+// this pass (k_bclaim) joins its tentative here.  The last block to finish
+// advances the round state (a launch of its own took about 4 us per round).
+template <bool BATCH>
+__global__ void __launch_bounds__(256) k_compact(RoundState* st, const int32_t* __restrict__ remain_in,
+                                                 int32_t* __restrict__ remain_out, CompactArgs C) {
+    __shared__ int s_min, s_applied, s_last;
+    if (st->done) return;
+    if (threadIdx.x == 0) {
+        s_min = 0x7fffffff;
+        s_applied = 0;
+    }
+    __syncthreads();
+    const int n = st->n_remain;
+    const int lane = threadIdx.x & 31;
+    const uint32_t pass = BATCH ? (uint32_t)st->pass : 0u;
+    const bool apply = BATCH && st->n_tent > 0 && !st->pair_overflow && !st->acc_overflow;
+    int local_min = 0x7fffffff;
+    unsigned applied = 0;
+    const int stride = gridDim.x * blockDim.x;
+    for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += stride) {
+        const int idx = base + lane;
+        int j = -1;
+        bool keep = false;
+        if (idx < n) {
+            j = remain_in[idx];
+            keep = C.cluster[j] == -1;
+            if (apply && keep) {
+                const uint32_t key = C.best[j];
+                if ((key >> 12) == pass) {
+                    C.cluster[j] = C.tent[4095u - (key & 0xfffu)];
+                    applied++;
+                    keep = false;
+                }
+            }
+        }
+        const unsigned m = __ballot_sync(kFull, keep);
+        if (!m) continue;
+        int pos = 0;
+        if (lane == 0) pos = atomicAdd(&st->n_next, __popc(m));
+        pos = __shfl_sync(kFull, pos, 0);
+        if (keep) {
+            remain_out[pos + __popc(m & ((1u << lane) - 1u))] = j;
+            local_min = min(local_min, j);
+        }
+    }
+    if (!BATCH) {
+        local_min = __reduce_min_sync(kFull, local_min);
+        if (lane == 0 && local_min != 0x7fffffff) atomicMin(&s_min, local_min);
+    } else {
+        applied = __reduce_add_sync(kFull, applied);
+        if (lane == 0 && applied) atomicAdd(&s_applied, (int)applied);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (!BATCH && s_min != 0x7fffffff) atomicMin(&st->next_min, s_min);
+        if (BATCH && s_applied) {
+            atomicAdd(&st->absorbed, s_applied);
+            atomicAdd(&st->cnt_accepted, (unsigned long long)s_applied);
+        }
+        __threadfence();
+        s_last = atomicAdd(&st->ticket, 1) == (int)gridDim.x - 1;
+        if (s_last) {
+            __threadfence();
+            st->ticket = 0;
+            if (BATCH)
+                advance_batch(st, C.tent, C.seg_cap, C.acc_cap, C.amb_cap, C.drop);
+            else
+                advance_plain(st, C.cluster, C.align_work);
+        }
+    }
+}
+
 // ---------------------------------------------------------------- batched form
 
 // Next R unclustered indices at or after the cursor, in increasing order.
 __global__ void __launch_bounds__(1024) k_bselect(RoundState* st, const int32_t* __restrict__ cluster,
                                                   int n, int32_t* tent, uint32_t* tidx,
-                                                  uint32_t* tt, uint32_t* ttrow, uint32_t* survive,
+                                                  uint32_t* tt, uint32_t* ttrow,
                                                   int* align_work) {
-    __shared__ int warp_cnt[32];
+    __shared__ int warp_cnt[4 * 32];
     __shared__ int s_nt;
     if (st->done) return;
     const int Rq = st->R;
@@ -943,36 +1104,57 @@ __global__ void __launch_bounds__(1024) k_bselect(RoundState* st, const int32_t*
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) s_nt = 0;
     __syncthreads();
+    // 4,096 reads per step (four per thread): once most reads are clustered the
+    // unclustered ones are far apart
     while (pos < n) {
         const int nt = s_nt;
         if (nt >= Rq) break;
-        const int idx = pos + threadIdx.x;
-        const bool un = idx < n && cluster[idx] == -1;
-        const unsigned m = __ballot_sync(kFull, un);
-        if (lane == 0) warp_cnt[warp] = __popc(m);
-        __syncthreads();
-        int before = 0, total = 0;
-        for (int w = 0; w < 32; w++) {
-            const int c = warp_cnt[w];
-            if (w < warp) before += c;
-            total += c;
+        unsigned m[4];
+        bool un[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int idx = pos + 1024 * k + threadIdx.x;
+            un[k] = idx < n && cluster[idx] == -1;
         }
-        const int rank = nt + before + __popc(m & ((1u << lane) - 1u));
-        if (un && rank < Rq) {
-            tent[rank] = idx;
-            tidx[idx] = ((uint32_t)pass << 12) | (uint32_t)rank;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            m[k] = __ballot_sync(kFull, un[k]);
+            if (lane == 0) warp_cnt[32 * k + warp] = __popc(m[k]);
         }
         __syncthreads();
-        if (threadIdx.x == 0) s_nt = min(Rq, nt + total);
-        pos += blockDim.x;
+        if (warp == 0) {
+            // exclusive prefix over the 128 (quarter, warp) counts
+            int run = nt;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int c = warp_cnt[32 * k + lane];
+                int incl = c;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int o = __shfl_up_sync(kFull, incl, d);
+                    if (lane >= d) incl += o;
+                }
+                warp_cnt[32 * k + lane] = run + incl - c;
+                run += __shfl_sync(kFull, incl, 31);
+            }
+            if (lane == 0) s_nt = min(Rq, run);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int idx = pos + 1024 * k + threadIdx.x;
+            const int rank = warp_cnt[32 * k + warp] + __popc(m[k] & ((1u << lane) - 1u));
+            if (un[k] && rank < Rq) {
+                tent[rank] = idx;
+                tidx[idx] = ((uint32_t)pass << 12) | (uint32_t)rank;
+            }
+        }
+        pos += 4 * blockDim.x;
         __syncthreads();
     }
     const int nt = s_nt;
     for (int i = threadIdx.x; i < nt * kTTWords; i += blockDim.x) tt[i] = 0u;
-    if (threadIdx.x < kTTWords) {
-        ttrow[threadIdx.x] = 0u;
-        survive[threadIdx.x] = 0u;
-    }
+    if (threadIdx.x < kTTWords) ttrow[threadIdx.x] = 0u;
     if (threadIdx.x == 0) {
         st->n_tent = nt;
         st->n_acc = 0;
@@ -2358,153 +2540,70 @@ __global__ void __launch_bounds__(kMaskThreads, 2) k_bfilter_mask(
     }
 }
 
-// Survival of the tentatives in greedy order (one warp): a tentative survives
-// iff no surviving earlier tentative accepted it.  Only rows with a bit can
-// claim anything, so only those are visited, in increasing order.
-__global__ void k_bsurvive(RoundState* st, const int32_t* __restrict__ tent,
-                           const uint32_t* __restrict__ tt, const uint32_t* __restrict__ ttrow,
-                           uint32_t* survive, int32_t* cluster) {
-    if (st->done || st->n_tent == 0) return;
-    if (st->pair_overflow || st->acc_overflow) return;
+// Survival of the tentatives in greedy order (a tentative survives iff no
+// surviving earlier tentative accepted it), then the claims: the first
+// surviving tentative of each accepted candidate, by keyed atomicMax.
+//
+// Row i of tt holds the tentatives that accepted tentative i (all before it).
+// Thread i decides tentative i: claimed once one of them survives, a survivor
+// once all of them are claimed.  Each step decides at least the first open
+// tentative, and in practice nearly all within a few steps, where one warp
+// going through the rows in order took 40 us a pass.  Every block repeats
+// this (the rows are in L2) instead of waiting for a launch that does it once.
+__global__ void __launch_bounds__(kMaxBatch) k_bclaim(RoundState* st, const int32_t* __restrict__ tent,
+                                                      const uint32_t* __restrict__ tt,
+                                                      const uint32_t* __restrict__ ttrow,
+                                                      const Pair* __restrict__ acc,
+                                                      const uint32_t* __restrict__ tidx,
+                                                      uint32_t* best, int32_t* cluster) {
+    __shared__ __align__(16) uint32_t surv[kTTWords], open[kTTWords];
+    if (st->done || st->n_tent == 0 || st->pair_overflow || st->acc_overflow) return;
     const int nt = st->n_tent;
-    const int lane = threadIdx.x;
-    uint32_t claimed = 0;  // bits [32*lane, 32*lane+32) of the claimed set
-    const uint32_t rows = ttrow[lane];
-    for (int w = 0; w < kTTWords; w++) {
-        uint32_t rw = __shfl_sync(kFull, rows, w);
-        while (rw) {
-            // the next eight rows with bits: their words are loaded together
-            // (they do not depend on the claims), then applied in order
-            constexpr int P = 8;
-            int hs[P];
-            uint32_t v[P];
+    const int na = st->n_acc;
+    // (a block without claims leaves them to the others; block 0 marks the survivors)
+    if (blockIdx.x > 0 && (long long)blockIdx.x * kMaxBatch >= na) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = threadIdx.x;
+    const uint32_t flagged = ttrow[warp];
+    bool undecided = i < nt && ((flagged >> lane) & 1u);
+    bool alive = i < nt && !undecided;
+    uint4 row[kTTWords / 4];
+    if (undecided) {
 #pragma unroll
-            for (int j = 0; j < P; j++) {
-                hs[j] = rw ? w * 32 + __ffs(rw) - 1 : -1;
-                rw &= rw - 1u;
+        for (int w = 0; w < kTTWords / 4; w++)
+            row[w] = reinterpret_cast<const uint4*>(tt)[(size_t)i * (kTTWords / 4) + w];
+    }
+    while (true) {
+        const unsigned ms = __ballot_sync(kFull, alive), mo = __ballot_sync(kFull, undecided);
+        if (lane == 0) surv[warp] = ms, open[warp] = mo;
+        if (!__syncthreads_or((int)mo)) break;
+        if (undecided) {
+            uint32_t by_surv = 0, by_open = 0;
+#pragma unroll
+            for (int w = 0; w < kTTWords / 4; w++) {
+                const uint4 s4 = reinterpret_cast<const uint4*>(surv)[w];
+                const uint4 o4 = reinterpret_cast<const uint4*>(open)[w];
+                by_surv |= (row[w].x & s4.x) | (row[w].y & s4.y) | (row[w].z & s4.z) | (row[w].w & s4.w);
+                by_open |= (row[w].x & o4.x) | (row[w].y & o4.y) | (row[w].z & o4.z) | (row[w].w & o4.w);
             }
-#pragma unroll
-            for (int j = 0; j < P; j++) v[j] = hs[j] >= 0 ? tt[hs[j] * kTTWords + lane] : 0u;
-#pragma unroll
-            for (int j = 0; j < P; j++) {
-                if (hs[j] < 0) break;  // warp-uniform
-                const uint32_t cw = __shfl_sync(kFull, claimed, hs[j] >> 5);
-                if (!((cw >> (hs[j] & 31)) & 1u)) claimed |= v[j];
-            }
+            if (by_surv) undecided = false;
+            else if (!by_open) undecided = false, alive = true;
+        }
+        __syncthreads();
+    }
+    if (blockIdx.x == 0) {
+        if (alive) cluster[tent[i]] = tent[i];
+        const int count = __syncthreads_count(alive);
+        if (threadIdx.x == 0) {
+            st->survivors = count;
+            st->rounds += count;
         }
     }
-    uint32_t valid;
-    const int lo = lane * 32;
-    valid = nt >= lo + 32 ? 0xffffffffu : (nt > lo ? ((1u << (nt - lo)) - 1u) : 0u);
-    const uint32_t surv = ~claimed & valid;
-    survive[lane] = surv;
-    uint32_t s = surv;
-    while (s) {
-        const int i = lo + __ffs(s) - 1;
-        s &= s - 1;
-        cluster[tent[i]] = tent[i];
-    }
-    const int count = warp_sum_i(__popc(surv));
-    if (lane == 0) {
-        st->survivors = count;
-        st->rounds += count;
-    }
-}
-
-__global__ void k_bclaim(RoundState* st, const Pair* __restrict__ acc,
-                         const uint32_t* __restrict__ tidx, const uint32_t* __restrict__ survive,
-                         uint32_t* best) {
-    if (st->done || st->n_tent == 0 || st->pair_overflow || st->acc_overflow) return;
-    const int na = st->n_acc;
     const uint32_t pass = (uint32_t)st->pass;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < na; k += gridDim.x * blockDim.x) {
         const Pair p = acc[k];
-        const int i = tidx[p.rep] & 0xfff;
-        if ((survive[i >> 5] >> (i & 31)) & 1u) atomicMax(&best[p.cand], (pass << 12) | (4095u - i));
+        const int t = tidx[p.rep] & 0xfff;
+        if ((surv[t >> 5] >> (t & 31)) & 1u) atomicMax(&best[p.cand], (pass << 12) | (4095u - t));
     }
-}
-
-__global__ void k_bapply(RoundState* st, const Pair* __restrict__ acc,
-                         const uint32_t* __restrict__ tidx, const uint32_t* __restrict__ best,
-                         int32_t* cluster) {
-    if (st->done || st->n_tent == 0 || st->pair_overflow || st->acc_overflow) return;
-    const int na = st->n_acc;
-    const uint32_t pass = (uint32_t)st->pass;
-    unsigned applied = 0;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < na; k += gridDim.x * blockDim.x) {
-        const Pair p = acc[k];
-        const int i = tidx[p.rep] & 0xfff;
-        if (best[p.cand] == ((pass << 12) | (4095u - i))) {
-            cluster[p.cand] = p.rep;
-            applied++;
-        }
-    }
-    applied = __reduce_add_sync(kFull, applied);
-    if ((threadIdx.x & 31) == 0 && applied) {
-        atomicAdd(&st->absorbed, (int)applied);
-        atomicAdd(&st->cnt_accepted, (unsigned long long)applied);
-    }
-}
-
-__global__ void k_badvance(RoundState* st, const int32_t* __restrict__ tent, int* align_work,
-                           int seg_cap, int acc_cap, int amb_cap, int drop) {
-    if (st->done) return;
-    st->passes += 1;
-    st->pass += 1;
-    if (st->error) {
-        st->done = 1;
-        return;
-    }
-    if (st->pair_overflow || st->acc_overflow) {
-        // queues too small for this many tentatives: the pass changed nothing
-        // (the compaction copied the remain list unchanged); redo it with fewer
-        if (st->R == 1) {
-            st->error = 2;
-            st->done = 1;
-            return;
-        }
-        st->R = max(1, st->R / 8);
-        st->n_next = 0;
-        return;
-    }
-    const int nt = st->n_tent;
-    if (nt > 0) st->cursor = tent[nt - 1] + 1;
-    const int surv = max(1, st->survivors);
-    // a pass that queued fewer pairs than the device keeps in flight ran on
-    // the latency of its longest pairs: grow R faster
-    int queued = 0, fullest = 0;
-    for (int c = 0; c < kAlignClasses; c++) {
-        queued += st->n_pairs[c];
-        fullest = max(fullest, st->n_pairs[c]);
-    }
-    if (st->absorbed > kAbsorbHigh * surv) {
-        st->R = max(1, st->R / 2);
-    } else {
-        // (drop mode has no filter pass to share between tentatives: R grows
-        // only while the passes are too small to fill the device, since every
-        // tentative that an earlier one absorbs wastes its alignments)
-        long long r = (long long)st->R * (queued < kFewPairs ? 8 : (drop ? 1 : 2));
-        // queue use grows with the tentatives: keep the fullest alignment
-        // queue and the accept list under 3/4 of their capacity (an overflow
-        // costs a redone pass; without the cap, drop mode, where every
-        // candidate pairs with every tentative, alternates between overflow
-        // and a small R)
-        if (nt > 0 && fullest > 0) r = min(r, (long long)nt * (3ll * seg_cap / 4) / fullest);
-        if (nt > 0 && st->n_acc > 0) r = min(r, (long long)nt * (3ll * acc_cap / 4) / st->n_acc);
-        // and the bitmap filter's queue of open pairs
-        if (nt > 0 && amb_cap > 0 && st->n_amb > 0)
-            r = min(r, (long long)nt * (3ll * amb_cap / 4) / st->n_amb);
-        st->R = (int)max(1ll, min((long long)st->R_max, r));
-    }
-    const int n = st->n_next;
-    st->n_next = 0;
-    st->next_min = 0x7fffffff;
-    if (n == 0) {
-        st->done = 1;
-        return;
-    }
-    st->n_remain = n;
-    if (st->pass_limit > 0 && st->passes >= st->pass_limit) st->done = 1;  // timing runs
 }
 
 __global__ void k_init(RoundState* st, int32_t* cluster, int32_t* remain, uint32_t* tidx,
@@ -2961,11 +3060,11 @@ void launch_plain_round(const DevReads& R, RoundBuffers& B, int drop, int parity
     if (ev4) cudaEventRecordWithFlags(ev4[1], s, cudaEventRecordExternal);
     launch_align_classes<false>(R, B, s);
     if (ev4) cudaEventRecordWithFlags(ev4[2], s, cudaEventRecordExternal);
-    k_compact<<<num_sms() * 4, 256, 0, s>>>(B.st, rin, rout, B.cluster);
-    k_advance<<<1, 1, 0, s>>>(B.st, B.cluster, align_work_of(B.st));
+    k_compact<false><<<num_sms() * 4, 256, 0, s>>>(
+        B.st, rin, rout, CompactArgs{B.cluster, align_work_of(B.st), nullptr, nullptr, 0, 0, 0, 0});
     if (ev4) cudaEventRecordWithFlags(ev4[3], s, cudaEventRecordExternal);
     if (count)
-        *count += 3 + align_launches<false>(R, B) + (R.pig_q && !drop ? 1 : 0) +
+        *count += 2 + align_launches<false>(R, B) + (R.pig_q && !drop ? 1 : 0) +
                   (!drop && R.k >= kWideK ? 2 : 0);
 }
 
@@ -2985,7 +3084,7 @@ void launch_batch_pass(const DevReads& R, RoundBuffers& B, int drop, int parity,
                        long long* count, cudaEvent_t* ev4) {
     const int32_t* rin = B.remain[parity];
     int32_t* rout = B.remain[parity ^ 1];
-    k_bselect<<<1, 1024, 0, s>>>(B.st, B.cluster, R.n, B.tent, B.tidx, B.tt, B.ttrow, B.survive,
+    k_bselect<<<1, 1024, 0, s>>>(B.st, B.cluster, R.n, B.tent, B.tidx, B.tt, B.ttrow,
                                  align_work_of(B.st));
     if (ev4) cudaEventRecordWithFlags(ev4[0], s, cudaEventRecordExternal);
     launch_filter_any<true>(R, B, rin, drop, s);
@@ -2993,16 +3092,15 @@ void launch_batch_pass(const DevReads& R, RoundBuffers& B, int drop, int parity,
     if (ev4) cudaEventRecordWithFlags(ev4[1], s, cudaEventRecordExternal);
     launch_align_classes<true>(R, B, s);
     if (ev4) cudaEventRecordWithFlags(ev4[2], s, cudaEventRecordExternal);
-    k_bsurvive<<<1, 32, 0, s>>>(B.st, B.tent, B.tt, B.ttrow, B.survive, B.cluster);
-    const int g = num_sms() * 2;
-    k_bclaim<<<g, 256, 0, s>>>(B.st, B.acc, B.tidx, B.survive, B.best);
-    k_bapply<<<g, 256, 0, s>>>(B.st, B.acc, B.tidx, B.best, B.cluster);
-    k_compact<<<num_sms() * 4, 256, 0, s>>>(B.st, rin, rout, B.cluster);
-    k_badvance<<<1, 1, 0, s>>>(B.st, B.tent, align_work_of(B.st), B.seg_cap, B.acc_cap,
-                               B.amb_cap, drop);
+    k_bclaim<<<num_sms(), kMaxBatch, 0, s>>>(B.st, B.tent, B.tt, B.ttrow, B.acc, B.tidx, B.best,
+                                             B.cluster);
+    k_compact<true><<<num_sms() * 4, 256, 0, s>>>(
+        B.st, rin, rout,
+        CompactArgs{B.cluster, align_work_of(B.st), B.best, B.tent, B.seg_cap, B.acc_cap, B.amb_cap,
+                    drop});
     if (ev4) cudaEventRecordWithFlags(ev4[3], s, cudaEventRecordExternal);
     if (count)
-        *count += 7 + align_launches<true>(R, B) + (!drop ? 1 : 0) +
+        *count += 4 + align_launches<true>(R, B) + (!drop ? 1 : 0) +
                   (R.pig_q && !drop ? 1 : 0) + (B.amb && !drop ? 4 : 0);
     // (a word-filter form launches two kernels, six with the open-pair
     // queue: the bitmap form k_filter, k_bfilter_bits, the mask form k_bmask,
