@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -72,6 +73,7 @@ struct Plan {
     bool idx_smem = false;  // that index fits the filter's shared memory (16-bit copy)
     bool bits = false;      // batched word filter by k-mer presence bitmaps
     bool masks = false;     // batched word filter by tentative masks
+    int hbuckets = 0;       // that form by hashed k-mer counts, their buckets
     int mask_planes = 8;    // their count planes (10 where a read has over 255 entries)
     // pigeon filter (p 1): low 16 bits of each read's offset in the
     // reference's padded layout (copyData, func.cu:119-137: L/16*16 + 16 per read)
@@ -93,6 +95,25 @@ int job_r_max(const gsdr_opts& o) {
 // kMaskMaxEntries k-mer entries, else the inverted index of the tentatives'
 // k-mers.  GSDR_BFILTER=table|index|bits|masks forces a form.
 constexpr int64_t kIndexDensity = 8;
+
+// Buckets of the hashed k-mer counts for reads of up to max_len bases, or 0:
+// the tentative masks.  Two unrelated reads of L k-mers each reach a product
+// sum of about L^2 / H, close to a Poisson variable; the fewest buckets that
+// leave the word cutoff five deviations above it (150 bp reads at t = 0.90:
+// 1,536, where about one unrelated pair in 1e5 stays open).  Longer reads would
+// need more buckets, each of which costs as much as any other, while the masks
+// cost by the k-mers a read has: 2,048 buckets at 1.0e12 pairs/s break even
+// with the masks at about 100 k-mers.
+int hash_buckets(int64_t max_len, int k, float t) {
+    const double L = (double)max_len - k + 1;
+    const double cut = L - std::ceil((double)max_len * (1.0 - (double)t)) * k;
+    if (L < 1 || cut < 1) return 0;
+    for (int h = kHashMinBuckets; h <= kHashMaxBuckets; h += 512) {
+        const double mean = L * L / h;
+        if (mean + 5.0 * std::sqrt(mean) <= cut) return h;
+    }
+    return 0;
+}
 
 int make_plan(const gsdr_reads* reads, const gsdr_opts& o, Plan& P, PlanPreset* pre) {
     const int n = reads->n;
@@ -167,6 +188,7 @@ int make_plan(const gsdr_reads* reads, const gsdr_opts& o, Plan& P, PlanPreset* 
         if (masks) index = false;
         P.bits = bits;
         P.masks = masks;
+        if (masks) P.hbuckets = hash_buckets(P.max_len, k, o.threshold);
         // automatic R: the largest, except for the table form at k = 7, whose
         // tables hold only 4 tentatives per CTA (200k reads of 150-5,000 bp at
         // t = 0.90: 3.7 s at 256 against 4.4 s at 1024; the bitmap form, on
@@ -250,10 +272,14 @@ size_t carve_all(char* base, int n, int64_t n_bytes, const Plan& P, bool drop, i
     B.amb = P.bits || P.masks ? c.take<Pair>((size_t)B.amb_cap) : nullptr;
     B.amb2 = P.bits || P.masks ? c.take<Pair>((size_t)B.amb_cap) : nullptr;
     B.amb_idx = P.bits || P.masks ? c.take<int32_t>(4 * (size_t)(kMaxBatch + 1)) : nullptr;
-    B.tmask_rwq = P.masks ? (P.r_max + 127) / 128 : 0;
+    R.hbuckets = P.hbuckets;
+    R.hrow = P.hbuckets ? c.take<uint4>((size_t)n * (P.hbuckets / 32)) : nullptr;
+    R.hextra = P.hbuckets ? c.take<int32_t>(n) : nullptr;
+    const bool tmasks = P.masks && !P.hbuckets;
+    B.tmask_rwq = tmasks ? (P.r_max + 127) / 128 : 0;
     B.tmask_planes = P.mask_planes;
-    B.tmask = P.masks ? c.take<uint4>(((size_t)1 << (2 * k)) * B.tmask_rwq) : nullptr;
-    B.tmask_ex = P.masks ? c.take<int32_t>(kMaxBatch) : nullptr;
+    B.tmask = tmasks ? c.take<uint4>(((size_t)1 << (2 * k)) * B.tmask_rwq) : nullptr;
+    B.tmask_ex = tmasks ? c.take<int32_t>(kMaxBatch) : nullptr;
     // word lengths 8..12: k-mer ids and counts apart, the global table, the
     // per-CTA hash scratch (slots: a power of two >= 2 x the longest read)
     const bool wide = !drop && k >= kWideK;
@@ -361,6 +387,7 @@ int Job::init(const gsdr_reads* reads, const gsdr_opts* opts_in, cudaStream_t s,
         P.idx_smem = false;
         P.bits = false;
         P.masks = false;
+        P.hbuckets = 0;
     }
     r_max_ = P.r_max;
     stats.batch = batched_ ? r_max_ : 1;
@@ -599,6 +626,10 @@ int Job::run(int pass_limit, const int32_t* resume) {
     if (!drop) {
         if (launch_kmers(R_, k, stream)) return fail(GSDR_EDEVICE, "k-mer kernel configuration");
         stats.kernel_launches += 1;
+        if (R_.hbuckets) {
+            launch_hash_rows(R_, stream);
+            stats.kernel_launches += 1;
+        }
         JCUDA(cudaGetLastError());
     }
     JCUDA(cudaEventRecord(ev_[2], stream));

@@ -78,6 +78,12 @@ struct DevReads {
     // max(count - 2, 0)
     uint32_t* kbits2;
     int32_t* kextra3;
+    // batched filter by hashed k-mer counts only (hbuckets 0 otherwise): per
+    // read a row of hbuckets 4-bit counts (hbuckets / 32 16-byte words) and
+    // the excess over 144 of its buckets' counts (rounds.cu, k_bfilter_hash)
+    uint4* hrow;
+    int32_t* hextra;
+    int32_t hbuckets;
     // pigeon filter (p 1; null otherwise), the reference's 4-mer position
     // index: pig[256 i + v] = inclusive prefix of read i's 4-mer bucket counts
     // (u16), pidx[off[i] + slot] = (u16) absolute position of a window's last
@@ -169,6 +175,9 @@ struct RoundState {
 void launch_pack(const DevReads& R, float t, int k, cudaStream_t s);
 // Distinct k-mers with multiplicities for every read.
 int launch_kmers(const DevReads& R, int k, cudaStream_t s);
+// The rows of the hashed k-mer count filter (after launch_kmers).
+void launch_hash_rows(const DevReads& R, cudaStream_t s);
+constexpr int kHashMinBuckets = 1024, kHashMaxBuckets = 2048;  // steps of 512
 // CTAs of the hash-based k-mer count (k >= 8): each owns R.khash_slots slots.
 constexpr int kHashCtas = 128;
 constexpr int kWideK = 8;  // word lengths from here on use the wide k-mer layout

@@ -302,6 +302,48 @@ int kmers_hist_launch(const DevReads& R, cudaStream_t s) {
     return 0;
 }
 
+// The rows of k_bfilter_hash (rounds.cu): one warp per read counts its k-mers
+// per bucket (16-bit halves in shared memory; a read holds at most 1,023) and
+// writes the counts as 4-bit E2M1 codes, rounded up.
+constexpr int kHashRowWarps = 8;
+__global__ void __launch_bounds__(32 * kHashRowWarps) k_hash_rows(DevReads R) {
+    __shared__ uint32_t cnt_all[kHashRowWarps][kHashMaxBuckets / 2];
+    const int lane = threadIdx.x & 31;
+    uint32_t* cnt = cnt_all[threadIdx.x >> 5];
+    const int H = R.hbuckets;
+    const int nw = gridDim.x * kHashRowWarps;
+    for (int r = blockIdx.x * kHashRowWarps + (threadIdx.x >> 5); r < R.n; r += nw) {
+        for (int i = lane; i < H / 2; i += 32) cnt[i] = 0;
+        __syncwarp();
+        const uint32_t* e = R.kmer + R.kmer_off[r];
+        const int ne = R.n_kmer[r];
+        for (int i = lane; i < ne; i += 32) {
+            const uint32_t v = __ldg(e + i);
+            // a multiplicative hash, its top 16 bits scaled to the buckets
+            const uint32_t b = (((v >> 16) * 0x9e3779b1u) >> 16) * (uint32_t)H >> 16;
+            atomicAdd(&cnt[b >> 1], (v & 0xffffu) << (16 * (b & 1)));
+        }
+        __syncwarp();
+        uint32_t* out = reinterpret_cast<uint32_t*>(R.hrow + (size_t)r * (H / 32));
+        int over = 0;
+        for (int w = lane; w < H / 8; w += 32) {
+            uint32_t o = 0;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const uint32_t n = (cnt[4 * w + (i >> 1)] >> (16 * (i & 1))) & 0xffffu;
+                // 1, 2, 3, 4, 6, 8 and 12 exist
+                const uint32_t code = n <= 4u ? n : n <= 6u ? 5u : n <= 8u ? 6u : 7u;
+                o |= code << (4 * i);
+                over += n > 144u ? (int)n - 144 : 0;
+            }
+            out[w] = o;
+        }
+        over = warp_sum(over);
+        if (lane == 0) R.hextra[r] = over;
+        __syncwarp();
+    }
+}
+
 }  // namespace
 
 int num_sms() {
@@ -443,6 +485,14 @@ __global__ void __launch_bounds__(kPigWarps * 32) k_pigeon_index(DevReads R) {
             __syncwarp();
         }
     }
+}
+
+void launch_hash_rows(const DevReads& R, cudaStream_t s) {
+    if (R.n <= 0 || !R.hbuckets) return;
+    int grid = (R.n + kHashRowWarps - 1) / kHashRowWarps;
+    const int cap = num_sms() * 6;
+    if (grid > cap) grid = cap;
+    k_hash_rows<<<grid, 32 * kHashRowWarps, 0, s>>>(R);
 }
 
 void launch_planes(const DevReads& R, cudaStream_t s) {

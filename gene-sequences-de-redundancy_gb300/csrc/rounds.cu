@@ -28,11 +28,13 @@
 // joins the first surviving tentative that accepted it.  That is exactly what
 // R consecutive reference rounds produce.
 //   k_bselect     next R unclustered indices from a forward cursor
-//   k_bfilter_tab / k_bfilter_idx / k_bfilter_bits / k_bfilter_mask (+ k_bexact_t)
+//   k_bfilter_tab / k_bfilter_idx / k_bfilter_bits / k_bfilter_hash /
+//   k_bfilter_mask (+ k_bexact_t)
 //                 prefilter + word filter of (tentative group, candidate):
 //                 transposed per-tentative tables, an inverted k-mer index,
-//                 k-mer count bitmaps or per-k-mer tentative masks (the last
-//                 two with exact sums for the pairs their bounds leave open);
+//                 k-mer count bitmaps, hashed k-mer counts or per-k-mer
+//                 tentative masks (the last three with exact sums for the pairs
+//                 their bounds leave open);
 //                 k_bprefilter in drop mode
 //   k_band, k_seg, k_align  as above, accepted pairs listed instead of applied
 //                 (k_band: a lane per pair, short reads with narrow bands)
@@ -1015,13 +1017,15 @@ struct CompactArgs {
     int seg_cap, acc_cap, amb_cap, drop;
 };
 
+constexpr int kCompactPer = 4;
+
 // Drops clustered reads from the remain list.  Batched: a candidate claimed in
 // this pass (k_bclaim) joins its tentative here.  The last block to finish
 // advances the round state (a launch of its own took about 4 us per round).
 template <bool BATCH>
 __global__ void __launch_bounds__(256) k_compact(RoundState* st, const int32_t* __restrict__ remain_in,
                                                  int32_t* __restrict__ remain_out, CompactArgs C) {
-    __shared__ int s_min, s_applied, s_last;
+    __shared__ int s_min, s_applied, s_base, s_warp[8];
     if (st->done) return;
     if (threadIdx.x == 0) {
         s_min = 0x7fffffff;
@@ -1034,32 +1038,56 @@ __global__ void __launch_bounds__(256) k_compact(RoundState* st, const int32_t* 
     const bool apply = BATCH && st->n_tent > 0 && !st->pair_overflow && !st->acc_overflow;
     int local_min = 0x7fffffff;
     unsigned applied = 0;
-    const int stride = gridDim.x * blockDim.x;
-    for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += stride) {
-        const int idx = base + lane;
-        int j = -1;
-        bool keep = false;
-        if (idx < n) {
-            j = remain_in[idx];
-            keep = C.cluster[j] == -1;
-            if (apply && keep) {
-                const uint32_t key = C.best[j];
-                if ((key >> 12) == pass) {
-                    C.cluster[j] = C.tent[4095u - (key & 0xfffu)];
-                    applied++;
-                    keep = false;
+    // a block takes kCompactPer x 256 entries at a time and reserves its output
+    // with one addition (one per warp and 32 entries, on one address, took
+    // most of the 23 us of a 900k-entry list)
+    constexpr int T = kCompactPer * 256;
+    for (int base = blockIdx.x * T; base < n; base += gridDim.x * T) {
+        int j[kCompactPer];
+        unsigned m[kCompactPer];
+        int mine = 0;  // kept entries of this warp
+#pragma unroll
+        for (int u = 0; u < kCompactPer; u++) {
+            const int idx = base + 256 * u + (int)threadIdx.x;
+            bool keep = false;
+            if (idx < n) {
+                j[u] = remain_in[idx];
+                keep = C.cluster[j[u]] == -1;
+                if (apply && keep) {
+                    const uint32_t key = C.best[j[u]];
+                    if ((key >> 12) == pass) {
+                        C.cluster[j[u]] = C.tent[4095u - (key & 0xfffu)];
+                        applied++;
+                        keep = false;
+                    }
                 }
             }
+            m[u] = __ballot_sync(kFull, keep);
+            mine += __popc(m[u]);
         }
-        const unsigned m = __ballot_sync(kFull, keep);
-        if (!m) continue;
-        int pos = 0;
-        if (lane == 0) pos = atomicAdd(&st->n_next, __popc(m));
-        pos = __shfl_sync(kFull, pos, 0);
-        if (keep) {
-            remain_out[pos + __popc(m & ((1u << lane) - 1u))] = j;
-            local_min = min(local_min, j);
+        if (lane == 0) s_warp[threadIdx.x >> 5] = mine;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int tot = 0;
+#pragma unroll
+            for (int w = 0; w < 8; w++) {
+                const int c = s_warp[w];
+                s_warp[w] = tot;
+                tot += c;
+            }
+            s_base = tot ? atomicAdd(&st->n_next, tot) : 0;
         }
+        __syncthreads();
+        int pos = s_base + s_warp[threadIdx.x >> 5];
+#pragma unroll
+        for (int u = 0; u < kCompactPer; u++) {
+            if ((m[u] >> lane) & 1u) {
+                remain_out[pos + __popc(m[u] & ((1u << lane) - 1u))] = j[u];
+                local_min = min(local_min, j[u]);
+            }
+            pos += __popc(m[u]);
+        }
+        __syncthreads();
     }
     if (!BATCH) {
         local_min = __reduce_min_sync(kFull, local_min);
@@ -1076,8 +1104,7 @@ __global__ void __launch_bounds__(256) k_compact(RoundState* st, const int32_t* 
             atomicAdd(&st->cnt_accepted, (unsigned long long)s_applied);
         }
         __threadfence();
-        s_last = atomicAdd(&st->ticket, 1) == (int)gridDim.x - 1;
-        if (s_last) {
+        if (atomicAdd(&st->ticket, 1) == (int)gridDim.x - 1) {
             __threadfence();
             st->ticket = 0;
             if (BATCH)
@@ -1477,13 +1504,12 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
                 const int buf = it & 1;
                 // (the first use of each accumulator passes at once)
                 ok = mbar_wait(&tempty[buf], ((it >> 1) & 1) ^ 1, limit, &s_quit);
-                tc_fence_after();
                 for (int c = 0; ok && c < CH; c++) {
                     ok = mbar_wait(&full[s], ph, limit, &s_quit);
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t a = smem_u32(stage0 + s * kBitsStageBytes);
-                    tc_mma_stage(tmem + buf * kTcMaxN, tmem, a, a + 128 * kTcRowBytes, idesc,
+                    const uint32_t a = tc_desc_lo(smem_u32(stage0 + s * kBitsStageBytes));
+                    tc_mma_stage(tmem + buf * kTcMaxN, tmem, a, a + 128 * kTcRowBytes / 16, idesc,
                                  c == 0);
                     tc_commit(&empty[s]);
                     if (++s == kBitsStages) s = 0, ph ^= 1;
@@ -1511,16 +1537,15 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
                 if (t0 == 0) bytes += kCandFixedBytes + 2ull * 16 * NQ;  // once per launch
             }
             const int buf = it & 1;
-            ok = mbar_wait(&tfull[buf], (it >> 1) & 1, limit, &s_quit);
-            if (!__all_sync(kFull, ok)) {
-                ok = false;
-                break;
-            }
+            ok = mbar_wait_warp(&tfull[buf], (it >> 1) & 1, limit, &s_quit);
+            if (!ok) break;
             tc_fence_after();
             const uint32_t addr = tmem + ((uint32_t)(warp & 3) << 21) + buf * kTcMaxN;
             for (int c0 = t0; c0 < t1; c0 += 16) {
+                uint32_t raw[16];
                 float v[16];
-                tc_load16(v, addr + (c0 - t0));
+                tc_load16(raw, addr + (c0 - t0));
+                tc_load_wait(raw, v);
                 // sixteen independent chains with no branch: which tentatives
                 // come before q and pass kernel_preFilter (func.cu:738-754),
                 // and which of those the bound does not reject
@@ -1626,7 +1651,7 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
         auto store = [&](const uint4 (&v)[kBitsRows]) {
 #pragma unroll
             for (int w = 0; w < 4; w++) {
-                ok = __all_sync(kFull, mbar_wait(&empty[s], ph, limit, &s_quit));
+                ok = mbar_wait_warp(&empty[s], ph, limit, &s_quit);
                 if (!ok) return;
                 uint8_t* base = stage0 + s * kBitsStageBytes + off0;
 #pragma unroll
@@ -2147,6 +2172,310 @@ __global__ void __launch_bounds__(1024, 1) k_bfilter_idx(
     }
 }
 
+// ---- word filter by hashed k-mer counts (short reads, sparse k-mer spaces) --
+//
+// A read's k-mers fall into H buckets by a hash; n(b) is the number of its
+// k-mers (with their multiplicities) in bucket b.  Since min(x, y) <= x y for
+// counts of at least one,
+//     S = sum over k-mers of min(c_t, c_q) <= sum over buckets of n_t n_q,
+// an entry of a matrix product again.  A row holds the counts as E2M1 values
+// (half the count: 1, 2, 3, 4, 6, 8 and 12 exist), rounded up, and 12 above 8.
+// That keeps the bound: where one of the two counts is at most 12 the product
+// of the stored ones is at least the smaller count, and where both are above
+// it is 144, so that
+//     S <= P + min(X_t, X_q),   X = sum over buckets of max(n - 144, 0).
+// A pair below its cutoff is rejected; the others go to k_bexact_t, which
+// forms S itself.  H is chosen per job (api.cu) so that unrelated reads rarely
+// reach the cutoff: P is about L^2 / H for reads of L k-mers.
+//
+// A CTA keeps the rows of its group of tentatives in shared memory for the
+// whole launch (up to 240 x H / 2 bytes) and streams tiles of 128 candidates
+// against them: four warps per stage copy rows with cp.async into a ring of
+// three 32 KB stages (512 buckets of 128 rows), one warp issues the MMAs, and
+// two teams of four warps, one per accumulator, compare the finished tiles' sums
+// with the rows' cutoffs while the next tile is summed in the other.
+//
+// 990k candidates x 1,024 tentatives, H = 1,536: 0.75 ms (1.35e12 pairs/s; the
+// masks 1.5 ms); 1M reads of 150 bp at t = 0.90 spend 127 ms in the filter stage
+// instead of 211.  An MMA (64 buckets) takes N / 2 cycles, and the MMAs alone
+// would take 0.36 ms; the MMA thread's wait for a stage adds about 200 cycles
+// that nothing covers (issuing blocks while the tensor pipe is busy), so a stage
+// holds eight MMAs.  On the way there, average of the first 249 passes (now 0.39
+// ms): 16 KB stages with eight warps on each 0.43 ms; an arrival per copying
+// thread 0.43; rows by TMA gathers of four 1.07 (67 cycles a gather); two warps
+// owning each 16 KB stage 0.41; the next stage's wait in the middle of the MMAs
+// 0.43; one team of four on the sums 0.43.
+constexpr int kHashEpilogue = 8;  // two teams of four, one per accumulator
+constexpr int kHashStages = 3;
+constexpr int kHashStepBuckets = 512;  // buckets per stage
+constexpr int kHashProducers = 4 * kHashStages;  // four warps per stage of the ring
+constexpr int kHashThreads = 32 * (1 + kHashEpilogue + kHashProducers);
+constexpr int kHashChunkBytes = 128 * kTcRowBytes;  // 256 buckets of 128 rows
+constexpr int kHashStageBytes = 2 * kHashChunkBytes;
+constexpr int kHashRowBytes = 125 * 1024;  // the tentatives' rows
+constexpr int kHashSmem = 1024 + kHashStages * kHashStageBytes + kHashRowBytes + 4 * kMaxBatch;
+
+// Tentatives per group for H buckets.
+__host__ __device__ __forceinline__ int hash_group(int buckets) {
+    const int n = (kHashRowBytes / (buckets / 2)) & ~15;
+    return n < kTcMaxN ? n : kTcMaxN;
+}
+
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool fill) {
+    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem),
+                 "r"(fill ? 16 : 0));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
+}
+
+__global__ void __launch_bounds__(kHashThreads, 1) k_bfilter_hash(
+    DevReads R, RoundState* st, const int32_t* __restrict__ remain,
+    const int32_t* __restrict__ tent, Pair* amb, int amb_cap) {
+    extern __shared__ __align__(1024) uint8_t hsm_raw[];
+    __shared__ uint64_t full[kHashStages], empty[kHashStages], tfull[2], tempty[2], drain;
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_quit;
+    if (st->done) return;
+    const int nt = st->n_tent;
+    if (nt == 0) return;
+    const int n = st->n_remain;
+    const int gmax = hash_group(R.hbuckets);
+    const int groups = (nt + gmax - 1) / gmax;
+    const int N = (((nt + groups - 1) / groups) + 15) & ~15;  // tentatives per group
+    const int step = max(1, (int)gridDim.x / groups);         // CTAs per group
+    const int mtiles = (n + 127) >> 7;
+    const int g = blockIdx.x % groups, m0 = blockIdx.x / groups;
+    if (m0 >= step || m0 >= mtiles) return;
+    const int t0 = g * N, t1 = min(nt, t0 + N);
+    const int CH = R.hbuckets / kHashStepBuckets;  // stages per tile
+    const int RQ = R.hbuckets >> 5;  // 16-byte pieces of a row
+    uint8_t* ring = reinterpret_cast<uint8_t*>(
+        (reinterpret_cast<uintptr_t>(hsm_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t* brow = ring + kHashStages * kHashStageBytes;
+    int32_t* s_tent = reinterpret_cast<int32_t*>(brow + kHashRowBytes);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kHashStages; i++) {
+            mbar_init(&full[i], kHashProducers / kHashStages);
+            mbar_init(&empty[i], 1);
+        }
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&tfull[i], 1);
+            mbar_init(&tempty[i], kHashEpilogue / 2);
+        }
+        mbar_init(&drain, 1);
+        s_quit = 0;
+        mbar_init_fence();
+    }
+    if (warp == 0) tmem_alloc_all(&s_tmem);
+    for (int t = threadIdx.x; t < nt; t += blockDim.x) s_tent[t] = tent[t];
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = s_tmem;
+    if (warp >= 1 && warp <= 4) tc_fill_scales(tmem, warp);
+    // the group's rows, chunk by chunk of 256 buckets (rows past the last
+    // tentative: read 0, whose sums are not looked at)
+    for (int i = threadIdx.x; i < N * RQ; i += blockDim.x) {
+        const int r = i / RQ, x = i - r * RQ, c = x >> 3, p = x & 7;
+        const int read = t0 + r < nt ? s_tent[t0 + r] : 0;
+        cp_async16(brow + (c * N + r) * kTcRowBytes + ((p ^ (r & 7)) << 4),
+                   R.hrow + (size_t)read * RQ + x, true);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const int limit = max(c_spin_limit, 1);
+    bool ok = true;  // this warp's waits all ended
+    if (warp == 0) {
+        if (lane == 0) {
+            const uint32_t idesc = tc_idesc_fp4(N);
+            const uint32_t a0 = tc_desc_lo(smem_u32(ring)), b0 = tc_desc_lo(smem_u32(brow));
+            int s = 0, it = 0;
+            uint32_t ph = 0;
+            for (int m = m0; ok && m < mtiles; m += step, it++) {
+                const int buf = it & 1;
+                // (the first use of each accumulator passes at once)
+                ok = mbar_wait(&tempty[buf], ((it >> 1) & 1) ^ 1, limit, &s_quit);
+                for (int c = 0; ok && c < CH; c++) {
+                    ok = mbar_wait(&full[s], ph, limit, &s_quit);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t a = a0 + s * (kHashStageBytes / 16);
+                    const uint32_t b = b0 + 2 * c * N * (kTcRowBytes / 16);
+                    tc_mma_stage(tmem + buf * kTcMaxN, tmem, a, b, idesc, c == 0);
+                    tc_mma_stage(tmem + buf * kTcMaxN, tmem, a + kHashChunkBytes / 16,
+                                 b + N * (kTcRowBytes / 16), idesc, false);
+                    tc_commit(&empty[s]);
+                    if (++s == kHashStages) s = 0, ph ^= 1;
+                }
+                if (ok) tc_commit(&tfull[buf]);
+            }
+        }
+    } else if (warp <= kHashEpilogue) {
+        const int row = (warp & 3) * 32 + lane, buf = (warp - 1) >> 2;
+        unsigned n_wf = 0;
+        unsigned long long n_pf = 0, bytes = 0;
+        uint32_t ph = 0;
+        const int first = m0 + buf * step;
+        int q = first * 128 + row < n ? remain[first * 128 + row] : -1;
+        int cw = q >= 0 ? R.cut_word[q] : 0, exq = q >= 0 ? R.hextra[q] : 0;
+        for (int m = first; m < mtiles; m += 2 * step, ph ^= 1) {
+            // this team's next row while its tile is summed
+            const int nidx = (m + 2 * step) * 128 + row;
+            const int nq = nidx < n ? remain[nidx] : -1;
+            ok = mbar_wait_warp(&tfull[buf], ph, limit, &s_quit);
+            if (!ok) break;
+            tc_fence_after();
+            const int ncw = nq >= 0 ? R.cut_word[nq] : 0, nexq = nq >= 0 ? R.hextra[nq] : 0;
+            // tentatives of the group before q (the list ascends)
+            int ntq = t1;
+            if (q <= s_tent[t1 - 1]) {
+                int lo = t0, hi = t1;
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (s_tent[mid] < q) lo = mid + 1;
+                    else hi = mid;
+                }
+                ntq = lo;
+            }
+            if (q >= 0) {
+                n_pf += (unsigned)(ntq - t0);
+                if (g == 0) bytes += kCandFixedBytes + 16ull * RQ;  // once per launch
+            }
+            __syncwarp();
+            // the row's cutoff in the accumulator's quarters; no pair of a row
+            // without a candidate reaches it
+            const float thr = q >= 0 && ntq > t0 ? 0.25f * (float)(cw - exq) : 3.0e38f;
+            const uint32_t addr = tmem + ((uint32_t)(warp & 3) << 21) + buf * kTcMaxN;
+            auto columns = [&](const float (&v)[16], int c0) {
+                float top = v[0];
+#pragma unroll
+                for (int j = 1; j < 16; j++) top = fmaxf(top, v[j]);
+                if (top >= thr) {
+                    uint32_t hit = 0;
+#pragma unroll
+                    for (int j = 0; j < 16; j++) hit |= v[j] >= thr ? 1u << j : 0u;
+                    if (c0 + 16 > ntq) hit &= ntq > c0 ? (1u << (ntq - c0)) - 1u : 0u;
+                    const int4 cq = R.comp[q];
+                    const int cbq = R.cut_base[q] - R.strict;
+                    while (hit) {
+                        const int j = __ffs(hit) - 1;
+                        hit &= hit - 1;
+                        const int rep = s_tent[c0 + j];
+                        if (exq > 0) {
+                            float vj = v[0];
+#pragma unroll
+                            for (int i = 1; i < 16; i++) vj = j == i ? v[i] : vj;
+                            if (4.0f * vj + (float)min(R.hextra[rep], exq) < (float)cw) continue;
+                        }
+                        n_wf++;
+                        // the composition bound (kernel_preFilter, func.cu:738-754)
+                        if (!prefilter_pass(R.comp[rep], cq, cbq)) continue;
+                        const int slot = atomicAdd(&st->n_amb, 1);
+                        if (slot < amb_cap) amb[slot] = Pair{rep, q};
+                        else st->pair_overflow = 1;
+                    }
+                }
+                __syncwarp();
+            };
+            // sixteen columns at a time, the next sixteen on their way
+            uint32_t ra[16], rb[16];
+            float v[16];
+            tc_load16(ra, addr);
+            for (int c0 = t0; c0 < t1; c0 += 32) {
+                tc_load_wait(ra, v);
+                if (c0 + 16 < t1) tc_load16(rb, addr + (c0 + 16 - t0));
+                columns(v, c0);
+                if (c0 + 16 >= t1) break;
+                tc_load_wait(rb, v);
+                if (c0 + 32 < t1) tc_load16(ra, addr + (c0 + 32 - t0));
+                columns(v, c0 + 16);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tempty[buf]);
+            q = nq;
+            cw = ncw;
+            exq = nexq;
+        }
+        n_wf = (unsigned)warp_sum_i((int)n_wf);
+        n_pf = warp_sum_ull(n_pf);
+        bytes = warp_sum_ull(bytes);
+        if (lane == 0) {
+            if (n_pf) atomicAdd(&st->cnt_prefilter, n_pf);
+            if (n_wf) atomicAdd(&st->cnt_word, (unsigned long long)n_wf);
+            if (bytes) atomicAdd(&st->filter_bytes, bytes);
+        }
+    } else {
+        // producers: a warp owns a quarter of the rows of one stage of the
+        // ring, so the stages' copies run independently and a stage is handed
+        // over the moment its own have landed.  Lane piece p of rows 4 k + lane
+        // / 8 of the quarter, both chunks.
+        const int w = warp - 1 - kHashEpilogue;
+        const int s = w % kHashStages, quarter = w / kHashStages;
+        const int p = lane & 7, r0 = quarter * 32 + (lane >> 3);
+        const int off0 = r0 * kTcRowBytes + ((p ^ (r0 & 7)) << 4);
+        const int odd = ((p ^ ((r0 + 4) & 7)) << 4) - ((p ^ (r0 & 7)) << 4);
+        uint8_t* d = ring + s * kHashStageBytes + off0;
+        const int total = (mtiles - m0 + step - 1) / step * CH;
+        constexpr int KR = 8;  // rows per lane: 32, four at a time
+        int idx[KR];
+        auto rows_of = [&](int i) {
+            const int m = m0 + i / CH * step;
+#pragma unroll
+            for (int k = 0; k < KR; k++) {
+                const int x = m * 128 + r0 + 4 * k;
+                idx[k] = i < total && x < n ? remain[x] : 0;
+            }
+        };
+        rows_of(s);
+        uint32_t ph = 1;  // the first round of stages is free
+        for (int i = s; i < total; i += kHashStages, ph ^= 1) {
+            ok = mbar_wait_warp(&empty[s], ph, limit, &s_quit);
+            if (!ok) break;
+            const uint4* src = R.hrow + 16 * (i % CH) + p;
+#pragma unroll
+            for (int k = 0; k < KR; k++) {
+                const uint4* r = src + (size_t)idx[k] * RQ;
+                uint8_t* to = d + 4 * k * kTcRowBytes + (k & 1 ? odd : 0);
+                cp_async16(to, r, true);
+                cp_async16(to + kHashChunkBytes, r + 8, true);
+            }
+            cp_async_commit();
+            rows_of(i + kHashStages);
+            cp_async_wait<0>();
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[s]);
+        }
+    }
+    if (!ok) {
+        // a wait gave up: the others stop at their next poll
+        s_quit = 1;
+        st->error = 1;
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        if (s_quit && lane == 0) {
+            // the MMAs in flight, before the accumulators are given back
+            const int none = 0;
+            tc_commit(&drain);
+            mbar_wait(&drain, 0, kSpinLimit, &none);
+        }
+        __syncwarp();
+        tmem_free_all(tmem);
+    }
+}
+
 // ---- word filter by tentative masks (short reads, sparse k-mer spaces) ----
 //
 // Per pass, for every k-mer m a row of R_max bits, bit t set iff tentative t
@@ -2269,17 +2598,6 @@ struct MaskCounts {
 // in flight hold no registers).
 constexpr int kMaskStages = 3;
 constexpr int kMaskStepBytes = 8 * 32 * 16;  // one step: 8 words of 16 bytes per lane
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool fill) {
-    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem),
-                 "r"(fill ? 16 : 0));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
 
 // Rows of 16-byte words: lane (g, x) of a warp, g = lane / LPR, x = lane %
 // LPR, works for candidate g of the warp's 32 / LPR consecutive candidates
@@ -2831,6 +3149,20 @@ void launch_bfilter_bits_t(const DevReads& R, RoundBuffers& B, const int32_t* re
 }
 
 template <int K>
+void launch_bfilter_hash_t(const DevReads& R, RoundBuffers& B, const int32_t* remain,
+                           cudaStream_t s) {
+    static bool attr = false;
+    if (!attr) {
+        cudaFuncSetAttribute(k_bfilter_hash, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kHashSmem);
+        attr = true;
+    }
+    k_bfilter_hash<<<num_sms(), kHashThreads, kHashSmem, s>>>(R, B.st, remain, B.tent, B.amb,
+                                                              B.amb_cap);
+    launch_exact_t<K>(R, B, s);
+}
+
+template <int K>
 void launch_bfilter_mask_t(const DevReads& R, RoundBuffers& B, const int32_t* remain,
                            cudaStream_t s) {
     static int grid8 = 0, grid10 = 0;
@@ -2866,6 +3198,15 @@ void launch_filter_any(const DevReads& R, RoundBuffers& B, const int32_t* remain
         k_gtab<<<64, 256, 0, s>>>(R, B.st, 0);
         k_filter_g<<<shaped(grid, R.filter_blocks), kFilterThreads, 0, s>>>(R, B.st, remain, B.pairs, B.seg_cap);
         k_gtab<<<64, 256, 0, s>>>(R, B.st, 1);
+        return;
+    }
+    if (BATCH && !drop && R.hbuckets) {
+        switch (R.k) {
+            case 4: launch_bfilter_hash_t<4>(R, B, remain, s); break;
+            case 5: launch_bfilter_hash_t<5>(R, B, remain, s); break;
+            case 6: launch_bfilter_hash_t<6>(R, B, remain, s); break;
+            default: launch_bfilter_hash_t<7>(R, B, remain, s); break;
+        }
         return;
     }
     if (BATCH && !drop && B.tmask) {

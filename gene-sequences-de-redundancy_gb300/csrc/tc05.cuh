@@ -50,6 +50,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int li
     return false;
 }
 
+// The same by a whole warp.  (Every lane polls: one lane polling for the others
+// adds its divergence to each hand-over, and took half again as long.)
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int limit,
+                                               const volatile int* quit) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit, quit)) != 0;
+}
+
 // All 512 columns of the SM's tensor memory (one CTA per SM: the kernels that
 // use it hold most of the shared memory), by one whole warp.
 __device__ __forceinline__ void tmem_alloc_all(uint32_t* dst) {
@@ -67,7 +74,9 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// shared-memory writes of this thread become visible to the tensor core
+// Shared-memory writes of this thread (its completed cp.async copies too) are
+// ordered before the MMAs of whoever observes its next arrival.  (It may also
+// wait for the thread's loads in flight: issue loads for later stages behind it.)
 __device__ __forceinline__ void fence_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
@@ -75,10 +84,11 @@ __device__ __forceinline__ void fence_async_smem() {
 // Descriptor of a K-major operand tile in shared memory: rows of 128 bytes,
 // 16-byte pieces xor-swizzled by the row's low three bits, eight rows per
 // 1,024-byte group (1,024-byte aligned).
-__device__ __forceinline__ uint64_t tc_desc(uint32_t addr) {
-    return (uint64_t)((addr & 0x3ffffu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)64 << 32) |
-           ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+// The low half moves with the address; the upper is the same for every tile.
+__device__ __forceinline__ uint32_t tc_desc_lo(uint32_t addr) {
+    return ((addr & 0x3ffffu) >> 4) | (1u << 16);
 }
+constexpr uint32_t kTcDescHi = 64u | (1u << 14) | (2u << 29);
 constexpr int kTcRowBytes = 128;  // 256 E2M1 values
 // D[128][n] += A[128][64] B[n][64]^T, E2M1 x E2M1 -> f32
 __device__ __forceinline__ uint32_t tc_idesc_fp4(int n) {
@@ -96,22 +106,25 @@ __device__ __forceinline__ void tc_fill_scales(uint32_t tmem, int warp) {
                      "r"(0x7f7f7f7fu));
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
-// The four MMAs of one 128-byte-wide stage (one thread).
+// The four MMAs of one 128-byte-wide stage (one thread).  a and b: tc_desc_lo
+// of the stage's operands; first: the sums start from zero.
 __device__ __forceinline__ void tc_mma_stage(uint32_t d, uint32_t tmem, uint32_t a, uint32_t b,
                                              uint32_t idesc, bool first) {
-    const uint64_t da = tc_desc(a), db = tc_desc(b);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const uint32_t acc = first && k == 0 ? 0u : 1u;
         asm volatile(
             "{\n\t"
             ".reg .pred p;\n\t"
+            ".reg .b64 da, db;\n\t"
             "setp.ne.u32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, "
+            "mov.b64 da, {%1, %7};\n\t"
+            "mov.b64 db, {%2, %7};\n\t"
+            "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], da, db, %3, "
             "[%5], [%6], p;\n\t"
             "}" ::"r"(d),
-            "l"(da + 2 * k), "l"(db + 2 * k), "r"(idesc), "r"(acc), "r"(tmem + kTcScaleA),
-            "r"(tmem + kTcScaleB)
+            "r"(a + 2 * k), "r"(b + 2 * k), "r"(idesc), "r"(acc), "r"(tmem + kTcScaleA),
+            "r"(tmem + kTcScaleB), "r"(kTcDescHi)
             : "memory");
     }
 }
@@ -123,9 +136,9 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
         : "memory");
 }
 // Sixteen accumulator columns of this lane's row (a whole warp; warp % 4 is
-// the quarter of the lanes it may read).
-__device__ __forceinline__ void tc_load16(float (&v)[16], uint32_t addr) {
-    uint32_t r[16];
+// the quarter of the lanes it may read); the values are there after
+// tc_load_wait.
+__device__ __forceinline__ void tc_load16(uint32_t (&r)[16], uint32_t addr) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
         "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -133,7 +146,14 @@ __device__ __forceinline__ void tc_load16(float (&v)[16], uint32_t addr) {
           "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
           "=r"(r[14]), "=r"(r[15])
         : "r"(addr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// Waits for this warp's loads; the values pass through so that no use moves
+// ahead of it.
+__device__ __forceinline__ void tc_load_wait(uint32_t (&r)[16], float (&v)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]),
+                   "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]),
+                   "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
