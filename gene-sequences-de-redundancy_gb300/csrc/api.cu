@@ -439,7 +439,10 @@ int Job::init(const gsdr_reads* reads, const gsdr_opts* opts_in, cudaStream_t s,
             R_.group_max_w = std::min(std::max(std::atoi(gw), 0), kSegMaxWords);
     R_.band_few = R_.group_max_w > 0 ? kBandFew : 0;
     // a window holds at most the longest read's rows
-    R_.wide = (P.max_len + 31) / 32 > R_.group_max_w ? 1 : 0;
+    const int64_t widest = (P.max_len + 31) / 32;
+    R_.wide = widest <= R_.group_max_w                                        ? 0
+              : R_.group_max_w == kSegMaxWords && widest <= kSegWideWords ? 1
+                                                                              : 2;
     refoff16_.swap(P.refoff16);
     pack_off_.swap(P.pack_off);
     kmer_off_.swap(P.kmer_off);
@@ -922,6 +925,7 @@ int Job::lcs_pairs(const int32_t* pat, const int32_t* txt, int n_pairs, int mapp
             if (T > 0 && cb > 0 && q >= cb && T >= cb) {
                 const int sw = seg_words(T, q, cb, kSegSteps32);
                 if (sw <= kSegMaxWords) c = seg_class(sw);
+                else if (sw <= kSegWideWords) c = kWideClass;
             }
         }
         if (greedy) {
@@ -949,7 +953,7 @@ int Job::lcs_pairs(const int32_t* pat, const int32_t* txt, int n_pairs, int mapp
     JCUDA(cudaMemsetAsync(B_.cluster, 0xff, sizeof(int32_t) * n, stream));
     JCUDA(cudaMemsetAsync(B_.tidx, 0xff, sizeof(uint32_t) * n, stream));
     JCUDA(cudaEventRecord(ev_[2], stream));
-    R_.wide = 1;      // the queues above fill the systolic classes too
+    R_.wide = 2;      // the queues above fill the systolic classes too
     R_.band_few = 0;  // and the lane-banded ones run on their own kernel
     launch_align_stage(R_, B_, mapping >= 1, stream);
     JCUDA(cudaGetLastError());

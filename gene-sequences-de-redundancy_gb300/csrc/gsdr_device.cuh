@@ -27,7 +27,8 @@ constexpr int64_t kMaxReadBases = 1ll << 24;  // longest read (raw bases) a job 
 constexpr int kBandClasses = 2;         // window classes (4, 8 words) of the lane-banded kernel
 constexpr int kSegClasses = 5;          // window classes of the segment kernel (seg_class)
 constexpr int kNarrowClass = kSysClasses + kBandClasses + kSegClasses;  // its narrow runs
-constexpr int kAlignClasses = kNarrowClass + 1;  // alignment queues
+constexpr int kWideClass = kNarrowClass + 1;  // its widest windows (up to kSegWideWords)
+constexpr int kAlignClasses = kWideClass + 1;  // alignment queues
 constexpr int kSingleWorkSlot = kAlignClasses;  // work counter of the merged single-warp systolic classes
 
 // Segment-kernel class of a window of at most kSegMaxWords words.
@@ -116,8 +117,8 @@ struct DevReads {
     // widest window (words) given to the segment kernel (kSegMaxWords; 0:
     // none, those pairs go to the systolic kernels)
     int32_t group_max_w;
-    // 1: some pair may need a wider window than that, so passes also launch
-    // the systolic kernels
+    // some pair may need a wider window than that: 1, passes also launch the
+    // segment kernel's wide form; 2, the systolic kernels too
     int32_t wide;
     // semantics (gsdr_opts::variant): 1 = the SYCL program's.  brk (variant 1
     // with filters, null otherwise): bit g of read i (word pack_off[i] + g/32)

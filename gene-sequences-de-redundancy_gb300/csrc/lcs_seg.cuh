@@ -49,15 +49,22 @@ namespace gsdr {
 
 constexpr int kSegMaxW = 16;        // words per lane
 constexpr int kSegMaxWords = 32 * kSegMaxW;  // widest window (512 words, 16,384 rows)
-constexpr int kSegSteps8 = 128;     // steps per segment, G = 8 and 16
-constexpr int kSegSteps32 = 256;    // G = 32 (the array takes G steps to fill and drain)
-constexpr int kSegNoBase = 4 * kSegMaxW * 32;  // table offset of the all-zero rows
-constexpr int kSegPeqWords = 5 * kSegMaxW * 32;
-constexpr int kSegVWords = kSegMaxWords + kSegMaxWords / 16;  // padded, seg_vidx
+constexpr int kSegWideW = 24;       // the same of the wide form (768 words, a warp per pair)
+constexpr int kSegWideWords = 32 * kSegWideW;
+constexpr int kSegSteps8 = 128;     // steps per segment, G = 8
+constexpr int kSegSteps32 = 256;    // G = 16 and 32 (the array takes G steps to fill and drain)
 // code entries per warp: groups x (leading G, S, trailing G)
 constexpr int kSegCodes = 4 * (kSegSteps8 + 2 * 8);
-static_assert(kSegCodes >= 2 * (kSegSteps8 + 2 * 16) && kSegCodes >= kSegSteps32 + 2 * 32, "codes");
-constexpr int kSegWarpWords = kSegPeqWords + kSegVWords + kSegCodes / 2;  // u32 per warp
+static_assert(kSegCodes >= 2 * (kSegSteps32 + 2 * 16) && kSegCodes >= kSegSteps32 + 2 * 32, "codes");
+// A warp's shared memory for up to M words per lane: the match masks and the
+// all-zero rows behind them, V between segments (padded, seg_vidx), the codes.
+template <int M>
+struct SegSmem {
+    static constexpr int kNoBase = 4 * M * 32;  // table offset of the all-zero rows
+    static constexpr int kPeq = 5 * M * 32;
+    static constexpr int kV = 32 * M + 2 * M;
+    static constexpr int kWords = kPeq + kV + kSegCodes / 2;  // u32
+};
 
 // Words of the widest window a pair can need (segments of S steps).
 __host__ __device__ __forceinline__ int seg_words(int T, int q, int c, int S) {
@@ -92,19 +99,48 @@ __host__ __device__ __forceinline__ bool seg_narrow(int T, int q, int c, int wor
 
 __device__ __forceinline__ int seg_vidx(int k) { return k + (k >> 4); }
 
-// Steps over the codes at e (one u16 table offset per step) on W words.
+// The match masks of a window: rows of 32 * W words per base code, then the
+// all-zero rows (SegSmem).  W a multiple of four: [code][W / 4][lane][4], one
+// 16-byte load per four words (a quarter of the load instructions); otherwise
+// [code][W][lane].  A lane's column starts at seg_lane<W>(lane); neither form has
+// bank conflicts, whatever rows the lanes are at.
+template <int W>
+__device__ __forceinline__ int seg_lane(int lane) {
+    return W % 4 == 0 ? 4 * lane : lane;
+}
+
+// Steps over the codes at e (one u16 table offset per step) on W words.  The
+// loop is unrolled only as far as its instructions stay near the scheduler's
+// instruction buffer: with 8 and 4 steps per iteration a third of the stalls
+// were for instructions (2-30 kbp reads: alignment 182 -> 153 ms).
 template <int W>
 __device__ __forceinline__ void seg_steps(const uint16_t* __restrict__ e,
                                           const uint32_t* __restrict__ peq, uint32_t (&V)[W],
                                           uint32_t en, int nsteps) {
     uint32_t from = 0;
-    constexpr int U = W <= 8 ? 8 : 4;
+    constexpr int U = W <= 4 ? 8 : W <= 8 ? 4 : 2;
 #pragma unroll 1
     for (int s = 0; s < nsteps; s += U) {
 #pragma unroll
         for (int k = 0; k < U; k++) {
             uint32_t cin = from;
-            peq_step<W>(V, peq + e[s + k], cin, en);
+            const uint32_t* pm = peq + e[s + k];
+            if constexpr (W % 4 == 0) {
+#pragma unroll
+                for (int i = 0; i < W; i += 4) {
+                    const uint4 m = *reinterpret_cast<const uint4*>(pm + 32 * i);
+                    uint32_t t0, t1, t2, t3;
+                    add4_carry_en(t0, t1, t2, t3, V[i], V[i + 1], V[i + 2], V[i + 3], V[i] & m.x,
+                                  V[i + 1] & m.y, V[i + 2] & m.z, V[i + 3] & m.w, cin,
+                                  i == 0 ? en : 0xffffffffu);
+                    V[i] = t0 | (V[i] & ~m.x);
+                    V[i + 1] = t1 | (V[i + 1] & ~m.y);
+                    V[i + 2] = t2 | (V[i + 2] & ~m.z);
+                    V[i + 3] = t3 | (V[i + 3] & ~m.w);
+                }
+            } else {
+                peq_step<W>(V, pm, cin, en);
+            }
             from = __shfl_up_sync(0xffffffffu, cin, 1);
         }
     }
@@ -146,21 +182,41 @@ __device__ __forceinline__ void seg_start(SegPair& P, int S, bool narrow) {
 // lane of a busy group -1 (go on), 1 (accept) or 0 (reject; with narrow set:
 // not accepted).  peq / vb / codes: the warp's shared memory, vb and codes
 // already offset to the group.
-template <int W>
+template <int W, int M>
 __device__ __forceinline__ int seg_segment(SegPair& P, uint32_t* peq, uint32_t* vb,
                                            uint16_t* codes, int G, int S, int lane, int& steps) {
+    constexpr uint32_t kNoBase = SegSmem<M>::kNoBase;
     const int j = lane & (G - 1);
-    peq += lane;
+    peq += seg_lane<W>(lane);
     uint32_t V[W];
     const int wb = P.w_lo + j * W;
     const int nwT = (P.T + 31) >> 5;
     // the window's match masks: the text's bit planes are the masks
+    if constexpr (W % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < W; i += 4) {
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                uint32_t m[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    m[u] = P.busy && wb + i + u < nwT
+                               ? __ldg(P.planes + c * P.stride + wb + i + u) : 0u;
+                *reinterpret_cast<uint4*>(peq + (c * W + i) * 32) =
+                    make_uint4(m[0], m[1], m[2], m[3]);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < W; i++) {
+            const bool in = P.busy && wb + i < nwT;
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                peq[(c * W + i) * 32] = in ? __ldg(P.planes + c * P.stride + wb + i) : 0u;
+        }
+    }
 #pragma unroll
     for (int i = 0; i < W; i++) {
-        const bool in = P.busy && wb + i < nwT;
-#pragma unroll
-        for (int c = 0; c < 4; c++)
-            peq[(c * W + i) * 32] = in ? __ldg(P.planes + c * P.stride + wb + i) : 0u;
         const int k = wb + i - P.w_prev;
         V[i] = k < P.keep ? vb[seg_vidx(k)] : 0xffffffffu;
     }
@@ -170,9 +226,9 @@ __device__ __forceinline__ int seg_segment(SegPair& P, uint32_t* peq, uint32_t* 
         uint32_t* d = reinterpret_cast<uint32_t*>(codes + G + 16 * w);
 #pragma unroll
         for (int t = 0; t < 16; t += 2) {
-            const uint32_t a = 16 * w + t < left ? ((v >> (30 - 2 * t)) & 3u) * (32u * W) : kSegNoBase;
+            const uint32_t a = 16 * w + t < left ? ((v >> (30 - 2 * t)) & 3u) * (32u * W) : kNoBase;
             const uint32_t b =
-                16 * w + t + 1 < left ? ((v >> (28 - 2 * t)) & 3u) * (32u * W) : kSegNoBase;
+                16 * w + t + 1 < left ? ((v >> (28 - 2 * t)) & 3u) * (32u * W) : kNoBase;
             d[t >> 1] = a | (b << 16);
         }
     }
@@ -228,29 +284,34 @@ __device__ __forceinline__ int seg_segment(SegPair& P, uint32_t* peq, uint32_t* 
     return -1;
 }
 
-// One segment at the words per lane the warp's widest window needs.
+// One segment at the words per lane the warp's widest window needs (at most M).
+template <int M>
 __device__ __forceinline__ int seg_dispatch(SegPair& P, int wl, uint32_t* peq, uint32_t* vb,
                                             uint16_t* codes, int G, int S, int lane,
                                             int& steps) {
+    if constexpr (M > 16) {
+        if (wl > 20) return seg_segment<24, M>(P, peq, vb, codes, G, S, lane, steps);
+        if (wl > 16) return seg_segment<20, M>(P, peq, vb, codes, G, S, lane, steps);
+    }
     switch (wl) {
-        case 1: return seg_segment<1>(P, peq, vb, codes, G, S, lane, steps);
-        case 2: return seg_segment<2>(P, peq, vb, codes, G, S, lane, steps);
-        case 3: return seg_segment<3>(P, peq, vb, codes, G, S, lane, steps);
-        case 4: return seg_segment<4>(P, peq, vb, codes, G, S, lane, steps);
-        case 5: return seg_segment<5>(P, peq, vb, codes, G, S, lane, steps);
-        case 6: return seg_segment<6>(P, peq, vb, codes, G, S, lane, steps);
+        case 1: return seg_segment<1, M>(P, peq, vb, codes, G, S, lane, steps);
+        case 2: return seg_segment<2, M>(P, peq, vb, codes, G, S, lane, steps);
+        case 3: return seg_segment<3, M>(P, peq, vb, codes, G, S, lane, steps);
+        case 4: return seg_segment<4, M>(P, peq, vb, codes, G, S, lane, steps);
+        case 5: return seg_segment<5, M>(P, peq, vb, codes, G, S, lane, steps);
+        case 6: return seg_segment<6, M>(P, peq, vb, codes, G, S, lane, steps);
         case 7:
-        case 8: return seg_segment<8>(P, peq, vb, codes, G, S, lane, steps);
+        case 8: return seg_segment<8, M>(P, peq, vb, codes, G, S, lane, steps);
         case 9:
-        case 10: return seg_segment<10>(P, peq, vb, codes, G, S, lane, steps);
+        case 10:
         case 11:
-        case 12: return seg_segment<12>(P, peq, vb, codes, G, S, lane, steps);
-        default: return seg_segment<16>(P, peq, vb, codes, G, S, lane, steps);
+        case 12: return seg_segment<12, M>(P, peq, vb, codes, G, S, lane, steps);
+        default: return seg_segment<16, M>(P, peq, vb, codes, G, S, lane, steps);
     }
 }
 // ... and the cells they step are counted at the same words.
 __device__ __forceinline__ int seg_tile(int wl) {
-    return wl <= 6 ? wl : wl <= 8 ? 8 : wl <= 10 ? 10 : wl <= 12 ? 12 : 16;
+    return wl <= 6 ? wl : wl <= 8 ? 8 : (wl + 3) & ~3;
 }
 
 }  // namespace gsdr

@@ -165,7 +165,7 @@ extern "C" int gsdr_lcs_decide_noalloc(const uint32_t* d_packed, const int64_t* 
     R.pack_off = d_pack_off;
     R.packed = const_cast<uint32_t*>(d_packed);
     R.cut_base = reinterpret_cast<int32_t*>(base + kOffCut);
-    R.wide = 1;  // packed sequences only: the systolic kernels decide every pair
+    R.wide = 2;  // packed sequences only: the systolic kernels decide every pair
     RoundBuffers B = {};
     B.st = reinterpret_cast<RoundState*>(base + kOffState);
     B.pairs = reinterpret_cast<Pair*>(base + kOffPairs);

@@ -89,6 +89,14 @@ __device__ __forceinline__ int align_class(int words) {
                          : words <= kMaxPatternWords ? 6 : kLongClass;
 }
 
+// Queue of a pair whose full window takes `words` words: the segment kernel's
+// class, its wide form's, or the systolic length class of the pattern.
+__device__ __forceinline__ int full_class(int words, int q, int seg_max_w) {
+    if (words <= seg_max_w) return seg_class(words);
+    if (seg_max_w == kSegMaxWords && words <= kSegWideWords) return kWideClass;
+    return align_class((q + 31) >> 5);
+}
+
 // Queue of a pair: a band class (windows of 4 and 8 words) when its band fits
 // and its serial work (text bases x window words: a lane works through its
 // pair alone, and a longer one would hold up its pass) stays below
@@ -105,7 +113,7 @@ __device__ __forceinline__ int pair_class(int T, int q, int c, int band_max_w,
         }
         const int sw = seg_words(T, q, c, kSegSteps32);
         if (seg_max_w > 0 && seg_narrow(T, q, c, sw)) return kNarrowClass;
-        if (sw <= seg_max_w) return seg_class(sw);
+        return full_class(sw, q, seg_max_w);
     } else if (seg_max_w > 0) {
         return seg_class(1);
     }
@@ -691,9 +699,16 @@ __global__ void __launch_bounds__(kAlignThreads) k_band(DevReads R, RoundState* 
 // t = 0.95 40.6 -> 20.9 ms (3.36e12 -> 1.67e12 cells), 3k reads of 2-30 kbp at
 // t = 0.80 420 -> 199 ms, 30k reads of 150-5,000 bp at t = 0.90 60 -> 34 ms
 // (most of its passes hold few pairs: latency), 1k such reads at t = 0.95
-// 2.66 -> 1.44 ms.
+// 2.66 -> 1.44 ms.  With the narrow runs, the wide form, short step loops and
+// 256 steps per segment for G = 16 (they fill and drain half as often): 13.6,
+// 116, 5.8 and 0.87 ms; 147 TCUPS stepped on the long reads, of 197 at three
+// ALU operations per 32 cells.
 //
-// NARROW: the pairs of the narrow class on their strip (8 lanes a pair, or a
+// MODE kSegWide: the pairs of the wide class, a warp each with up to 24 words
+// per lane (half the warps per SM: the masks take 15 KB a warp).  They ran on
+// four or eight warps of k_align, whose bits are the whole pattern: 7,400 pairs
+// of 3k reads of 2-30 kbp took 53 ms there, 17 here.
+// MODE kSegNarrow: the pairs of the narrow class on their strip (8 lanes a pair, or a
 // warp), launched first; a pair it does not accept goes to the queue of its
 // full window behind it.  It took the place of a greedy walk with one thread
 // per pair, whose longest walk (up to 4,096 dependent steps) held up every
@@ -701,16 +716,27 @@ __global__ void __launch_bounds__(kAlignThreads) k_band(DevReads R, RoundState* 
 // on: alignment stage 20.9 -> 18.2 ms (200k reads of 300-10,000 bp), 34 -> 16.7
 // ms (30k reads of 150-5,000 bp, t = 0.90, 92 passes), 29.6 -> 15.0 ms (100k
 // such reads, t = 0.95, 103 passes), 2.9 -> 1.05 ms (10k reads, 14 passes).
-template <bool BATCH, bool NARROW>
-__global__ void __launch_bounds__(kAlignThreads, 2) k_seg(DevReads R, RoundState* st,
-                                                          AlignArgs A) {
-    extern __shared__ __align__(16) uint32_t seg_sm[];  // kSegWarpWords per warp
+constexpr int kSegFull = 0, kSegNarrow = 1, kSegWide = 2;
+template <int MODE>
+constexpr int kSegModeW = MODE == kSegWide ? kSegWideW : kSegMaxW;
+
+template <bool BATCH, int MODE>
+__global__ void __launch_bounds__(kAlignThreads, MODE == kSegWide ? 1 : 2) k_seg(DevReads R,
+                                                                                RoundState* st,
+                                                                                AlignArgs A) {
+    constexpr bool NARROW = MODE == kSegNarrow;
+    constexpr int M = kSegModeW<MODE>;
+    using L = SegSmem<M>;
+    extern __shared__ __align__(16) uint32_t seg_sm[];  // L::kWords per warp
     if (st->done) return;
     if (BATCH && (st->pair_overflow || st->n_tent == 0)) return;
-    constexpr int c0 = NARROW ? kNarrowClass : kSysClasses + kBandClasses;
-    constexpr int nc = NARROW ? 1 : kSegClasses;
+    constexpr int c0 = MODE == kSegNarrow ? kNarrowClass
+                       : MODE == kSegWide ? kWideClass
+                                          : kSysClasses + kBandClasses;
+    constexpr int nc = MODE == kSegFull ? kSegClasses : 1;
     // the lane-banded classes' pairs too when they are few (k_band)
-    const int first = !NARROW && BATCH && band_pairs(st) <= R.band_few ? -kBandClasses : 0;
+    const int first =
+        MODE == kSegFull && BATCH && band_pairs(st) <= R.band_few ? -kBandClasses : 0;
     int total = 0;
     for (int c = first; c < nc; c++) total += min(st->n_pairs[c0 + c], A.seg_cap);
     if (total <= 0) return;
@@ -718,21 +744,21 @@ __global__ void __launch_bounds__(kAlignThreads, 2) k_seg(DevReads R, RoundState
     const int pass = BATCH ? st->pass : 0;
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
-    uint32_t* peq = seg_sm + (threadIdx.x >> 5) * kSegWarpWords;
-    for (int i = lane; i < kSegMaxW * 32; i += 32) peq[kSegNoBase + i] = 0u;
+    uint32_t* peq = seg_sm + (threadIdx.x >> 5) * L::kWords;
+    for (int i = lane; i < M * 32; i += 32) peq[L::kNoBase + i] = 0u;
     unsigned long long cells = 0, done = 0;
     unsigned acc = 0;
     for (int cls = nc - 1; cls >= first; cls--) {
         const int np = min(st->n_pairs[c0 + cls], A.seg_cap);
         if (np <= 0) continue;
-        const int G = alone || cls == 4 ? 32 : cls == 3 ? 16 : 8;
-        const int S = G == 32 && !NARROW ? kSegSteps32 : kSegSteps8;
+        const int G = MODE == kSegWide || alone || cls == 4 ? 32 : cls == 3 ? 16 : 8;
+        const int S = G >= 16 && !NARROW ? kSegSteps32 : kSegSteps8;
         const int g = lane / G;
         const bool leader = (lane & (G - 1)) == 0;
-        uint32_t* vb = peq + kSegPeqWords + g * (G * kSegMaxW + G);
-        uint16_t* codes = reinterpret_cast<uint16_t*>(peq + kSegPeqWords + kSegVWords);
+        uint32_t* vb = peq + L::kPeq + g * (G * M + G * M / 16);
+        uint16_t* codes = reinterpret_cast<uint16_t*>(peq + L::kPeq + L::kV);
         __syncwarp();
-        for (int i = lane; i < kSegCodes; i += 32) codes[i] = kSegNoBase;
+        for (int i = lane; i < kSegCodes; i += 32) codes[i] = L::kNoBase;
         codes += g * (S + 2 * G);
         const Pair* list = A.pairs + (size_t)(c0 + cls) * A.seg_cap;
         int* work = A.work + c0 + cls;
@@ -778,15 +804,14 @@ __global__ void __launch_bounds__(kAlignThreads, 2) k_seg(DevReads R, RoundState
             const int wl =
                 __reduce_max_sync(kFull, P.busy ? (P.n_words + G - 1) / G : 1);
             int steps = 0;
-            const int d = seg_dispatch(P, wl, peq, vb, codes, G, S, lane, steps);
+            const int d = seg_dispatch<M>(P, wl, peq, vb, codes, G, S, lane, steps);
             if (!P.busy) continue;
             if (leader) done += (unsigned long long)steps * (32 * G * seg_tile(wl));
             if (d < 0) continue;
             if (leader) {
                 if (NARROW && d == 0) {
-                    const int sw = seg_words(P.T, P.q, P.c, kSegSteps32);
-                    const int to = sw <= R.group_max_w ? seg_class(sw)
-                                                       : align_class((P.q + 31) >> 5);
+                    const int to = full_class(seg_words(P.T, P.q, P.c, kSegSteps32), P.q,
+                                              R.group_max_w);
                     const int slot = atomicAdd(&st->n_pairs[to], 1);
                     if (slot < A.seg_cap)
                         const_cast<Pair*>(A.pairs)[(size_t)to * A.seg_cap + slot] = p;
@@ -3283,17 +3308,17 @@ void launch_align_t(const DevReads& R, RoundBuffers& B, int cls, cudaStream_t s)
     k_align<G, W, BATCH><<<shaped(grid, R.align_blocks), kAlignThreads, smem, s>>>(R, B.st, align_args(B), cls);
 }
 
-template <bool BATCH, bool NARROW>
+template <bool BATCH, int MODE>
 void launch_seg_t(const DevReads& R, RoundBuffers& B, cudaStream_t s) {
-    constexpr int smem = (kAlignThreads / 32) * kSegWarpWords * 4;
+    constexpr int smem = (kAlignThreads / 32) * SegSmem<kSegModeW<MODE>>::kWords * 4;
     static int grid = 0;
     if (!grid) {
-        cudaFuncSetAttribute(k_seg<BATCH, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(k_seg<BATCH, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              smem);
-        grid = grid_for(k_seg<BATCH, NARROW>, kAlignThreads, smem, 8);
+        grid = grid_for(k_seg<BATCH, MODE>, kAlignThreads, smem, 8);
     }
-    k_seg<BATCH, NARROW><<<shaped(grid, R.align_blocks), kAlignThreads, smem, s>>>(R, B.st,
-                                                                             align_args(B));
+    k_seg<BATCH, MODE><<<shaped(grid, R.align_blocks), kAlignThreads, smem, s>>>(R, B.st,
+                                                                           align_args(B));
 }
 
 template <int W, bool BATCH>
@@ -3319,8 +3344,8 @@ void launch_align_long_t(const DevReads& R, RoundBuffers& B, cudaStream_t s) {
 // Kernels launch_align_classes launches.
 template <bool BATCH>
 int align_launches(const DevReads& R, const RoundBuffers& B) {
-    return (BATCH ? kBandClasses : 0) + (R.group_max_w > 0 ? 2 : 0) +
-           (R.wide ? (BATCH ? 4 : 7) + (B.long_carry ? 1 : 0) : 0);
+    return (BATCH ? kBandClasses : 0) + (R.group_max_w > 0 ? 2 + (R.wide ? 1 : 0) : 0) +
+           (R.wide == 2 ? (BATCH ? 4 : 7) + (B.long_carry ? 1 : 0) : 0);
 }
 
 template <bool BATCH>
@@ -3330,10 +3355,11 @@ void launch_align_classes(const DevReads& R, RoundBuffers& B, cudaStream_t s) {
         launch_band_t<8, BATCH>(R, B, kSysClasses + 1, s);
     }
     if (R.group_max_w > 0) {
-        launch_seg_t<BATCH, true>(R, B, s);
-        launch_seg_t<BATCH, false>(R, B, s);
+        launch_seg_t<BATCH, kSegNarrow>(R, B, s);
+        if (R.wide) launch_seg_t<BATCH, kSegWide>(R, B, s);  // the longest work first
+        launch_seg_t<BATCH, kSegFull>(R, B, s);
     }
-    if (!R.wide) return;
+    if (R.wide < 2) return;
     if constexpr (!BATCH) {
         launch_align_t<1, 1, BATCH>(R, B, 0, s);
         launch_align_t<1, 2, BATCH>(R, B, 1, s);

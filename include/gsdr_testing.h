@@ -22,7 +22,7 @@ extern "C" {
  * form's, 2 = the batched form's with the banded one-pair-per-lane kernel for
  * every pair whose band fits its 8 words and the segment kernel up to 32,
  * 3 = the batched form's with the segment kernel (one pair per 8..32 lanes)
- * for every pair whose window fits its 512 words; greedy: 1 = a
+ * for every pair whose window fits its 768 words; greedy: 1 = a
  * narrow run (a lower bound of the LCS) first where a pass would take one.
  * accept[k] receives 0/1; *ms the device time of the alignment stage. */
 int gsdr_lcs_decide(const char* bytes, int64_t n_bytes, const int64_t* off, const int32_t* len,
