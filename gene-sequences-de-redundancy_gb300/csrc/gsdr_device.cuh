@@ -237,6 +237,7 @@ struct RoundBuffers {
     uint4* tmask;        // 4^k rows
     int32_t* tmask_ex;   // kMaxBatch
     int32_t tmask_rwq;   // 16-byte words per row: ceil(r_max / 128)
+    bool chained;        // the pass's kernels are launched with programmatic edges
     int32_t tmask_planes;  // count planes: 8 (every read <= kMaskEntries8 entries) or 10
 };
 void init_rounds(const DevReads& R, RoundBuffers& B, int batched, int r_max, cudaStream_t s,

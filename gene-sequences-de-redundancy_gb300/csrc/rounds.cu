@@ -58,6 +58,19 @@ namespace gsdr {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
+
+// A pass is a chain of short kernels.  Those launched with launch_next may be
+// set up while the kernel before them drains (programmatic dependent launch),
+// so each begins with chain_wait, which returns when that kernel has finished
+// and its writes are visible.  Every path through such a kernel passes it: a
+// kernel that ended without it would let the next one run beside the one
+// before it.  (One representative per round 147 -> 132 ms a call of 7,097
+// rounds; 14 passes of 10k reads 3.04 -> 2.96 ms.  Letting the next kernel's
+// blocks in at this kernel's start instead of its end took 10% longer on a
+// burst of served jobs: they wait in places other streams could use.)
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 constexpr int kFilterThreads = 256;
 constexpr int kAlignThreads = 256;  // 8 warps: 8/G groups of G warps
 constexpr int kAbsorbHigh = 64;     // absorbed reads per representative that shrink R
@@ -196,6 +209,7 @@ __global__ void __launch_bounds__(kFilterThreads, 6) k_filter(DevReads R, RoundS
     constexpr bool BITS = !DROP && K <= kMaxBitsK;
     constexpr int NBW = BITS ? (1 << (2 * K)) / 32 : 4;
     __shared__ __align__(16) uint32_t rbits[NBW];
+    chain_wait();
     if (st->done) return;
     if (tent && st->n_tent != 1) return;
     const int rep = tent ? tent[0] : st->rep;
@@ -619,6 +633,7 @@ __global__ void __launch_bounds__(kAlignThreads) k_band(DevReads R, RoundState* 
                                                         int cls) {
     // text bases per unrolled group
     constexpr int G = 8;
+    chain_wait();
     if (st->done) return;
     if (BATCH && (st->pair_overflow || st->n_tent == 0)) return;
     if (band_pairs(st) <= R.band_few) return;  // k_seg's
@@ -728,6 +743,7 @@ __global__ void __launch_bounds__(kAlignThreads, MODE == kSegWide ? 1 : 2) k_seg
     constexpr int M = kSegModeW<MODE>;
     using L = SegSmem<M>;
     extern __shared__ __align__(16) uint32_t seg_sm[];  // L::kWords per warp
+    chain_wait();
     if (st->done) return;
     if (BATCH && (st->pair_overflow || st->n_tent == 0)) return;
     constexpr int c0 = MODE == kSegNarrow ? kNarrowClass
@@ -929,7 +945,7 @@ __global__ void __launch_bounds__(kAlignThreads, 1) k_align_long(DevReads R, Rou
     if (lane == 0 && done) atomicAdd(&st->cells_done, done);
 }
 
-__device__ void reset_align_counters(volatile RoundState* st, int* align_work) {
+__device__ void reset_align_counters(RoundState* st, int* align_work) {
     st->n_pig = 0;
     for (int c = 0; c < kAlignClasses; c++) {
         st->n_pairs[c] = 0;
@@ -938,12 +954,11 @@ __device__ void reset_align_counters(volatile RoundState* st, int* align_work) {
     align_work[kSingleWorkSlot] = 0;  // k_align_single's shared queue
 }
 
-// Next representative (plain form).  Runs in one thread of the last block of
-// k_compact; `st` is volatile so that the other blocks' additions are read
-// from L2.
-__device__ void advance_plain(volatile RoundState* st, int32_t* cluster, int* align_work) {
-    st->rounds = st->rounds + 1;
-    st->passes = st->passes + 1;
+// Next representative (plain form), on the last block's copy of the round
+// state (k_compact).
+__device__ void advance_plain(RoundState* st, int32_t* cluster) {
+    st->rounds++;
+    st->passes++;
     if (st->error || st->pair_overflow) {
         st->done = 1;
         return;
@@ -966,14 +981,15 @@ __device__ void advance_plain(volatile RoundState* st, int32_t* cluster, int* al
     st->n_remain = n;
     st->n_next = 0;
     st->next_min = 0x7fffffff;
-    reset_align_counters(st, align_work);
+    st->n_pig = 0;
+    for (int c = 0; c < kAlignClasses; c++) st->n_pairs[c] = 0;
 }
 
 // The batched form's state for the next pass (in the same place).
-__device__ void advance_batch(volatile RoundState* st, const int32_t* tent, int seg_cap,
+__device__ void advance_batch(RoundState* st, const int32_t* tent, int seg_cap,
                               int acc_cap, int amb_cap, int drop) {
-    st->passes = st->passes + 1;
-    st->pass = st->pass + 1;
+    st->passes++;
+    st->pass++;
     if (st->error) {
         st->done = 1;
         return;
@@ -1051,6 +1067,7 @@ template <bool BATCH>
 __global__ void __launch_bounds__(256) k_compact(RoundState* st, const int32_t* __restrict__ remain_in,
                                                  int32_t* __restrict__ remain_out, CompactArgs C) {
     __shared__ int s_min, s_applied, s_base, s_warp[8];
+    chain_wait();
     if (st->done) return;
     if (threadIdx.x == 0) {
         s_min = 0x7fffffff;
@@ -1129,15 +1146,29 @@ __global__ void __launch_bounds__(256) k_compact(RoundState* st, const int32_t* 
             atomicAdd(&st->cnt_accepted, (unsigned long long)s_applied);
         }
         __threadfence();
-        if (atomicAdd(&st->ticket, 1) == (int)gridDim.x - 1) {
-            __threadfence();
-            st->ticket = 0;
-            if (BATCH)
-                advance_batch(st, C.tent, C.seg_cap, C.acc_cap, C.amb_cap, C.drop);
-            else
-                advance_plain(st, C.cluster, C.align_work);
-        }
+        s_base = atomicAdd(&st->ticket, 1) == (int)gridDim.x - 1;
     }
+    __syncthreads();
+    if (!s_base || threadIdx.x >= 32) return;
+    // the last block's first warp: the state comes over in one go, past L1
+    // (read field by field, 17 queue sizes among them, it took 6 us)
+    __shared__ RoundState s_st;
+    constexpr int W = sizeof(RoundState) / 4;
+    static_assert(sizeof(RoundState) % 4 == 0, "whole words");
+    __threadfence();
+    int* words = reinterpret_cast<int*>(&s_st);
+    for (int i = lane; i < W; i += 32) words[i] = __ldcg(reinterpret_cast<const int*>(st) + i);
+    if (!BATCH && lane <= kSingleWorkSlot) C.align_work[lane] = 0;
+    __syncwarp();
+    if (lane == 0) {
+        s_st.ticket = 0;
+        if (BATCH)
+            advance_batch(&s_st, C.tent, C.seg_cap, C.acc_cap, C.amb_cap, C.drop);
+        else
+            advance_plain(&s_st, C.cluster);
+    }
+    __syncwarp();
+    for (int i = lane; i < W; i += 32) reinterpret_cast<int*>(st)[i] = words[i];
 }
 
 // ---------------------------------------------------------------- batched form
@@ -1149,6 +1180,7 @@ __global__ void __launch_bounds__(1024) k_bselect(RoundState* st, const int32_t*
                                                   int* align_work) {
     __shared__ int warp_cnt[4 * 32];
     __shared__ int s_nt;
+    chain_wait();
     if (st->done) return;
     const int Rq = st->R;
     const int pass = st->pass;
@@ -1371,6 +1403,7 @@ __global__ void __launch_bounds__(kFilterThreads) k_bprefilter(DevReads R, Round
     constexpr int RG = 32;
     __shared__ int4 tcomp[RG];
     __shared__ int ttent[RG];
+    chain_wait();
     if (st->done || st->n_tent == 0) return;
     const int nt = st->n_tent;
     const int n = st->n_remain;
@@ -1478,6 +1511,7 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
     __shared__ uint64_t full[kBitsStages], empty[kBitsStages], tfull[2], tempty[2], drain;
     __shared__ uint32_t s_tmem;
     __shared__ int s_quit;
+    chain_wait();
     if (st->done) return;
     const int nt = st->n_tent;
     if (nt <= 1) return;  // a single tentative's pass runs k_filter instead
@@ -1755,6 +1789,7 @@ __global__ void __launch_bounds__(kAmbThreads) k_amb_count(RoundState* st, const
                                                           int amb_cap, const uint32_t* __restrict__ tidx,
                                                           int* amb_idx) {
     __shared__ int h[kMaxBatch];
+    chain_wait();
     if (st->done || st->n_tent == 0) return;
     const int na = amb_n(st, amb_cap);
     if (na <= 0) return;
@@ -1772,6 +1807,7 @@ __global__ void __launch_bounds__(kAmbThreads) k_amb_count(RoundState* st, const
 // go back to zero for the next pass.
 __global__ void __launch_bounds__(1024) k_amb_scan(RoundState* st, int amb_cap, int* amb_idx) {
     __shared__ int ws[2][32];
+    chain_wait();
     if (st->done || st->n_tent == 0) return;
     if (amb_n(st, amb_cap) <= 0) return;
     const int nt = st->n_tent;
@@ -1811,6 +1847,7 @@ __global__ void __launch_bounds__(kAmbThreads) k_amb_place(RoundState* st, const
                                                           int amb_cap, const uint32_t* __restrict__ tidx,
                                                           int* amb_idx, Pair* amb2) {
     __shared__ int h[kMaxBatch];
+    chain_wait();
     if (st->done || st->n_tent == 0) return;
     const int na = amb_n(st, amb_cap);
     if (na <= 0) return;
@@ -1846,6 +1883,7 @@ __global__ void __launch_bounds__(kAmbThreads) k_bexact_t(DevReads R, RoundState
     constexpr int NB = 1 << (2 * K);
     extern __shared__ __align__(16) uint16_t xtab[];  // NB counts
     __shared__ int s_items[kMaxBatch + 1];
+    chain_wait();
     if (st->done || st->n_tent == 0) return;
     if (amb_n(st, amb_cap) <= 0) return;
     const int nt = st->n_tent;
@@ -2264,6 +2302,7 @@ __global__ void __launch_bounds__(kHashThreads, 1) k_bfilter_hash(
     __shared__ uint64_t full[kHashStages], empty[kHashStages], tfull[2], tempty[2], drain;
     __shared__ uint32_t s_tmem;
     __shared__ int s_quit;
+    chain_wait();
     if (st->done) return;
     const int nt = st->n_tent;
     if (nt == 0) return;
@@ -2900,6 +2939,7 @@ __global__ void __launch_bounds__(kMaxBatch) k_bclaim(RoundState* st, const int3
                                                       const uint32_t* __restrict__ tidx,
                                                       uint32_t* best, int32_t* cluster) {
     __shared__ __align__(16) uint32_t surv[kTTWords], open[kTTWords];
+    chain_wait();
     if (st->done || st->n_tent == 0 || st->pair_overflow || st->acc_overflow) return;
     const int nt = st->n_tent;
     const int na = st->n_acc;
@@ -2971,7 +3011,8 @@ __global__ void k_init(RoundState* st, int32_t* cluster, int32_t* remain, uint32
         s.next_min = 0x7fffffff;
         s.done = n <= 0 ? 1 : 0;
         s.pass = 1;
-        s.R = 1;
+        // as many tentatives as leave the device idle in any case (kFewPairs)
+        s.R = min(r_max, max(1, kFewPairs / max(n, 1)));
         s.R_max = r_max;
         s.pass_limit = pass_limit;
         *st = s;
@@ -3042,6 +3083,25 @@ __global__ void k_resume_start(RoundState* st, int32_t* cluster, int batched) {
 
 // ---------------------------------------------------------------- launchers
 
+// Launch of a kernel that begins with chain_wait; with B.chained behind a
+// programmatic edge (not between the events of a timed step, which stand
+// between the kernels).
+template <class... P, class... A>
+void launch_next(const RoundBuffers& B, void (*kernel)(P...), int grid, int threads, int smem,
+                 cudaStream_t s, A... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = B.chained ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 template <class KernelT>
 int grid_for(KernelT kernel, int threads, int smem, int cap_per_sm) {
     int per_sm = 0;
@@ -3071,8 +3131,7 @@ void launch_filter_t(const DevReads& R, RoundBuffers& B, const int32_t* remain, 
                                  smem);
         grid = grid_for(k_filter<K, DROP>, kFilterThreads, smem, 8);
     }
-    k_filter<K, DROP><<<shaped(grid, R.filter_blocks), kFilterThreads, smem, s>>>(R, B.st, remain, B.pairs, B.seg_cap,
-                                                         tent);
+    launch_next(B, k_filter<K, DROP>, shaped(grid, R.filter_blocks), kFilterThreads, smem, s, R, B.st, remain, B.pairs, B.seg_cap, tent);
 }
 
 template <int K>
@@ -3098,7 +3157,7 @@ void launch_bfilter_t(const DevReads& R, RoundBuffers& B, const int32_t* remain,
     } else {
         static int grid = 0;
         if (!grid) grid = grid_for(k_bprefilter, kFilterThreads, 0, 8);
-        k_bprefilter<<<shaped(grid, R.filter_blocks), kFilterThreads, 0, s>>>(R, B.st, remain, B.tent, B.pairs, B.seg_cap);
+        launch_next(B, k_bprefilter, shaped(grid, R.filter_blocks), kFilterThreads, 0, s, R, B.st, remain, B.tent, B.pairs, B.seg_cap);
     }
 }
 
@@ -3149,11 +3208,10 @@ void launch_exact_t(const DevReads& R, RoundBuffers& B, cudaStream_t s) {
         grid = grid_for(k_bexact_t<K>, kAmbThreads, xsmem, 8);
     }
     const int ga = num_sms() * 2;
-    k_amb_count<<<ga, kAmbThreads, 0, s>>>(B.st, B.amb, B.amb_cap, B.tidx, B.amb_idx);
-    k_amb_scan<<<1, 1024, 0, s>>>(B.st, B.amb_cap, B.amb_idx);
-    k_amb_place<<<ga, kAmbThreads, 0, s>>>(B.st, B.amb, B.amb_cap, B.tidx, B.amb_idx, B.amb2);
-    k_bexact_t<K><<<shaped(grid, R.filter_blocks), kAmbThreads, xsmem, s>>>(
-        R, B.st, B.amb2, B.amb_idx, B.amb_cap, B.tent, B.pairs, B.seg_cap);
+    launch_next(B, k_amb_count, ga, kAmbThreads, 0, s, B.st, B.amb, B.amb_cap, B.tidx, B.amb_idx);
+    launch_next(B, k_amb_scan, 1, 1024, 0, s, B.st, B.amb_cap, B.amb_idx);
+    launch_next(B, k_amb_place, ga, kAmbThreads, 0, s, B.st, B.amb, B.amb_cap, B.tidx, B.amb_idx, B.amb2);
+    launch_next(B, k_bexact_t<K>, shaped(grid, R.filter_blocks), kAmbThreads, xsmem, s,  R, B.st, B.amb2, B.amb_idx, B.amb_cap, B.tent, B.pairs, B.seg_cap);
 }
 
 template <int K>
@@ -3168,8 +3226,7 @@ void launch_bfilter_bits_t(const DevReads& R, RoundBuffers& B, const int32_t* re
                              kBitsSmem);
         grid = grid_for(k_bfilter_bits<K>, kBitsThreads, kBitsSmem, 1);
     }
-    k_bfilter_bits<K><<<grid, kBitsThreads, kBitsSmem, s>>>(R, B.st, remain, B.tent, B.pairs,
-                                                            B.seg_cap, B.amb, B.amb_cap);
+    launch_next(B, k_bfilter_bits<K>, grid, kBitsThreads, kBitsSmem, s, R, B.st, remain, B.tent, B.pairs, B.seg_cap, B.amb, B.amb_cap);
     launch_exact_t<K>(R, B, s);
 }
 
@@ -3182,8 +3239,7 @@ void launch_bfilter_hash_t(const DevReads& R, RoundBuffers& B, const int32_t* re
                              kHashSmem);
         attr = true;
     }
-    k_bfilter_hash<<<num_sms(), kHashThreads, kHashSmem, s>>>(R, B.st, remain, B.tent, B.amb,
-                                                              B.amb_cap);
+    launch_next(B, k_bfilter_hash, num_sms(), kHashThreads, kHashSmem, s, R, B.st, remain, B.tent, B.amb, B.amb_cap);
     launch_exact_t<K>(R, B, s);
 }
 
@@ -3317,15 +3373,14 @@ void launch_seg_t(const DevReads& R, RoundBuffers& B, cudaStream_t s) {
                              smem);
         grid = grid_for(k_seg<BATCH, MODE>, kAlignThreads, smem, 8);
     }
-    k_seg<BATCH, MODE><<<shaped(grid, R.align_blocks), kAlignThreads, smem, s>>>(R, B.st,
-                                                                           align_args(B));
+    launch_next(B, k_seg<BATCH, MODE>, shaped(grid, R.align_blocks), kAlignThreads, smem, s, R, B.st, align_args(B));
 }
 
 template <int W, bool BATCH>
 void launch_band_t(const DevReads& R, RoundBuffers& B, int cls, cudaStream_t s) {
     static int grid = 0;
     if (!grid) grid = grid_for(k_band<W, BATCH>, kAlignThreads, 0, 8);
-    k_band<W, BATCH><<<shaped(grid, R.align_blocks), kAlignThreads, 0, s>>>(R, B.st, align_args(B), cls);
+    launch_next(B, k_band<W, BATCH>, shaped(grid, R.align_blocks), kAlignThreads, 0, s, R, B.st, align_args(B), cls);
 }
 
 template <bool BATCH>
@@ -3421,14 +3476,14 @@ void launch_plain_round(const DevReads& R, RoundBuffers& B, int drop, int parity
                         long long* count, cudaEvent_t* ev4) {
     const int32_t* rin = B.remain[parity];
     int32_t* rout = B.remain[parity ^ 1];
+    B.chained = ev4 == nullptr;
     if (ev4) cudaEventRecordWithFlags(ev4[0], s, cudaEventRecordExternal);
     launch_filter_any<false>(R, B, rin, drop, s);
     if (R.pig_q && !drop) k_pigeon<false><<<num_sms() * 8, 256, 0, s>>>(R, B.st, B.pairs, B.seg_cap);
     if (ev4) cudaEventRecordWithFlags(ev4[1], s, cudaEventRecordExternal);
     launch_align_classes<false>(R, B, s);
     if (ev4) cudaEventRecordWithFlags(ev4[2], s, cudaEventRecordExternal);
-    k_compact<false><<<num_sms() * 4, 256, 0, s>>>(
-        B.st, rin, rout, CompactArgs{B.cluster, align_work_of(B.st), nullptr, nullptr, 0, 0, 0, 0});
+    launch_next(B, k_compact<false>, num_sms() * 4, 256, 0, s,  B.st, rin, rout, CompactArgs{B.cluster, align_work_of(B.st), nullptr, nullptr, 0, 0, 0, 0});
     if (ev4) cudaEventRecordWithFlags(ev4[3], s, cudaEventRecordExternal);
     if (count)
         *count += 2 + align_launches<false>(R, B) + (R.pig_q && !drop ? 1 : 0) +
@@ -3451,20 +3506,16 @@ void launch_batch_pass(const DevReads& R, RoundBuffers& B, int drop, int parity,
                        long long* count, cudaEvent_t* ev4) {
     const int32_t* rin = B.remain[parity];
     int32_t* rout = B.remain[parity ^ 1];
-    k_bselect<<<1, 1024, 0, s>>>(B.st, B.cluster, R.n, B.tent, B.tidx, B.tt, B.ttrow,
-                                 align_work_of(B.st));
+    B.chained = ev4 == nullptr;
+    launch_next(B, k_bselect, 1, 1024, 0, s, B.st, B.cluster, R.n, B.tent, B.tidx, B.tt, B.ttrow, align_work_of(B.st));
     if (ev4) cudaEventRecordWithFlags(ev4[0], s, cudaEventRecordExternal);
     launch_filter_any<true>(R, B, rin, drop, s);
     if (R.pig_q && !drop) k_pigeon<true><<<num_sms() * 8, 256, 0, s>>>(R, B.st, B.pairs, B.seg_cap);
     if (ev4) cudaEventRecordWithFlags(ev4[1], s, cudaEventRecordExternal);
     launch_align_classes<true>(R, B, s);
     if (ev4) cudaEventRecordWithFlags(ev4[2], s, cudaEventRecordExternal);
-    k_bclaim<<<num_sms(), kMaxBatch, 0, s>>>(B.st, B.tent, B.tt, B.ttrow, B.acc, B.tidx, B.best,
-                                             B.cluster);
-    k_compact<true><<<num_sms() * 4, 256, 0, s>>>(
-        B.st, rin, rout,
-        CompactArgs{B.cluster, align_work_of(B.st), B.best, B.tent, B.seg_cap, B.acc_cap, B.amb_cap,
-                    drop});
+    launch_next(B, k_bclaim, num_sms(), kMaxBatch, 0, s, B.st, B.tent, B.tt, B.ttrow, B.acc, B.tidx, B.best, B.cluster);
+    launch_next(B, k_compact<true>, num_sms() * 4, 256, 0, s,  B.st, rin, rout, CompactArgs{B.cluster, align_work_of(B.st), B.best, B.tent, B.seg_cap, B.acc_cap, B.amb_cap, drop});
     if (ev4) cudaEventRecordWithFlags(ev4[3], s, cudaEventRecordExternal);
     if (count)
         *count += 4 + align_launches<true>(R, B) + (!drop ? 1 : 0) +
