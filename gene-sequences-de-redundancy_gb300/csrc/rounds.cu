@@ -216,9 +216,18 @@ __global__ void __launch_bounds__(kFilterThreads, 6) k_filter(DevReads R, RoundS
     const int band_w = tent ? kBandMaxW : kPlainBandMaxW;
     const int n = st->n_remain;
     if (n <= 0) return;
-    // a block with no candidate skips its copy of the representative's table
+    // a block with no candidate skips its copy of the representative's tables
     if ((long long)blockIdx.x * (kFilterThreads / 32) >= n) return;
-    if (!DROP) {
+    const int lane = threadIdx.x & 31;
+    const int nwarps = gridDim.x * (kFilterThreads / 32);
+    const int idx0 = blockIdx.x * (kFilterThreads / 32) + (threadIdx.x >> 5);
+    unsigned n_pf = 0, n_wf = 0, n_al = 0;
+    unsigned long long bytes = 0;
+    const int4 crep = R.comp[rep];
+    // kernel_filter (func.cu:803-826): S = sum over distinct k-mers of
+    // min(count in representative, count in candidate) against the candidate's
+    // word cutoff, from the candidate's list and the representative's table
+    auto make_table = [&]() {
         constexpr int NB = 1 << (2 * K);
         uint32_t* t32 = reinterpret_cast<uint32_t*>(table);
         for (int i = threadIdx.x; i < NB / 2; i += blockDim.x) t32[i] = 0u;
@@ -230,23 +239,42 @@ __global__ void __launch_bounds__(kFilterThreads, 6) k_filter(DevReads R, RoundS
             const uint32_t c = v & 0xffffu;
             if (c) table[v >> 16] = (uint16_t)c;  // kernel_makeTable: only order > 0
         }
-        if (BITS)
-            for (int i = threadIdx.x; i < NBW; i += blockDim.x) rbits[i] = R.kbits[(size_t)rep * NBW + i];
         __syncthreads();
+    };
+    auto word_sum = [&](int q) {
+        const int ne4 = (R.n_kmer[q] + 3) >> 2;
+        const uint4* e4 = reinterpret_cast<const uint4*>(R.kmer + R.kmer_off[q]);
+        bytes += 16ull * ne4;
+        int sum = 0;
+#pragma unroll 4
+        for (int i = lane; i < ne4; i += 32) {
+            const uint4 v = __ldcs(e4 + i);
+            sum += min((uint32_t)table[v.x >> 16], v.x & 0xffffu);
+            sum += min((uint32_t)table[v.y >> 16], v.y & 0xffffu);
+            sum += min((uint32_t)table[v.z >> 16], v.z & 0xffffu);
+            sum += min((uint32_t)table[v.w >> 16], v.w & 0xffffu);
+        }
+        return warp_sum_i(sum);
+    };
+    // With one or two candidates per warp (the later rounds) the bitmaps
+    // decide nearly all of them, so the table waits until some warp of the
+    // block needs it; with more it is made at once.
+    const bool late = BITS && n <= 4 * nwarps;
+    constexpr int kLate = 4;  // a late block has at most this many candidates per warp
+    int open[kLate], n_open = 0;
+    if (BITS) {
+        for (int i = threadIdx.x; i < NBW; i += blockDim.x) rbits[i] = R.kbits[(size_t)rep * NBW + i];
+        if (late) __syncthreads();
     }
+    if (!DROP && !late) make_table();
     const int rep_extra = BITS ? R.kextra[rep] : 0;
-    const int lane = threadIdx.x & 31;
-    const int4 crep = R.comp[rep];
-    unsigned n_pf = 0, n_wf = 0, n_al = 0;
-    unsigned long long bytes = 0;
-    const int nwarps = gridDim.x * (kFilterThreads / 32);
     // Software pipeline over this warp's candidates: while candidate i is
     // decided, the composition and cutoff of candidate i+1 are already in
     // flight and the index of candidate i+2 too, so part of the chain of
     // dependent loads (remain -> scalars -> list) overlaps the previous
     // candidate's list stream.  (Prefetching the bitmap as well needs 48
     // registers, five CTAs per SM instead of six, and measured slower.)
-    int idx = blockIdx.x * (kFilterThreads / 32) + (threadIdx.x >> 5);
+    int idx = idx0;
     int q_nx = idx < n ? __ldg(remain + idx) : -1;
     int q_af = idx + nwarps < n ? __ldg(remain + idx + nwarps) : -1;
     int4 comp_nx = make_int4(0, 0, 0, 0);
@@ -272,13 +300,8 @@ __global__ void __launch_bounds__(kFilterThreads, 6) k_filter(DevReads R, RoundS
         // kernel_preFilter (func.cu:738-754); lossless, so also used in drop mode.
         if (!prefilter_pass(crep, comp_q, cb_q - R.strict)) continue;
         if (!DROP) {
-            // kernel_filter (func.cu:803-826): S = sum over distinct k-mers of
-            // min(count in representative, count in candidate), compared with
-            // the candidate's word cutoff.
             n_wf++;
             const int cw = R.cut_word[q];
-            const int64_t koff = R.kmer_off[q];
-            const int nk = R.n_kmer[q];
             bool decided = false, pass = false;
             if (BITS) {
                 // D = shared k-mers (non-zero counts) bounds S: D <= S <= D + min(excesses)
@@ -296,25 +319,30 @@ __global__ void __launch_bounds__(kFilterThreads, 6) k_filter(DevReads R, RoundS
                 else if (d + min(q_extra, rep_extra) < cw) decided = true;
             }
             if (!decided) {
-                const int ne4 = (nk + 3) >> 2;
-                const uint4* e4 = reinterpret_cast<const uint4*>(R.kmer + koff);
-                bytes += 16ull * ne4;
-                int sum = 0;
-#pragma unroll 4
-                for (int i = lane; i < ne4; i += 32) {
-                    const uint4 v = __ldcs(e4 + i);
-                    sum += min((uint32_t)table[v.x >> 16], v.x & 0xffffu);
-                    sum += min((uint32_t)table[v.y >> 16], v.y & 0xffffu);
-                    sum += min((uint32_t)table[v.z >> 16], v.z & 0xffffu);
-                    sum += min((uint32_t)table[v.w >> 16], v.w & 0xffffu);
+                if (late) {
+#pragma unroll
+                    for (int u = 0; u < kLate; u++)
+                        if (u == n_open) open[u] = q;
+                    n_open++;
+                    continue;
                 }
-                sum = warp_sum_i(sum);
-                pass = !(sum < cw);
+                pass = !(word_sum(q) < cw);
             }
             if (!pass) continue;
         }
         n_al++;
         if (lane == 0) push_pair(st, pairs, seg_cap, R, rep, q, band_w);
+    }
+    if (BITS && late && __syncthreads_or(n_open)) {
+        make_table();
+#pragma unroll
+        for (int u = 0; u < kLate; u++) {
+            if (u >= n_open) break;
+            const int q = open[u];
+            if (word_sum(q) < R.cut_word[q]) continue;
+            n_al++;
+            if (lane == 0) push_pair(st, pairs, seg_cap, R, rep, q, band_w);
+        }
     }
     // one addition per block and counter: the counters share a cache line, and
     // one per warp (7,296 warps) took most of a 10k-candidate launch's 21.9 us
@@ -749,7 +777,11 @@ __global__ void __launch_bounds__(kAlignThreads, MODE == kSegWide ? 1 : 2) k_seg
     constexpr int c0 = MODE == kSegNarrow ? kNarrowClass
                        : MODE == kSegWide ? kWideClass
                                           : kSysClasses + kBandClasses;
-    constexpr int nc = MODE == kSegFull ? kSegClasses : 1;
+    // plain rounds: the narrow class runs here too, a warp per pair, first (one
+    // launch less per round; its pairs go on to their full window in place)
+    constexpr bool BOTH = MODE == kSegFull && !BATCH;
+    static_assert(kNarrowClass == kSysClasses + kBandClasses + kSegClasses, "the class after");
+    constexpr int nc = MODE == kSegFull ? kSegClasses + (BOTH ? 1 : 0) : 1;
     // the lane-banded classes' pairs too when they are few (k_band)
     const int first =
         MODE == kSegFull && BATCH && band_pairs(st) <= R.band_few ? -kBandClasses : 0;
@@ -767,8 +799,11 @@ __global__ void __launch_bounds__(kAlignThreads, MODE == kSegWide ? 1 : 2) k_seg
     for (int cls = nc - 1; cls >= first; cls--) {
         const int np = min(st->n_pairs[c0 + cls], A.seg_cap);
         if (np <= 0) continue;
-        const int G = MODE == kSegWide || alone || cls == 4 ? 32 : cls == 3 ? 16 : 8;
-        const int S = G >= 16 && !NARROW ? kSegSteps32 : kSegSteps8;
+        const bool narrow = NARROW || (BOTH && cls == kSegClasses);
+        const int G = MODE == kSegWide || alone || (BOTH && narrow) || cls == 4 ? 32
+                      : cls == 3                                                ? 16
+                                                                                : 8;
+        const int S = G >= 16 && !narrow ? kSegSteps32 : kSegSteps8;
         const int g = lane / G;
         const bool leader = (lane & (G - 1)) == 0;
         uint32_t* vb = peq + L::kPeq + g * (G * M + G * M / 16);
@@ -802,9 +837,9 @@ __global__ void __launch_bounds__(kAlignThreads, MODE == kSegWide ? 1 : 2) k_seg
                         P.stride = (int)((R.pack_off[p.rep + 1] - po) >> 1);
                         P.planes = R.bm + 2 * po;
                         P.pq = R.packed + R.pack_off[p.cand];
-                        P.slope = NARROW ? seg_narrow_slope(T, q, c) : 0.0f;
+                        P.slope = narrow ? seg_narrow_slope(T, q, c) : 0.0f;
                         P.busy = true;
-                        seg_start(P, S, NARROW);
+                        seg_start(P, S, narrow);
                     } else if (leader) {
                         cells += (unsigned long long)T * (unsigned long long)q;
                         if (trivial) {
@@ -824,8 +859,13 @@ __global__ void __launch_bounds__(kAlignThreads, MODE == kSegWide ? 1 : 2) k_seg
             if (!P.busy) continue;
             if (leader) done += (unsigned long long)steps * (32 * G * seg_tile(wl));
             if (d < 0) continue;
+            if (BOTH && d == 0 && P.narrow &&
+                seg_words(P.T, P.q, P.c, kSegSteps32) <= kSegMaxWords) {
+                seg_start(P, S, false);
+                continue;
+            }
             if (leader) {
-                if (NARROW && d == 0) {
+                if (P.narrow && d == 0) {
                     const int to = full_class(seg_words(P.T, P.q, P.c, kSegSteps32), P.q,
                                               R.group_max_w);
                     const int slot = atomicAdd(&st->n_pairs[to], 1);
@@ -3399,7 +3439,8 @@ void launch_align_long_t(const DevReads& R, RoundBuffers& B, cudaStream_t s) {
 // Kernels launch_align_classes launches.
 template <bool BATCH>
 int align_launches(const DevReads& R, const RoundBuffers& B) {
-    return (BATCH ? kBandClasses : 0) + (R.group_max_w > 0 ? 2 + (R.wide ? 1 : 0) : 0) +
+    return (BATCH ? kBandClasses : 0) +
+           (R.group_max_w > 0 ? (BATCH ? 2 : 1) + (R.wide ? 1 : 0) : 0) +
            (R.wide == 2 ? (BATCH ? 4 : 7) + (B.long_carry ? 1 : 0) : 0);
 }
 
@@ -3410,9 +3451,14 @@ void launch_align_classes(const DevReads& R, RoundBuffers& B, cudaStream_t s) {
         launch_band_t<8, BATCH>(R, B, kSysClasses + 1, s);
     }
     if (R.group_max_w > 0) {
-        launch_seg_t<BATCH, kSegNarrow>(R, B, s);
-        if (R.wide) launch_seg_t<BATCH, kSegWide>(R, B, s);  // the longest work first
-        launch_seg_t<BATCH, kSegFull>(R, B, s);
+        if constexpr (BATCH) {
+            launch_seg_t<BATCH, kSegNarrow>(R, B, s);
+            if (R.wide) launch_seg_t<BATCH, kSegWide>(R, B, s);  // the longest work first
+            launch_seg_t<BATCH, kSegFull>(R, B, s);
+        } else {
+            launch_seg_t<BATCH, kSegFull>(R, B, s);  // and the narrow runs
+            if (R.wide) launch_seg_t<BATCH, kSegWide>(R, B, s);
+        }
     }
     if (R.wide < 2) return;
     if constexpr (!BATCH) {
