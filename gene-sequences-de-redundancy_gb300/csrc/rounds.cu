@@ -200,7 +200,10 @@ __device__ __forceinline__ void add_counts(RoundState* st, int lane, unsigned lo
 // kernel takes the passes with a single tentative: that tentative is the
 // smallest unclustered read, so every other remaining read is its candidate
 // and the pass is a plain round; k_bfilter_tab takes the passes with more.
-template <int K, bool DROP>
+// LATE (plain rounds): the representative's table may wait (below); the
+// batched form's passes with one tentative stream every candidate, and the
+// queue of open candidates would cost them registers.
+template <int K, bool DROP, bool LATE>
 __global__ void __launch_bounds__(kFilterThreads, 6) k_filter(DevReads R, RoundState* st,
                                                            const int32_t* __restrict__ remain,
                                                            Pair* pairs, int seg_cap,
@@ -256,10 +259,10 @@ __global__ void __launch_bounds__(kFilterThreads, 6) k_filter(DevReads R, RoundS
         }
         return warp_sum_i(sum);
     };
-    // With one or two candidates per warp (the later rounds) the bitmaps
-    // decide nearly all of them, so the table waits until some warp of the
-    // block needs it; with more it is made at once.
-    const bool late = BITS && n <= 4 * nwarps;
+    // With a few candidates per warp (the later rounds) the bitmaps decide
+    // nearly all of them, so the table waits until some warp of the block
+    // needs it; with more it is made at once.
+    const bool late = LATE && BITS && n <= 4 * nwarps;
     constexpr int kLate = 4;  // a late block has at most this many candidates per warp
     int open[kLate], n_open = 0;
     if (BITS) {
@@ -319,7 +322,7 @@ __global__ void __launch_bounds__(kFilterThreads, 6) k_filter(DevReads R, RoundS
                 else if (d + min(q_extra, rep_extra) < cw) decided = true;
             }
             if (!decided) {
-                if (late) {
+                if (LATE && late) {
 #pragma unroll
                     for (int u = 0; u < kLate; u++)
                         if (u == n_open) open[u] = q;
@@ -333,7 +336,7 @@ __global__ void __launch_bounds__(kFilterThreads, 6) k_filter(DevReads R, RoundS
         n_al++;
         if (lane == 0) push_pair(st, pairs, seg_cap, R, rep, q, band_w);
     }
-    if (BITS && late && __syncthreads_or(n_open)) {
+    if (LATE && BITS && late && __syncthreads_or(n_open)) {
         make_table();
 #pragma unroll
         for (int u = 0; u < kLate; u++) {
@@ -1510,8 +1513,9 @@ __global__ void __launch_bounds__(kFilterThreads) k_bprefilter(DevReads R, Round
 // to end, 0/1) times the tentatives' transposed.  k_bfilter_bits forms it on
 // the tensor cores: tiles of 128 candidates x up to 240 tentatives, the
 // bitmaps spread to 4-bit values on their way into shared memory (any fixed
-// order of a read's k-mers gives the same sum, so the spread is three shifts
-// and four masks per 32 k-mers), accumulators in tensor memory.
+// order of a read's k-mers gives the same sum, so the spread is two
+// multiplications, a shift and four masks per 32 k-mers), accumulators in
+// tensor memory.
 //
 // A CTA per SM: one warp issues the MMAs, 23 warps load and spread the
 // bitmaps into a ring of four stages (256 k-mers of every row), and four warps
@@ -1523,9 +1527,12 @@ __global__ void __launch_bounds__(kFilterThreads) k_bprefilter(DevReads R, Round
 //
 // 84,800 candidates x 1,024 tentatives, k = 6: 0.42 ms (2.1e11 pairs/s), ALU
 // pipe 71% (the spread and the composition bound), shared-memory pipe 64%,
-// tensor pipe 35%; the AND + POPC kernel before it took about 3 ms.  Filter stage: 149 -> 27 ms (100k reads of 150-5,000 bp, t = 0.95),
-// 42 -> 8.1 ms (30k, t = 0.90, k = 7, with R_max 1024 instead of 256, which the
-// lanes' form could not stage), 2.36 -> 0.91 ms (10k reads of 200-1,000 bp).
+// tensor pipe 35%; the AND + POPC kernel before it took about 3 ms.  With
+// two of the spread's shifts as multiplications (off the ALU pipe) the filter
+// stage of the first workload below went from 26.3 to 23.9 ms.
+// Filter stage: 149 -> 24 ms (100k reads of 150-5,000 bp, t = 0.95),
+// 42 -> 5.9 ms (30k, t = 0.90, k = 7, with R_max 1024 instead of 256, which the
+// lanes' form could not stage), 2.36 -> 0.88 ms (10k reads of 200-1,000 bp).
 // On the way there: eight producer loads of 32 bytes of a row each (shared
 // pipe 71%, 0.49 ms); 12 producers (0.53 ms: every warp takes part in every
 // stage, so a stage lasts as long as one warp's share of it); the MMAs issued
@@ -1656,7 +1663,7 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
                     const int2 te = tte[t];
                     before |= te.x < q ? 1u << j : 0u;
                     pre |= prefilter_pass(tcomp[t], cq, cbq) ? 1u << j : 0u;
-                    hit |= (int)(4.0f * v[j]) + min(te.y, exq) >= cw ? 1u << j : 0u;
+                    hit |= (int)(kTcSpreadUnit * v[j]) + min(te.y, exq) >= cw ? 1u << j : 0u;
                 }
                 before &= ncol >= 16 ? 0xffffu : (1u << ncol) - 1u;
                 pre &= before;
@@ -1670,7 +1677,7 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
 #pragma unroll
                     for (int i = 1; i < 16; i++) vj = j == i ? v[i] : vj;
                     const int rep = tte[c0 + j].x;
-                    if ((int)(4.0f * vj) >= cw) {
+                    if ((int)(kTcSpreadUnit * vj) >= cw) {
                         push_pair(st, pairs, seg_cap, R, rep, q, kBandMaxW);
                         n_al++;
                     } else {
@@ -3160,18 +3167,19 @@ int shaped(int grid, int blocks) {
 
 // tent: null for a plain round; the batched form's tentatives otherwise (the
 // kernel then runs only in a pass with a single tentative).
-template <int K, bool DROP>
+template <int K, bool DROP, bool LATE>
 void launch_filter_t(const DevReads& R, RoundBuffers& B, const int32_t* remain, cudaStream_t s,
                      const int32_t* tent = nullptr) {
     const int smem = DROP ? 0 : (1 << (2 * K)) * 2;
     static int grid = 0;
     if (!grid) {
         if (smem > 0)
-            cudaFuncSetAttribute(k_filter<K, DROP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 smem);
-        grid = grid_for(k_filter<K, DROP>, kFilterThreads, smem, 8);
+            cudaFuncSetAttribute(k_filter<K, DROP, LATE>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        grid = grid_for(k_filter<K, DROP, LATE>, kFilterThreads, smem, 8);
     }
-    launch_next(B, k_filter<K, DROP>, shaped(grid, R.filter_blocks), kFilterThreads, smem, s, R, B.st, remain, B.pairs, B.seg_cap, tent);
+    launch_next(B, k_filter<K, DROP, LATE>, shaped(grid, R.filter_blocks), kFilterThreads, smem, s,
+                R, B.st, remain, B.pairs, B.seg_cap, tent);
 }
 
 template <int K>
@@ -3180,7 +3188,7 @@ void launch_bfilter_tab_t(const DevReads& R, RoundBuffers& B, const int32_t* rem
     // passes with one tentative (the first passes of adaptive R) stream the
     // candidates once against one table: the plain kernel does that at HBM
     // speed, the grouped-table kernel skips them
-    launch_filter_t<K, false>(R, B, remain, s, B.tent);
+    launch_filter_t<K, false, false>(R, B, remain, s, B.tent);
     constexpr int smem = TabGroup<K>::smem;
     static int grid = 0;
     if (!grid) {
@@ -3259,7 +3267,7 @@ void launch_bfilter_bits_t(const DevReads& R, RoundBuffers& B, const int32_t* re
                            cudaStream_t s) {
     // passes with one tentative (the first passes of adaptive R) go to the
     // plain kernel, which streams the candidates against one table
-    launch_filter_t<K, false>(R, B, remain, s, B.tent);
+    launch_filter_t<K, false, false>(R, B, remain, s, B.tent);
     static int grid = 0;
     if (!grid) {
         cudaFuncSetAttribute(k_bfilter_bits<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -3359,21 +3367,21 @@ void launch_filter_any(const DevReads& R, RoundBuffers& B, const int32_t* remain
     }
     if (drop) {
         if (BATCH) launch_bfilter_t<4, true>(R, B, remain, s);
-        else launch_filter_t<4, true>(R, B, remain, s);
+        else launch_filter_t<4, true, true>(R, B, remain, s);
         return;
     }
     switch (R.k) {
         case 4:
-            BATCH ? launch_bfilter_t<4, false>(R, B, remain, s) : launch_filter_t<4, false>(R, B, remain, s);
+            BATCH ? launch_bfilter_t<4, false>(R, B, remain, s) : launch_filter_t<4, false, true>(R, B, remain, s);
             break;
         case 5:
-            BATCH ? launch_bfilter_t<5, false>(R, B, remain, s) : launch_filter_t<5, false>(R, B, remain, s);
+            BATCH ? launch_bfilter_t<5, false>(R, B, remain, s) : launch_filter_t<5, false, true>(R, B, remain, s);
             break;
         case 6:
-            BATCH ? launch_bfilter_t<6, false>(R, B, remain, s) : launch_filter_t<6, false>(R, B, remain, s);
+            BATCH ? launch_bfilter_t<6, false>(R, B, remain, s) : launch_filter_t<6, false, true>(R, B, remain, s);
             break;
         default:
-            BATCH ? launch_bfilter_t<7, false>(R, B, remain, s) : launch_filter_t<7, false>(R, B, remain, s);
+            BATCH ? launch_bfilter_t<7, false>(R, B, remain, s) : launch_filter_t<7, false, true>(R, B, remain, s);
             break;
     }
 }

@@ -3,10 +3,8 @@
 //
 // The filters multiply 0/1 matrices (and small counts) held as E2M1 values:
 // kind::mxf4 takes 4-bit operands with one scale per 32 of them, here 1.0
-// everywhere, and accumulates in 32-bit floats.  A one is stored as 0.5 (bit
-// pattern 0001), so a product is 0.25 and a sum of n products n / 4: exact for
-// every count the filters form (checked against popcounts up to 32,768 ones
-// on both sides).
+// everywhere, and accumulates in 32-bit floats: exact for every count the
+// filters form (checked against popcounts up to 32,768 ones on both sides).
 #pragma once
 #include <stdint.h>
 
@@ -157,11 +155,14 @@ __device__ __forceinline__ void tc_load_wait(uint32_t (&r)[16], float (&v)[16]) 
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
-// 32 bits as 32 E2M1 values (0.5 where the bit is set), in an order that is
-// the same for every row: 4-bit field f of word s takes bit 4 f + s.
+// 32 bits as 32 E2M1 values (2.0 where the bit is set), in an order that is
+// the same for every row: 4-bit field f of word s takes bit 4 f + 2 - s (bit 4 f
+// + 3 for s = 3).  Bit 2 of a field is 2.0, and the two shifts to the left can be
+// multiplications, off the ALU pipe.
 __device__ __forceinline__ uint4 tc_spread(uint32_t v) {
-    return make_uint4(v & 0x11111111u, (v >> 1) & 0x11111111u, (v >> 2) & 0x11111111u,
-                      (v >> 3) & 0x11111111u);
+    return make_uint4(v & 0x44444444u, (v * 2u) & 0x44444444u, (v * 4u) & 0x44444444u,
+                      (v >> 1) & 0x44444444u);
 }
+constexpr float kTcSpreadUnit = 0.25f;  // times a sum of products: the count
 
 }  // namespace gsdr
