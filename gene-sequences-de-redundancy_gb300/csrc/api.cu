@@ -74,6 +74,7 @@ struct Plan {
     bool bits = false;      // batched word filter by k-mer presence bitmaps
     bool masks = false;     // batched word filter by tentative masks
     int hbuckets = 0;       // that form by hashed k-mer counts, their buckets
+    int ents_max = 0;       // its longest k-mer list
     int mask_planes = 8;    // their count planes (10 where a read has over 255 entries)
     // pigeon filter (p 1): low 16 bits of each read's offset in the
     // reference's padded layout (copyData, func.cu:119-137: L/16*16 + 16 per read)
@@ -188,6 +189,7 @@ int make_plan(const gsdr_reads* reads, const gsdr_opts& o, Plan& P, PlanPreset* 
         if (masks) index = false;
         P.bits = bits;
         P.masks = masks;
+        P.ents_max = (int)ents_max;
         if (masks) P.hbuckets = hash_buckets(P.max_len, k, o.threshold);
         // automatic R: the largest, except for the table form at k = 7, whose
         // tables hold only 4 tentatives per CTA (200k reads of 150-5,000 bp at
@@ -270,9 +272,14 @@ size_t carve_all(char* base, int n, int64_t n_bytes, const Plan& P, bool drop, i
     // (four alignment queues' worth: a pass whose open pairs overflow it is redone)
     B.amb_cap = P.bits || P.masks ? 4 * B.seg_cap : 0;
     B.amb = P.bits || P.masks ? c.take<Pair>((size_t)B.amb_cap) : nullptr;
-    B.amb2 = P.bits || P.masks ? c.take<Pair>((size_t)B.amb_cap) : nullptr;
-    B.amb_idx = P.bits || P.masks ? c.take<int32_t>(4 * (size_t)(kMaxBatch + 1)) : nullptr;
+    // (sorted by tentative, except in the hashed form)
+    const bool sorted_amb = P.bits || (P.masks && !P.hbuckets);
+    B.amb2 = sorted_amb ? c.take<Pair>((size_t)B.amb_cap) : nullptr;
+    B.amb_idx = sorted_amb ? c.take<int32_t>(4 * (size_t)(kMaxBatch + 1)) : nullptr;
     R.hbuckets = P.hbuckets;
+    // tables of at least twice the longest list (at most kMaskMaxEntries)
+    R.hslots = 64;
+    while (R.hslots < 2 * P.ents_max && P.hbuckets) R.hslots <<= 1;
     R.hrow = P.hbuckets ? c.take<uint4>((size_t)n * (P.hbuckets / 32)) : nullptr;
     R.hextra = P.hbuckets ? c.take<int32_t>(n) : nullptr;
     const bool tmasks = P.masks && !P.hbuckets;

@@ -85,6 +85,7 @@ struct DevReads {
     uint4* hrow;
     int32_t* hextra;
     int32_t hbuckets;
+    int32_t hslots;      // k_bexact_d's table
     // pigeon filter (p 1; null otherwise), the reference's 4-mer position
     // index: pig[256 i + v] = inclusive prefix of read i's 4-mer bucket counts
     // (u16), pidx[off[i] + slot] = (u16) absolute position of a window's last

@@ -1990,6 +1990,117 @@ __global__ void __launch_bounds__(kAmbThreads) k_bexact_t(DevReads R, RoundState
     if (lane == 0 && n_al) atomicAdd(&st->cnt_aligned, (unsigned long long)n_al);
 }
 
+// The word sum S of the open pairs where reads are short (the hashed form: at
+// most 1,023 k-mers): one warp per pair, straight from the queue.  The
+// representative's k-mers set bits of a presence bitmap of the warp's own in
+// shared memory, the candidate's look them up: D shared k-mers and the two
+// reads' excesses over distinct k-mers bound S (D <= S <= D + the smaller
+// excess).  In short reads few k-mers repeat, so that decides nearly every
+// pair; the rest is summed with an open-addressed table in the same place
+// (hslots words, a power of two and at least twice the longest list).
+//
+// Instruction issue and the chain of loads (pair, offsets, lists: ~10 us in a
+// pass of few pairs) bound it.  1M reads of 100-150 bp, k = 7, t = 0.90, passes
+// of ~25,000 open pairs: 17 us; 38 us with a table for every pair (850
+// instructions each); 62 us sorted by tentative with a table of all k-mers
+// each, as for longer reads (32 KB of table for some 25 pairs).  The job's
+// passes: 140.4 -> 130.9 ms.
+constexpr int kDirectWarps = 8;
+constexpr int kDirectMaxSlots = 2048;
+
+__device__ __forceinline__ int direct_words(const DevReads& R) {
+    return max(R.hslots, (1 << (2 * R.k)) / 32);
+}
+
+// S by the table; the lists are distinct k-mers, so the table's inserts end.
+__device__ __noinline__ int direct_sum(uint32_t* tab, int slots, const uint32_t* er, int nr,
+                                       const uint32_t* eq, int nq) {
+    constexpr uint32_t kEmpty = 0xffffffffu;  // no entry: a k-mer has at most 14 bits
+    const int lane = threadIdx.x & 31, mask = slots - 1, shift = 33 - __ffs(slots);
+    for (int i = lane; i < slots; i += 32) tab[i] = kEmpty;
+    __syncwarp();
+    for (int i = lane; i < nr; i += 32) {
+        const uint32_t v = __ldg(er + i);
+        int h = ((v >> 16) * 0x9e3779b1u) >> shift;
+        for (int n = 0; n < slots && atomicCAS(tab + h, kEmpty, v) != kEmpty; n++)
+            h = (h + 1) & mask;
+    }
+    __syncwarp();
+    int sum = 0;
+    for (int i = lane; i < nq; i += 32) {
+        const uint32_t v = __ldg(eq + i);
+        int h = ((v >> 16) * 0x9e3779b1u) >> shift;
+        uint32_t e = tab[h];
+        for (int n = 0; n < slots && e != kEmpty && e >> 16 != v >> 16; n++)
+            e = tab[h = (h + 1) & mask];
+        if (e >> 16 == v >> 16) sum += (int)min(e & 0xffffu, v & 0xffffu);
+    }
+    __syncwarp();
+    return __reduce_add_sync(kFull, sum);
+}
+
+__global__ void __launch_bounds__(32 * kDirectWarps) k_bexact_d(DevReads R, RoundState* st,
+                                                              const Pair* __restrict__ amb,
+                                                              int amb_cap, Pair* pairs,
+                                                              int seg_cap) {
+    extern __shared__ __align__(16) uint32_t dtab[];
+    constexpr int U = 5;  // 150 bp reads in one go
+    chain_wait();
+    if (st->done || st->n_tent == 0) return;
+    const int na = amb_n(st, amb_cap);
+    const int nw = gridDim.x * kDirectWarps;
+    const int lane = threadIdx.x & 31;
+    if (blockIdx.x * kDirectWarps >= na) return;
+    const int words = (1 << (2 * R.k)) / 32;
+    uint32_t* bits = dtab + (threadIdx.x >> 5) * direct_words(R);
+    unsigned n_al = 0;
+    for (int k = blockIdx.x * kDirectWarps + (threadIdx.x >> 5); k < na; k += nw) {
+        const Pair p = amb[k];
+        const uint32_t* er = R.kmer + R.kmer_off[p.rep];
+        const uint32_t* eq = R.kmer + R.kmer_off[p.cand];
+        const int nr = R.n_kmer[p.rep], nq = R.n_kmer[p.cand];
+        const int cw = R.cut_word[p.cand];
+        for (int i = lane; i < words / 4; i += 32)
+            reinterpret_cast<uint4*>(bits)[i] = make_uint4(0u, 0u, 0u, 0u);
+        __syncwarp();
+        // (an absent entry stands as a k-mer with count 1 that sets no bit)
+        int ex_r = 0, d_ex = 0;  // d_ex: the candidate's excess << 16 | shared k-mers
+        for (int i0 = lane; i0 < nr; i0 += 32 * U) {
+            uint32_t v[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) v[u] = i0 + 32 * u < nr ? __ldg(er + i0 + 32 * u) : 1u;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (i0 + 32 * u < nr) atomicOr(bits + (v[u] >> 21), 1u << ((v[u] >> 16) & 31));
+                ex_r += (int)(v[u] & 0xffffu) - 1;
+            }
+        }
+        __syncwarp();
+        for (int i0 = lane; i0 < nq; i0 += 32 * U) {
+            uint32_t v[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) v[u] = i0 + 32 * u < nq ? __ldg(eq + i0 + 32 * u) : 1u;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const uint32_t hit = bits[v[u] >> 21] >> ((v[u] >> 16) & 31) & 1u;
+                d_ex += (int)((v[u] & 0xffffu) - 1u) << 16;
+                d_ex += i0 + 32 * u < nq ? (int)hit : 0;
+            }
+        }
+        __syncwarp();
+        ex_r = __reduce_add_sync(kFull, ex_r);
+        d_ex = __reduce_add_sync(kFull, d_ex);
+        int sum = d_ex & 0xffff;
+        if (sum < cw && sum + min(ex_r, d_ex >> 16) >= cw)
+            sum = direct_sum(bits, R.hslots, er, nr, eq, nq);
+        if (sum >= cw) {
+            if (lane == 0) push_pair(st, pairs, seg_cap, R, p.rep, p.cand, kBandMaxW);
+            n_al++;
+        }
+    }
+    add_counts(st, lane, 0, 0, n_al, 0);
+}
+
 // ---- word filter by inverted index (sparse k-mer spaces) -------------------
 //
 // With short reads and k = 7 a tentative holds ~1% of the 4^k k-mers, so the
@@ -3278,17 +3389,21 @@ void launch_bfilter_bits_t(const DevReads& R, RoundBuffers& B, const int32_t* re
     launch_exact_t<K>(R, B, s);
 }
 
-template <int K>
-void launch_bfilter_hash_t(const DevReads& R, RoundBuffers& B, const int32_t* remain,
+void launch_bfilter_hash(const DevReads& R, RoundBuffers& B, const int32_t* remain,
                            cudaStream_t s) {
     static bool attr = false;
     if (!attr) {
         cudaFuncSetAttribute(k_bfilter_hash, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kHashSmem);
+        cudaFuncSetAttribute(k_bexact_d, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kDirectWarps * kDirectMaxSlots * (int)sizeof(uint32_t));
         attr = true;
     }
     launch_next(B, k_bfilter_hash, num_sms(), kHashThreads, kHashSmem, s, R, B.st, remain, B.tent, B.amb, B.amb_cap);
-    launch_exact_t<K>(R, B, s);
+    const int words = std::max(R.hslots, (1 << (2 * R.k)) / 32);  // as direct_words()
+    const int smem = kDirectWarps * words * (int)sizeof(uint32_t);
+    const int grid = num_sms() * std::min(8, 220 * 1024 / (smem + 1024));
+    launch_next(B, k_bexact_d, shaped(grid, R.filter_blocks), 32 * kDirectWarps, smem, s, R, B.st, B.amb, B.amb_cap, B.pairs, B.seg_cap);
 }
 
 template <int K>
@@ -3330,12 +3445,7 @@ void launch_filter_any(const DevReads& R, RoundBuffers& B, const int32_t* remain
         return;
     }
     if (BATCH && !drop && R.hbuckets) {
-        switch (R.k) {
-            case 4: launch_bfilter_hash_t<4>(R, B, remain, s); break;
-            case 5: launch_bfilter_hash_t<5>(R, B, remain, s); break;
-            case 6: launch_bfilter_hash_t<6>(R, B, remain, s); break;
-            default: launch_bfilter_hash_t<7>(R, B, remain, s); break;
-        }
+        launch_bfilter_hash(R, B, remain, s);
         return;
     }
     if (BATCH && !drop && B.tmask) {
@@ -3573,10 +3683,11 @@ void launch_batch_pass(const DevReads& R, RoundBuffers& B, int drop, int parity,
     if (ev4) cudaEventRecordWithFlags(ev4[3], s, cudaEventRecordExternal);
     if (count)
         *count += 4 + align_launches<true>(R, B) + (!drop ? 1 : 0) +
-                  (R.pig_q && !drop ? 1 : 0) + (B.amb && !drop ? 4 : 0);
-    // (a word-filter form launches two kernels, six with the open-pair
-    // queue: the bitmap form k_filter, k_bfilter_bits, the mask form k_bmask,
-    // k_bfilter_mask, then k_amb_count, k_amb_scan, k_amb_place, k_bexact_t)
+                  (R.pig_q && !drop ? 1 : 0) + (B.amb && !drop && !R.hbuckets ? 4 : 0);
+    // (a word-filter form launches two kernels, six with the sorted queue of
+    // open pairs: the bitmap form k_filter, k_bfilter_bits, the mask form
+    // k_bmask, k_bfilter_mask, then k_amb_count, k_amb_scan, k_amb_place,
+    // k_bexact_t; the hashed form k_bfilter_hash and k_bexact_d)
 }
 
 // Whether a job's per-pass k-mer index (at most `cap` postings) is kept in

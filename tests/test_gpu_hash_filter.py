@@ -60,3 +60,20 @@ def test_both_sides_of_the_rule(tmp_path, length):
     # from some length on the job takes the tentative masks instead (the same form)
     data = gsdr.synth_fasta(2, n_reads=1200, seed=74, len_lo=length, len_hi=length)
     _check(tmp_path, data, 0.90, word_filter=4)
+
+
+@pytest.mark.parametrize("unit", [0, 3, 40, 400])
+def test_open_pairs_of_long_lists(tmp_path, unit):
+    # lists of up to ~900 k-mers: several loads of a lane's five entries, the
+    # largest tables; repeats of `unit` bases raise the counts, so that the
+    # presence bits leave pairs open and the tables form their sums
+    rng = np.random.default_rng(75)
+    recs = []
+    for i in range(400):
+        base = rng.integers(0, 4, 900) if not unit else np.tile(rng.integers(0, 4, unit), 900)[:900]
+        for v in range(3):
+            s = base.copy()
+            at = rng.integers(0, 900, (8, 20, 30)[v])
+            s[at] = rng.integers(0, 4, at.size)
+            recs.append(f">r{i}_{v}\n{''.join('ACGT'[x] for x in s[:900 - 7 * v])}\n")
+    _check(tmp_path, "".join(recs).encode(), 0.97, word_length=7, word_filter=4)
