@@ -69,6 +69,7 @@ struct Plan {
     std::vector<int64_t> pack_off, kmer_off;
     int64_t max_len = 0;
     int r_max = 1;          // largest R (tentatives per pass)
+    bool r_auto = false;    // not the caller's
     int64_t idx_cap = 0;    // > 0: batched word filter by inverted index, postings capacity
     bool idx_smem = false;  // that index fits the filter's shared memory (16-bit copy)
     bool bits = false;      // batched word filter by k-mer presence bitmaps
@@ -121,6 +122,7 @@ int make_plan(const gsdr_reads* reads, const gsdr_opts& o, Plan& P, PlanPreset* 
     const bool drop = o.drop == 1;
     const int k = o.word_length;
     P.variant = o.variant;
+    P.r_auto = o.batch == 0;
     P.r_max = (o.batch == 1 || (!drop && k >= kWideK)) ? 1 : job_r_max(o);
     const int64_t kcap = (int64_t)1 << (2 * (k > 0 ? k : 1));
     // the per-read layout (plan_chunks.h): the caller's, when it computed it
@@ -263,6 +265,7 @@ size_t carve_all(char* base, int n, int64_t n_bytes, const Plan& P, bool drop, i
     B.acc_cap = 2 * B.seg_cap;
     B.acc = c.take<Pair>((size_t)B.acc_cap);
     B.r_max = P.r_max;
+    B.r_auto = P.r_auto;
     B.idx_cap = P.idx_cap;
     B.idx_off = P.idx_cap > 0 ? c.take<uint32_t>(((size_t)1 << (2 * k)) + 1) : nullptr;
     B.idx_post = P.idx_cap > 0 ? c.take<uint32_t>((size_t)P.idx_cap) : nullptr;

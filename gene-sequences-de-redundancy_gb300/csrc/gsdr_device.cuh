@@ -222,6 +222,7 @@ struct RoundBuffers {
     uint16_t* idx_off16;   // 16-bit copies for the shared-memory form (null otherwise)
     uint16_t* idx_post16;
     int64_t idx_cap;
+    int32_t r_auto;      // the caller left R to the job
     int32_t r_max;       // largest R of the job (sizes the index filter's shared memory)
     // batched word filter by k-mer presence bitmaps or by tentative masks
     // (null = another form): pairs the bound D <= S <= D + min(excess)

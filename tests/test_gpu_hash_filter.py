@@ -77,3 +77,18 @@ def test_open_pairs_of_long_lists(tmp_path, unit):
             s[at] = rng.integers(0, 4, at.size)
             recs.append(f">r{i}_{v}\n{''.join('ACGT'[x] for x in s[:900 - 7 * v])}\n")
     _check(tmp_path, "".join(recs).encode(), 0.97, word_length=7, word_filter=4)
+
+
+def test_full_groups_of_tentatives(tmp_path):
+    # enough remaining reads for passes that take only full groups of tentatives,
+    # and later ones that take R_max; a caller's R is taken as it is
+    data = gsdr.synth_fasta(2, n_reads=230_000, seed=76, n_seeds=40_000)
+    f = gsdr.Fasta.parse(data)
+    try:
+        a, sa = gsdr.clustering(f, gsdr.default_opts(threshold=0.90), stats=True)
+        b, sb = gsdr.clustering(f, gsdr.default_opts(threshold=0.90, batch=512), stats=True)
+    finally:
+        f.close()
+    assert sa.word_index == sb.word_index == 3
+    assert sa.batch == 1024
+    np.testing.assert_array_equal(a, b)
