@@ -251,6 +251,9 @@ size_t carve_all(char* base, int n, int64_t n_bytes, const Plan& P, bool drop, i
     R.kextra = bits ? c.take<int32_t>(n) : nullptr;
     R.kbits2 = P.bits ? c.take<uint32_t>((size_t)n * nbw) : nullptr;
     R.kextra3 = P.bits ? c.take<int32_t>(n) : nullptr;
+    const bool folds = P.bits && k >= kMinFoldK;
+    R.kfold = folds ? c.take<uint32_t>((size_t)n * (nbw / 2 + nbw / 4)) : nullptr;
+    R.kfextra = folds ? c.take<int32_t>(2 * (size_t)n) : nullptr;
     B.st = reinterpret_cast<RoundState*>(c.take<char>(sizeof(RoundState) + 4 * 64));
     B.cluster = c.take<int32_t>(n);
     B.remain[0] = c.take<int32_t>(n);

@@ -40,6 +40,7 @@ constexpr int kMaxBatch = 1024;         // tentative representatives per batched
 constexpr int kTTWords = kMaxBatch / 32;
 constexpr int kMaxBitsK = 6;            // k-mer presence bitmaps for k <= 6 (4^k bits per read)
 constexpr int kMaxBits2K = 7;           // the batched two-level bitmap filter: k <= 7
+constexpr int kMinFoldK = 6;  // word lengths with folded bitmaps
 constexpr int kMaskMaxEntries = 1023;   // tentative-mask filter: reads of at most 1,023 k-mers
 constexpr int kMaskEntries8 = 255;      // ... with eight count planes up to 255, else ten
 
@@ -79,6 +80,12 @@ struct DevReads {
     // max(count - 2, 0)
     uint32_t* kbits2;
     int32_t* kextra3;
+    // batched bitmap filter with k >= 6 (null otherwise): bitmaps of 4^k / 2
+    // and 4^k / 4 bits, the presence bitmap's halves and quarters or'd (all
+    // reads' halves, then all quarters), and their excesses, sum(count) - set
+    // bits (n each)
+    uint32_t* kfold;
+    int32_t* kfextra;
     // batched filter by hashed k-mer counts only (hbuckets 0 otherwise): per
     // read a row of hbuckets 4-bit counts (hbuckets / 32 16-byte words) and
     // the excess over 144 of its buckets' counts (rounds.cu, k_bfilter_hash)
@@ -156,6 +163,10 @@ struct RoundState {
     int32_t acc_overflow;
     int32_t survivors;  // representatives confirmed this pass
     int32_t absorbed;   // reads absorbed this pass
+    int32_t bits_depth;    // bitmaps of the last pass (k_bfilter_bits)
+    int32_t bits_cap;      // the most that the next bits_hold passes may take
+    int32_t bits_hold;
+    int32_t bits_fails;    // passes that left too many pairs open
     int32_t n_amb;      // pairs the bitmap or mask bound left to the exact word filter
     int32_t n_pig;      // pairs queued for the pigeon filter
     int32_t ticket;     // blocks of the compaction that have finished

@@ -205,7 +205,8 @@ __global__ void __launch_bounds__(256) k_kmers_hist(DevReads R) {
     uint32_t* hist = sm;
     uint16_t* list = reinterpret_cast<uint16_t*>(sm + NB);
     __shared__ uint32_t bits[NBW], bits2[NBW];
-    __shared__ int nlist, sumcnt, sum3;
+    __shared__ int nlist, sumcnt, sum3, lost2, lost4;
+    const bool folds = BITS_T && K >= kMinFoldK && R.kfold != nullptr;
     const bool BITS = BITS_T && R.kbits != nullptr;
     const bool level2 = BITS && R.kbits2 != nullptr;
     for (int i = threadIdx.x; i < NB; i += blockDim.x) hist[i] = 0;
@@ -214,6 +215,7 @@ __global__ void __launch_bounds__(256) k_kmers_hist(DevReads R) {
         nlist = 0;
         sumcnt = 0;
         sum3 = 0;
+        lost2 = lost4 = 0;
     }
     __syncthreads();
     for (int r = blockIdx.x; r < R.n; r += gridDim.x) {
@@ -260,7 +262,37 @@ __global__ void __launch_bounds__(256) k_kmers_hist(DevReads R) {
         __syncthreads();
         if (BITS) {
             uint32_t* ob = R.kbits + (size_t)r * NBW;
-            for (int i = threadIdx.x; i < NBW; i += blockDim.x) {
+            if (folds) {
+                // a thread owns the four words that fold together
+                constexpr int Q = NBW / 4;
+                uint32_t* o2 = R.kfold + (size_t)r * (2 * Q);
+                uint32_t* o4 = R.kfold + (size_t)R.n * (2 * Q) + (size_t)r * Q;
+                int l2 = 0, l4 = 0;  // bits lost to another k-mer's
+                for (int i = threadIdx.x; i < Q; i += blockDim.x) {
+                    uint32_t w[4];
+                    int set = 0;
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        w[j] = bits[i + j * Q];
+                        ob[i + j * Q] = w[j];
+                        bits[i + j * Q] = 0;
+                        set += __popc(w[j]);
+                    }
+                    const uint32_t a = w[0] | w[2], b = w[1] | w[3];
+                    o2[i] = a;
+                    o2[i + Q] = b;
+                    o4[i] = a | b;
+                    l2 += set - __popc(a) - __popc(b);
+                    l4 += set - __popc(a | b);
+                }
+                l2 = warp_sum(l2);
+                l4 = warp_sum(l4);
+                if ((threadIdx.x & 31) == 0) {
+                    if (l2) atomicAdd(&lost2, l2);
+                    if (l4) atomicAdd(&lost4, l4);
+                }
+                __syncthreads();
+            } else for (int i = threadIdx.x; i < NBW; i += blockDim.x) {
                 ob[i] = bits[i];
                 bits[i] = 0;
             }
@@ -276,6 +308,11 @@ __global__ void __launch_bounds__(256) k_kmers_hist(DevReads R) {
             R.n_kmer[r] = nl;
             if (BITS) R.kextra[r] = sumcnt;
             if (level2) R.kextra3[r] = sum3;
+            if (folds) {
+                R.kfextra[r] = sumcnt + lost2;
+                R.kfextra[(size_t)R.n + r] = sumcnt + lost4;
+                lost2 = lost4 = 0;
+            }
             nlist = 0;
             sumcnt = 0;
             sum3 = 0;

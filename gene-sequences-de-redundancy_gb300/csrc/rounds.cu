@@ -80,6 +80,11 @@ constexpr int kAbsorbHigh = 64;     // absorbed reads per representative that sh
 // 27 more passes).  On 200k reads at t = 0.95, where the filter is a smaller
 // part of a pass, 960 throughout took 1% longer.
 constexpr int kEvenRemain = 200000;
+// Shorter bitmaps of k_bfilter_bits: 1 one level, 2 folded to half, 3 to a quarter.
+constexpr int kMaxDepth = 3;
+// Open pairs of a pass, one in so many, above which the next passes take longer
+// bitmaps than the estimate asks for.
+constexpr int kOpenLimit = 128;
 constexpr int kFewPairs = 16384;    // queued pairs below which R grows 8x, not 2x
 // Widest band window (words) sent to the lane-banded kernel: batched passes,
 // plain rounds.  A plain round waits for its slowest pair, and a lane works
@@ -1043,6 +1048,16 @@ __device__ void advance_batch(RoundState* st, const int32_t* tent, int seg_cap,
         st->done = 1;
         return;
     }
+    // shorter bitmaps that left too many pairs open (reads that are less
+    // random than the filter's estimate assumes): longer ones for some passes,
+    // twice as many every time
+    if (st->bits_hold > 0) st->bits_hold--;
+    if (st->bits_depth > 0 &&
+        (long long)kOpenLimit * st->n_amb > (long long)st->n_tent * st->n_remain) {
+        st->bits_cap = st->bits_depth - 1;
+        st->bits_hold = 1 << min(++st->bits_fails, 16);
+    }
+    st->bits_depth = 0;
     if (st->pair_overflow || st->acc_overflow) {
         // queues too small for this many tentatives: the pass changed nothing
         // (the compaction copied the remain list unchanged); redo it with fewer
@@ -1525,35 +1540,54 @@ __global__ void __launch_bounds__(kFilterThreads) k_bprefilter(DevReads R, Round
 // multiplications, a shift and four masks per 32 k-mers), accumulators in
 // tensor memory.
 //
+// A pass takes as short bitmaps as decide its pairs: both levels (depth 0),
+// the first alone (1: S <= D + the smaller sum(count - 1)), or the first with
+// its halves or quarters or'd together (2, 3: k-mers that share a bit count as
+// one, their counts added; D no longer bounds S from below).  Every CTA
+// estimates, from a sample of the pass's own pairs taken as unrelated reads,
+// how many each depth would leave open, and takes the cheapest: the longest
+// reads need both levels (5,000 bp hold most of the 6-mers),
+// reads of 1,000 bp a quarter of the first.
+//
 // A CTA per SM: one warp issues the MMAs, 23 warps load and spread the
-// bitmaps into a ring of four stages (256 k-mers of every row), and four warps
+// bitmaps into a ring of two stages (512 k-mers of every row), and four warps
 // read the finished tile's sums, apply the composition bound and queue the
 // pairs while the next tile is summed in the other accumulator.  A producer
 // lane loads 16 bytes of a row, eight lanes 128 contiguous bytes, and word w of
-// its 16 bytes goes to the w-th of four stages: full lines from L2 and whole
+// its 16 bytes goes to the w-th chunk of 256 k-mers: full lines from L2 and whole
 // rows of shared memory per store.
 //
-// 84,800 candidates x 1,024 tentatives, k = 6: 0.42 ms (2.1e11 pairs/s), ALU
-// pipe 71% (the spread and the composition bound), shared-memory pipe 64%,
-// tensor pipe 35%; the AND + POPC kernel before it took about 3 ms.  With
-// two of the spread's shifts as multiplications (off the ALU pipe) the filter
-// stage of the first workload below went from 26.3 to 23.9 ms.
-// Filter stage: 149 -> 24 ms (100k reads of 150-5,000 bp, t = 0.95),
-// 42 -> 5.9 ms (30k, t = 0.90, k = 7, with R_max 1024 instead of 256, which the
-// lanes' form could not stage), 2.36 -> 0.88 ms (10k reads of 200-1,000 bp).
-// On the way there: eight producer loads of 32 bytes of a row each (shared
-// pipe 71%, 0.49 ms); 12 producers (0.53 ms: every warp takes part in every
-// stage, so a stage lasts as long as one warp's share of it); the MMAs issued
-// by a producer (0.73 ms); branches per column in the epilogue (0.63 ms).
+// The producers' hand-overs bound it: every warp takes part in every stage, so
+// a stage lasts as long as one warp's wait, stores, fence and arrival.  Filter
+// stage of 100k reads of 150-5,000 bp, t = 0.95 (90 passes of up to 92,000 x
+// 1,024 pairs): 149 ms (AND + POPC lanes), 26.3 (four stages of 256 k-mers),
+// 23.9 (two of the spread's shifts as multiplications), 21.8 (the depths, and
+// an epilogue of 8 instead of ~17 ALU operations a pair, which alone changed
+// nothing), 19.7 (stages of 512 k-mers, splits of the tentatives that fill the
+// last wave).  30k reads, t = 0.90, k = 7: 42 -> 4.85 ms, with R_max 1024
+// instead of 256, which the lanes' form could not stage; 10k reads of 200-1,000
+// bp: 2.36 -> 0.75 ms.
+// On the way there, with four stages, 84,800 x 1,024 pairs, 0.42 ms: eight
+// producer loads of 32 bytes of a row each 0.49; 12 producers 0.53; the MMAs
+// issued by a producer 0.73; branches per column in the epilogue 0.63.
+// An open pair's exact sum (2 to 4 ns) in products of 1,024 bits of a pair (0.6
+// ps): what a shorter bitmap may leave open for what it saves.
+constexpr float kOpenCost = 6000.0f;
 constexpr int kBitsProducers = 23;  // 4 rows per 8 lanes, 28 warps: 72 registers each
 constexpr int kBitsEpilogue = 4;
 constexpr int kBitsThreads = 32 * (1 + kBitsEpilogue + kBitsProducers);
-constexpr int kBitsStages = 4;
-constexpr int kBitsStageBytes = (128 + kTcMaxN) * kTcRowBytes;
+constexpr int kBitsStages = 2;  // of two chunks of 256 k-mers
+constexpr int kBitsChunkBytes = (128 + kTcMaxN) * kTcRowBytes;
+constexpr int kBitsStageBytes = 2 * kBitsChunkBytes;
 constexpr int kTentPad = kMaxBatch + 16;  // a tile's columns are read sixteen at a time
-constexpr int kBitsSmem = 1024 + kBitsStages * kBitsStageBytes + kTentPad * (16 + 8);
+constexpr int kBitsSmem = 1024 + kBitsStages * kBitsStageBytes + kTentPad * (16 + 8 + 4 + 4);
 static_assert(128 % 8 == 0 && kTcMaxN % 16 == 0, "whole groups of eight rows");
 constexpr int kBitsRows = (128 + kTcMaxN + 4 * kBitsProducers - 1) / (4 * kBitsProducers);
+
+__device__ __forceinline__ uint2 comp_halves(const int4 c) {
+    return make_uint2((uint32_t)min(c.x, 0xffff) | (uint32_t)min(c.y, 0xffff) << 16,
+                      (uint32_t)min(c.z, 0xffff) | (uint32_t)min(c.w, 0xffff) << 16);
+}
 
 template <int K>
 __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
@@ -1561,25 +1595,39 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
     const int32_t* __restrict__ tent, Pair* pairs, int seg_cap, Pair* amb, int amb_cap) {
     constexpr int NQ = (1 << (2 * K)) / 128;        // 16-byte words of one bitmap
     constexpr int GL = NQ >= 8 ? NQ / 8 : 1;        // groups of four stages per level
-    constexpr int CH = 4 * (K == 4 ? 1 : 2 * GL);   // stages per tile (k = 4: half of them zeros)
+    constexpr int DEPTHS = K >= kMinFoldK ? kMaxDepth : K == 5 ? 1 : 0;
     extern __shared__ __align__(1024) uint8_t bsm_raw[];
     __shared__ uint64_t full[kBitsStages], empty[kBitsStages], tfull[2], tempty[2], drain;
     __shared__ uint32_t s_tmem;
-    __shared__ int s_quit;
+    __shared__ int s_quit, s_open[kMaxDepth + 1];
+    if (threadIdx.x <= kMaxDepth) s_open[threadIdx.x] = 0;
     chain_wait();
     if (st->done) return;
     const int nt = st->n_tent;
     if (nt <= 1) return;  // a single tentative's pass runs k_filter instead
     const int n = st->n_remain;
-    const int tiles_n = (nt + kTcMaxN - 1) / kTcMaxN;
+    const int lane = threadIdx.x & 31, mtiles = (n + 127) >> 7;
+    // The tentatives' split: a tile costs about its rows, candidates' and
+    // tentatives', and the launch the most tiles of a CTA.  Each lane weighs
+    // one split (every warp of every CTA finds the same).
+    int tiles_n = (nt + kTcMaxN - 1) / kTcMaxN + lane;
+    {
+        const int cols = (((nt + tiles_n - 1) / tiles_n) + 15) & ~15;
+        const int waves = (mtiles * tiles_n + (int)gridDim.x - 1) / (int)gridDim.x;
+        tiles_n = (int)(__reduce_min_sync(kFull, (unsigned)(waves * (128 + cols)) << 6 |
+                                                     (unsigned)tiles_n) & 63u);
+    }
     const int N = (((nt + tiles_n - 1) / tiles_n) + 15) & ~15;  // tentatives per tile
-    const int tiles = ((n + 127) >> 7) * tiles_n;
+    tiles_n = (nt + N - 1) / N;
+    const int tiles = mtiles * tiles_n;
     if ((int)blockIdx.x >= tiles) return;
     uint8_t* stage0 = reinterpret_cast<uint8_t*>(
         (reinterpret_cast<uintptr_t>(bsm_raw) + 1023) & ~(uintptr_t)1023);
     int4* tcomp = reinterpret_cast<int4*>(stage0 + kBitsStages * kBitsStageBytes);
-    int2* tte = reinterpret_cast<int2*>(tcomp + kTentPad);  // tentative and its excess
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint2* tpair = reinterpret_cast<uint2*>(tcomp + kTentPad);   // comp in 16-bit halves
+    float* tex = reinterpret_cast<float*>(tpair + kTentPad);     // excess / kTcSpreadUnit
+    int32_t* s_tent = reinterpret_cast<int32_t*>(tex + kTentPad);
+    const int warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
         for (int i = 0; i < kBitsStages; i++) {
             mbar_init(&full[i], kBitsProducers);
@@ -1596,14 +1644,53 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
     if (warp == 0) tmem_alloc_all(&s_tmem);
     for (int t = threadIdx.x; t < nt; t += blockDim.x) {
         const int rep = tent[t];
-        tcomp[t] = R.comp[rep];
-        tte[t] = make_int2(rep, R.kextra3[rep]);
+        const int4 c = R.comp[rep];
+        s_tent[t] = rep;
+        tcomp[t] = c;
+        tpair[t] = comp_halves(c);
+    }
+    __syncthreads();
+    if (DEPTHS > 0) {
+        // the chance that a sampled pair of unrelated reads stays open
+        const int rep = tent[threadIdx.x % nt];
+        const int q = remain[(int)((long long)threadIdx.x * n / kBitsThreads)];
+        const int xq = R.kextra[q], xr = R.kextra[rep], cw = R.cut_word[q];
+        const int kq = R.n_kmer[q] + xq, kr = R.n_kmer[rep] + xr;
+#pragma unroll
+        for (int d = 1; d <= DEPTHS; d++) {
+            const int eq = d == 1 ? xq : R.kfextra[(size_t)(d - 2) * R.n + q];
+            const int er = d == 1 ? xr : R.kfextra[(size_t)(d - 2) * R.n + rep];
+            const float w = 1.0f / (float)((1 << (2 * K)) >> (d - 1));
+            const float fq = (float)(kq - eq) * w, mean = (float)(kr - er) * fq;
+            const float var = mean * (1.0f - fq) * (1.0f - (float)(kr - er) * w);
+            const float z = ((float)(cw - min(eq, er)) - mean) * rsqrtf(2.0f * var + 1.0f);
+            int open = rep < q ? (int)(32768.0f * erfcf(z)) : 0;
+            open = __reduce_add_sync(kFull, open);
+            if (lane == 0 && open) atomicAdd(&s_open[d], open);
+        }
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
     if (warp >= 1 && warp <= 4) tc_fill_scales(tmem, warp);
+    int depth = 0;
+    float cost = (float)(2 * GL);
+#pragma unroll
+    for (int d = 1; d <= DEPTHS; d++) {
+        const float c = (float)(GL >> (d - 1)) +
+                        kOpenCost * (float)s_open[d] * (1.0f / (65536.0f * kBitsThreads));
+        if ((st->bits_hold == 0 || d <= st->bits_cap) && c < cost) depth = d, cost = c;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->bits_depth = depth;
+    // groups of two stages (1,024 bits) per tile (k = 4: half of them zeros)
+    const int groups = K == 4 ? 1 : depth == 0 ? 2 * GL : GL >> (depth - 1);
+    const int CH = 2 * groups;
+    const int32_t* ex = depth == 0   ? R.kextra3
+                        : depth == 1 ? R.kextra
+                                     : R.kfextra + (size_t)(depth - 2) * R.n;
+    for (int t = threadIdx.x; t < nt; t += blockDim.x)
+        tex[t] = (float)ex[s_tent[t]] * (1.0f / kTcSpreadUnit);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1623,8 +1710,11 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t a = tc_desc_lo(smem_u32(stage0 + s * kBitsStageBytes));
-                    tc_mma_stage(tmem + buf * kTcMaxN, tmem, a, a + 128 * kTcRowBytes / 16, idesc,
-                                 c == 0);
+#pragma unroll
+                    for (int u = 0; u < 2; u++)
+                        tc_mma_stage(tmem + buf * kTcMaxN, tmem, a + u * kBitsChunkBytes / 16,
+                                     a + (u * kBitsChunkBytes + 128 * kTcRowBytes) / 16, idesc,
+                                     c == 0 && u == 0);
                     tc_commit(&empty[s]);
                     if (++s == kBitsStages) s = 0, ph ^= 1;
                 }
@@ -1645,35 +1735,69 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
             if (idx < n) {
                 q = remain[idx];
                 cw = R.cut_word[q];
-                exq = R.kextra3[q];
+                exq = ex[q];
                 cq = R.comp[q];
                 cbq = R.cut_base[q] - R.strict;
-                if (t0 == 0) bytes += kCandFixedBytes + 2ull * 16 * NQ;  // once per launch
+                // once per launch
+                if (t0 == 0) bytes += kCandFixedBytes + (K == 4 ? 64ull : 128ull * groups);
             }
             const int buf = it & 1;
             ok = mbar_wait_warp(&tfull[buf], (it >> 1) & 1, limit, &s_quit);
             if (!ok) break;
             tc_fence_after();
             const uint32_t addr = tmem + ((uint32_t)(warp & 3) << 21) + buf * kTcMaxN;
+            // tentatives of the tile before q (the list ascends)
+            int ntq = q < 0 ? t0 : t1;
+            if (q >= 0 && q <= s_tent[t1 - 1]) {
+                int lo = t0, hi = t1;
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (s_tent[mid] < q) lo = mid + 1;
+                    else hi = mid;
+                }
+                ntq = lo;
+            }
+            // the sums' scale, and the composition in 16-bit halves (no row
+            // with a count above that takes the short form below)
+            const float cwf = (float)cw * (1.0f / kTcSpreadUnit);
+            const float exf = (float)exq * (1.0f / kTcSpreadUnit);
+            const uint2 ch = comp_halves(cq);
+            const bool halves = max(max(cq.x, cq.y), max(cq.z, cq.w)) <= 0xffff;
             for (int c0 = t0; c0 < t1; c0 += 16) {
                 uint32_t raw[16];
                 float v[16];
+                const int ncol = ntq - c0;
+                if (!__any_sync(kFull, ncol > 0)) break;
                 tc_load16(raw, addr + (c0 - t0));
                 tc_load_wait(raw, v);
-                // sixteen independent chains with no branch: which tentatives
-                // come before q and pass kernel_preFilter (func.cu:738-754),
-                // and which of those the bound does not reject
-                const int ncol = t1 - c0;
-                uint32_t before = 0, pre = 0, hit = 0;
+                if (__all_sync(kFull, ncol >= 16 && halves)) {
+                    // sixteen independent chains: the largest bound, and how
+                    // many fail kernel_preFilter (func.cu:738-754)
+                    float top[2] = {-1.0f, -1.0f};
+                    uint32_t fail[2] = {0, 0};
 #pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    const int t = c0 + j;  // (entries past nt: any values, masked below)
-                    const int2 te = tte[t];
-                    before |= te.x < q ? 1u << j : 0u;
-                    pre |= prefilter_pass(tcomp[t], cq, cbq) ? 1u << j : 0u;
-                    hit |= (int)(kTcSpreadUnit * v[j]) + min(te.y, exq) >= cw ? 1u << j : 0u;
+                    for (int j = 0; j < 16; j++) {
+                        const uint2 tp = tpair[c0 + j];
+                        const uint32_t d =
+                            __dp2a_lo(__vminu2(tp.x, ch.x), 0x0101u,
+                                      __dp2a_lo(__vminu2(tp.y, ch.y), 0x0101u, 0u - (uint32_t)cbq));
+                        fail[j & 1] += d >> 31;
+                        top[j & 1] = fmaxf(top[j & 1], v[j] + fminf(tex[c0 + j], exf));
+                    }
+                    if (!__any_sync(kFull, fmaxf(top[0], top[1]) >= cwf)) {
+                        n_pf += 16;
+                        n_wf += 16 - (fail[0] + fail[1]);
+                        continue;
+                    }
                 }
-                before &= ncol >= 16 ? 0xffffu : (1u << ncol) - 1u;
+                // a row at its own place in the tentatives, or a pair left open
+                uint32_t pre = 0, hit = 0;
+#pragma unroll
+                for (int j = 0; j < 16; j++) {  // (entries past nt: any values, masked below)
+                    pre |= prefilter_pass(tcomp[c0 + j], cq, cbq) ? 1u << j : 0u;
+                    hit |= v[j] + fminf(tex[c0 + j], exf) >= cwf ? 1u << j : 0u;
+                }
+                const uint32_t before = ncol >= 16 ? 0xffffu : ncol > 0 ? (1u << ncol) - 1u : 0u;
                 pre &= before;
                 hit &= pre;
                 n_pf += __popc(before);
@@ -1684,8 +1808,8 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
                     float vj = v[0];
 #pragma unroll
                     for (int i = 1; i < 16; i++) vj = j == i ? v[i] : vj;
-                    const int rep = tte[c0 + j].x;
-                    if ((int)(kTcSpreadUnit * vj) >= cw) {
+                    const int rep = s_tent[c0 + j];
+                    if (depth < 2 && vj >= cwf) {
                         push_pair(st, pairs, seg_cap, R, rep, q, kBandMaxW);
                         n_al++;
                     } else {
@@ -1714,8 +1838,10 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
         // producers: lane piece p = lane % 8 (16 bytes of 128) of rows r0 +
         // 92 j (rows 0..127: the tile's candidates, then its tentatives)
         const int tid = threadIdx.x - 32 * (1 + kBitsEpilogue);
-        const uint4* kb1 = reinterpret_cast<const uint4*>(R.kbits);
+        const uint4* kb1 = reinterpret_cast<const uint4*>(
+            depth < 2 ? R.kbits : R.kfold + (depth == 3 ? (size_t)R.n * (2 * NQ) : 0));
         const uint4* kb2 = reinterpret_cast<const uint4*>(R.kbits2);
+        const int rowq = depth < 2 ? NQ : NQ >> (depth - 1);
         const int p = tid & 7, r0 = tid >> 3;
         constexpr int RS = 4 * kBitsProducers;  // rows per sweep
         static_assert(RS % 8 == 4 && RS * kBitsRows == 128 + kTcMaxN, "row layout");
@@ -1745,11 +1871,11 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
                     v[j] = make_uint4(0u, 0u, 0u, 0u);
                     if (p < 4) v[j] = __ldg((p < 2 ? kb1 : kb2) + (size_t)cur[j] * NQ + (p & 1));
                 } else {
-                    v[j] = __ldg((fg < GL ? kb1 : kb2) + (size_t)cur[j] * NQ +
+                    v[j] = __ldg((fg < GL ? kb1 : kb2) + (size_t)cur[j] * rowq +
                                  8 * (fg & (GL - 1)) + p);
                 }
             }
-            if (++fg == CH / 4) {
+            if (++fg == groups) {
                 fg = 0;
                 ft += gridDim.x;
 #pragma unroll
@@ -1761,20 +1887,21 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
         };
         int s = 0;
         uint32_t ph = 1;  // the first round of stages is free
-        // the four stages of one group
+        // the two stages of one group
         auto store = [&](const uint4 (&v)[kBitsRows]) {
 #pragma unroll
-            for (int w = 0; w < 4; w++) {
+            for (int w = 0; w < 4; w += 2) {
                 ok = mbar_wait_warp(&empty[s], ph, limit, &s_quit);
                 if (!ok) return;
                 uint8_t* base = stage0 + s * kBitsStageBytes + off0;
 #pragma unroll
                 for (int j = 0; j < kBitsRows; j++) {
                     // (row r0 + RS j: RS is 4 mod 8, so the swizzle alternates)
-                    if (j < rows)
-                        *reinterpret_cast<uint4*>(base + j * RS * kTcRowBytes +
-                                                  (j & 1 ? odd : 0)) =
-                            tc_spread(w == 0 ? v[j].x : w == 1 ? v[j].y : w == 2 ? v[j].z : v[j].w);
+                    if (j >= rows) break;
+                    uint8_t* d = base + j * RS * kTcRowBytes + (j & 1 ? odd : 0);
+                    *reinterpret_cast<uint4*>(d) = tc_spread(w ? v[j].z : v[j].x);
+                    *reinterpret_cast<uint4*>(d + kBitsChunkBytes) =
+                        tc_spread(w ? v[j].w : v[j].y);
                 }
                 fence_async_smem();
                 __syncwarp();
@@ -1783,7 +1910,7 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
             }
         };
         const int mine =
-            (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * (CH / 4);
+            (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * groups;
         uint4 va[kBitsRows], vb[kBitsRows];
         load(va);
         for (int i = 0; ok && i < mine; i += 2) {
