@@ -194,22 +194,31 @@ __device__ __forceinline__ bool window_broken(const uint32_t* brk, int p, int k)
     return ((v >> sh) & ((1ull << nbits) - 1ull)) != 0ull;
 }
 
-template <int K>
+// SHORT (reads of at most kMaskMaxEntries k-mers): counts in 16-bit halves and a
+// list of that many, 34 KB instead of 96 at k = 7, so that an SM counts six
+// reads at a time instead of two (their four barriers bound a read of 150 bp):
+// 1M reads of 100-150 bp 4.12 -> 1.49 ms.
+constexpr int kShortThreads = 128;
+constexpr int kShortList = (kMaskMaxEntries + 4) & ~3;
+
+template <int K, bool SHORT>
 __global__ void __launch_bounds__(256) k_kmers_hist(DevReads R) {
     constexpr int NB = 1 << (2 * K);
+    constexpr int HW = SHORT ? NB / 2 : NB;  // words of the histogram
     // presence bitmaps: k <= 6 always (the plain filter's bound), k = 7 only
     // for the batched two-level filter (kbits allocated)
-    constexpr bool BITS_T = K <= kMaxBits2K;
+    constexpr bool BITS_T = K <= (SHORT ? kMaxBitsK : kMaxBits2K);
     constexpr int NBW = BITS_T ? NB / 32 : 1;
     extern __shared__ __align__(16) uint32_t sm[];
     uint32_t* hist = sm;
-    uint16_t* list = reinterpret_cast<uint16_t*>(sm + NB);
+    uint16_t* half = reinterpret_cast<uint16_t*>(sm);
+    uint16_t* list = reinterpret_cast<uint16_t*>(sm + HW);
     __shared__ uint32_t bits[NBW], bits2[NBW];
     __shared__ int nlist, sumcnt, sum3, lost2, lost4;
     const bool folds = BITS_T && K >= kMinFoldK && R.kfold != nullptr;
     const bool BITS = BITS_T && R.kbits != nullptr;
     const bool level2 = BITS && R.kbits2 != nullptr;
-    for (int i = threadIdx.x; i < NB; i += blockDim.x) hist[i] = 0;
+    for (int i = threadIdx.x; i < HW; i += blockDim.x) hist[i] = 0;
     for (int i = threadIdx.x; i < NBW; i += blockDim.x) bits[i] = bits2[i] = 0;
     if (threadIdx.x == 0) {
         nlist = 0;
@@ -229,7 +238,11 @@ __global__ void __launch_bounds__(256) k_kmers_hist(DevReads R) {
             const int w = p >> 4, o = p & 15;
             const uint64_t v = ((uint64_t)__ldg(pk + w) << 32) | __ldg(pk + w + 1);
             const uint32_t km = (uint32_t)(v >> (64 - 2 * o - 2 * K)) & (uint32_t)(NB - 1);
-            const uint32_t old = atomicAdd(&hist[km], 1u);
+            uint32_t old;
+            if (SHORT)
+                old = (atomicAdd(&hist[km >> 1], 1u << (16 * (km & 1))) >> (16 * (km & 1))) & 0xffffu;
+            else
+                old = atomicAdd(&hist[km], 1u);
             if (old == 0) list[atomicAdd(&nlist, 1)] = (uint16_t)km;
         }
         __syncthreads();
@@ -237,9 +250,11 @@ __global__ void __launch_bounds__(256) k_kmers_hist(DevReads R) {
         int my_sum = 0, my_sum3 = 0;
         for (int s = threadIdx.x; s < nl; s += blockDim.x) {
             const uint32_t km = list[s];
-            const uint32_t c = hist[km] & 0xffffu;  // the reference's u16 multiplicity
+            // the reference's u16 multiplicity
+            const uint32_t c = SHORT ? half[km] : hist[km] & 0xffffu;
             out[s] = (km << 16) | c;
-            hist[km] = 0;
+            if (SHORT) half[km] = 0;
+            else hist[km] = 0;
             if (BITS && c) {
                 atomicOr(&bits[km >> 5], 1u << (km & 31));
                 my_sum += (int)c - 1;
@@ -321,21 +336,22 @@ __global__ void __launch_bounds__(256) k_kmers_hist(DevReads R) {
     }
 }
 
-template <int K>
+template <int K, bool SHORT>
 int kmers_hist_launch(const DevReads& R, cudaStream_t s) {
     constexpr int NB = 1 << (2 * K);
-    const int smem = NB * 4 + NB * 2;
+    const int threads = SHORT ? kShortThreads : 256;
+    const int smem = SHORT ? NB * 2 + kShortList * 2 : NB * 4 + NB * 2;
     if (smem > 0) {
-        cudaError_t e = cudaFuncSetAttribute(k_kmers_hist<K>,
+        cudaError_t e = cudaFuncSetAttribute(k_kmers_hist<K, SHORT>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return 1;
     }
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_kmers_hist<K>, 256, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_kmers_hist<K, SHORT>, threads, smem);
     if (per_sm < 1) per_sm = 1;
     int grid = num_sms() * per_sm;
     if (grid > R.n) grid = R.n > 0 ? R.n : 1;
-    k_kmers_hist<K><<<grid, 256, smem, s>>>(R);
+    k_kmers_hist<K, SHORT><<<grid, threads, smem, s>>>(R);
     return 0;
 }
 
@@ -627,10 +643,10 @@ int launch_kmers(const DevReads& R, int k, cudaStream_t s) {
     if (R.n <= 0) return 0;
     if (k >= kWideK && R.khash) k_khash_init<<<num_sms() * 4, 256, 0, s>>>(R);
     switch (k) {
-        case 4: return kmers_hist_launch<4>(R, s);
-        case 5: return kmers_hist_launch<5>(R, s);
-        case 6: return kmers_hist_launch<6>(R, s);
-        case 7: return kmers_hist_launch<7>(R, s);
+        case 4: return R.hbuckets ? kmers_hist_launch<4, true>(R, s) : kmers_hist_launch<4, false>(R, s);
+        case 5: return R.hbuckets ? kmers_hist_launch<5, true>(R, s) : kmers_hist_launch<5, false>(R, s);
+        case 6: return R.hbuckets ? kmers_hist_launch<6, true>(R, s) : kmers_hist_launch<6, false>(R, s);
+        case 7: return R.hbuckets ? kmers_hist_launch<7, true>(R, s) : kmers_hist_launch<7, false>(R, s);
         default:
             if (k < kWideK || k > 12 || !R.khash) return 2;
             k_kmers_hash<<<R.khash_ctas, 256, 0, s>>>(R, k);

@@ -35,7 +35,7 @@ def test_tentatives_per_pass(tmp_path, batch):
     _check(tmp_path, data, 0.90, word_index=3 if batch > 1 else 0, batch=batch)
 
 
-@pytest.mark.parametrize("t,w", [(0.90, 7), (0.92, 7), (0.95, 6), (0.97, 6)])
+@pytest.mark.parametrize("t,w", [(0.90, 7), (0.92, 7), (0.95, 6), (0.97, 6), (0.97, 5)])
 def test_thresholds_and_ragged_lengths(tmp_path, t, w):
     data = gsdr.synth_fasta(0, n_reads=1500, seed=72, n_seeds=900, len_lo=20, len_hi=160)
     _check(tmp_path, data, t, word_length=w)
