@@ -179,12 +179,12 @@ def filter_roofline(r, figures):
     kernel = {"table": "k_bfilter_tab (per-tentative k-mer tables in shared memory, "
                        "transposed, paired 16-bit min/add)",
               "index": "k_bindex + k_bfilter_idx (inverted k-mer index in shared memory)",
-              "bits": "k_bfilter_bits + k_bexact_t (two-level k-mer count bitmaps: AND + POPC "
-                      "per tentative, exact sums for the pairs the bound leaves open, grouped "
+              "bits": "k_bfilter_bits + k_bexact_t (k-mer count bitmaps, their products on the "
+                      "tensor cores, exact sums for the pairs the bound leaves open, grouped "
                       "by tentative)",
-              "masks": "k_bmask + k_bfilter_mask + k_bexact_t (per-k-mer rows of tentative "
-                       "bits in L2, bit-sliced counts per candidate, exact sums for the pairs "
-                       "the bound leaves open, grouped by tentative)"}[form]
+              "masks": "k_bfilter_hash + k_bexact_d (hashed k-mer counts, their products on the "
+                       "tensor cores, exact sums for the pairs the bound leaves open) or "
+                       "k_bmask + k_bfilter_mask + k_bexact_t (tentative masks)"}[form]
     ratio = figures.get("c%d.filter_%s.dram_over_input" % (r["config"], form))
     return {"bound": "hbm", "kernel": kernel,
             "achieved": achieved, "peak": r["peak"], "unit": "GB/s",
@@ -212,20 +212,20 @@ def measured_filter_bound(form, figures):
                     "c1.filter_table.bank_conflict_wavefront_share"),
                 "source": "profiles/k_bfilter_tab_c1_smem.md (200k-read workload)"}
     if form == "bits" and figures.get("c1.filter_bits.alu_pipe_pct") is not None:
-        return {"resource": "POPC (XU) and ALU pipes", "kernel": "k_bfilter_bits<6>",
-                "sm_throughput_pct": figures.get("c1.filter_bits.sm_throughput_pct"),
-                "xu_pipe_pct": figures.get("c1.filter_bits.xu_pipe_pct"),
+        return {"resource": "waits of the loading warps (L2, hand-overs)",
+                "kernel": "k_bfilter_bits<6>",
+                "tensor_pipe_pct": figures.get("c1.filter_bits.tensor_pipe_pct"),
                 "alu_pipe_pct": figures["c1.filter_bits.alu_pipe_pct"],
                 "ipc_of_4": figures.get("c1.filter_bits.ipc"),
                 "dram_pct_of_peak": figures.get("c1.filter_bits.dram_pct"),
-                "source": "profiles/k_bfilter_bits_c1.md (200k-read workload)"}
-    if form == "masks" and figures.get("c2.filter_masks.ipc") is not None:
-        return {"resource": "ALU pipe and L2 latency", "kernel": "k_bfilter_mask",
-                "ipc_of_4": figures["c2.filter_masks.ipc"],
-                "alu_pipe_pct": figures.get("c2.filter_masks.alu_pipe_pct"),
-                "l2_pct_of_peak": figures.get("c2.filter_masks.l2_pct"),
-                "dram_pct_of_peak": figures.get("c2.filter_masks.dram_pct"),
-                "source": "profiles/k_bfilter_mask_c2_300k.md (2M-read workload slice)"}
+                "source": "profiles/k_bfilter_bits_100k.md (100k reads of 150-5,000 bp)"}
+    if form == "masks" and figures.get("c2.filter_hash.tensor_pipe_pct") is not None:
+        return {"resource": "tensor pipe and the wait per stage", "kernel": "k_bfilter_hash",
+                "tensor_pipe_pct": figures["c2.filter_hash.tensor_pipe_pct"],
+                "alu_pipe_pct": figures.get("c2.filter_hash.alu_pipe_pct"),
+                "ipc_of_4": figures.get("c2.filter_hash.ipc"),
+                "dram_pct_of_peak": figures.get("c2.filter_hash.dram_pct"),
+                "source": "profiles/k_bfilter_hash_400k.md (400k reads of 150 bp)"}
     if form == "index" and figures.get("c2.filter_index.ipc") is not None:
         return {"resource": "instruction issue", "kernel": "k_bfilter_idx<7>",
                 "ipc_of_4": figures["c2.filter_index.ipc"],
@@ -240,10 +240,10 @@ def align_roofline(r, figures):
     ncu measured for its dominant kernel."""
     ms = r["align_ms"]
     done = r.get("cells_computed") or 0.0
-    return {"bound": "int_alu", "kernel": "k_align_single / k_align",
+    return {"bound": "int_alu", "kernel": "k_seg",
             "gcups": r["gcups"], "stage_ms": ms, "cells": r["stats"]["cells"],
             "gcups_note": "cells = full-DP q x T of every aligned pair (the reference's DP "
-                          "work); early exits, bands and the greedy bound skip most of them",
+                          "work); most are not stepped: rows no long enough path can be on",
             "cells_computed": done,
             "computed_over_full_dp": done / r["stats"]["cells"] if r["stats"]["cells"] else None,
             "computed_gcups": done / (ms * 1e-3) / 1e9 if ms > 0 else None,

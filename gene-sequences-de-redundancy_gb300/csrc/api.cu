@@ -583,7 +583,7 @@ int Job::loop_timed() {
             // per-step trace on stderr: the state after the step
             RoundState h;
             if (cudaMemcpy(&h, B_.st, sizeof(h), cudaMemcpyDeviceToHost) == cudaSuccess) {
-                // queues: systolic classes | lane-band classes | group-band classes
+                // queues: systolic classes | lane-band classes | segment classes, narrow, wide
                 std::string q;
                 for (int c = 0; c < kAlignClasses; c++)
                     q += (c == kSysClasses || c == kSysClasses + kBandClasses ? " | " : " ") +

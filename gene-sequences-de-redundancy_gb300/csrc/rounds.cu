@@ -29,7 +29,7 @@
 // R consecutive reference rounds produce.
 //   k_bselect     next R unclustered indices from a forward cursor
 //   k_bfilter_tab / k_bfilter_idx / k_bfilter_bits / k_bfilter_hash /
-//   k_bfilter_mask (+ k_bexact_t)
+//   k_bfilter_mask (+ k_bexact_t, k_bexact_d)
 //                 prefilter + word filter of (tentative group, candidate):
 //                 transposed per-tentative tables, an inverted k-mer index,
 //                 k-mer count bitmaps, hashed k-mer counts or per-k-mer
@@ -2540,7 +2540,7 @@ __global__ void __launch_bounds__(1024, 1) k_bfilter_idx(
 // of the stored ones is at least the smaller count, and where both are above
 // it is 144, so that
 //     S <= P + min(X_t, X_q),   X = sum over buckets of max(n - 144, 0).
-// A pair below its cutoff is rejected; the others go to k_bexact_t, which
+// A pair below its cutoff is rejected; the others go to k_bexact_d, which
 // forms S itself.  H is chosen per job (api.cu) so that unrelated reads rarely
 // reach the cutoff: P is about L^2 / H for reads of L k-mers.
 //
@@ -2552,12 +2552,12 @@ __global__ void __launch_bounds__(1024, 1) k_bfilter_idx(
 // with the rows' cutoffs while the next tile is summed in the other.
 //
 // 990k candidates x 1,024 tentatives, H = 1,536: 0.75 ms (1.35e12 pairs/s; the
-// masks 1.5 ms); 1M reads of 150 bp at t = 0.90 spend 127 ms in the filter stage
-// instead of 211.  An MMA (64 buckets) takes N / 2 cycles, and the MMAs alone
+// masks 1.5 ms); 1M reads of 100-150 bp at t = 0.90 spent 127 ms in the filter
+// stage instead of 211, and 108 since k_bexact_d and hash_even_r.  An MMA (64 buckets) takes N / 2 cycles, and the MMAs alone
 // would take 0.36 ms; the MMA thread's wait for a stage adds about 200 cycles
 // that nothing covers (issuing blocks while the tensor pipe is busy), so a stage
-// holds eight MMAs.  On the way there, average of the first 249 passes (now 0.39
-// ms): 16 KB stages with eight warps on each 0.43 ms; an arrival per copying
+// holds eight MMAs.  On the way there, average of the first 249 passes (0.39
+// ms as it is): 16 KB stages with eight warps on each 0.43 ms; an arrival per copying
 // thread 0.43; rows by TMA gathers of four 1.07 (67 cycles a gather); two warps
 // owning each 16 KB stage 0.41; the next stage's wait in the middle of the MMAs
 // 0.43; one team of four on the sums 0.43.

@@ -51,9 +51,11 @@ typedef struct {
     int32_t verbose;      /* 1: print the reference's progress lines to stdout */
     int32_t word_filter;  /* batched word filter form: 0 automatic, 1 per-tentative k-mer
                              tables, 2 inverted k-mer index, 3 two-level k-mer count
-                             bitmaps (k <= 7), 4 per-k-mer tentative masks (k <= 7,
-                             reads of at most 1,023 k-mers; otherwise the automatic
-                             form); the result is the same in every form */
+                             bitmaps (k <= 7), 4 the short reads' form (k <= 7, at most
+                             1,023 k-mers a read, otherwise the automatic form): hashed
+                             k-mer counts where 2,048 buckets or fewer tell unrelated
+                             reads apart, else per-k-mer tentative masks; the result is
+                             the same in every form */
     int32_t variant;      /* semantics: 0 = cuda-version (func.cu, the default);
                              1 = the top-level SYCL program (func.cpp): k from t by
                              func.cpp:36-45, w 4..8, no drop mode and no pigeon filter,
@@ -101,7 +103,8 @@ typedef struct {
     double cells;             /* sum over aligned pairs of gap-free q x T (full-DP cells) */
     double filter_bytes;      /* input bytes of the filter stage: per launch, each remaining
                                  candidate's 28 bytes of composition, cutoffs and index and
-                                 its (k-mer, count) list (word_index = 2: its k-mer bitmap);
+                                 its (k-mer, count) list (word_index = 2: the k-mer bitmaps
+                                 that the launch reads; hashed counts: its row of them);
                                  the plain form counts the list only where the filter
                                  reads it (composition bound passed), the batched forms
                                  once per launch (re-reads by other tentatives not counted) */
@@ -113,7 +116,8 @@ typedef struct {
                                  tables, 1 per-pass inverted k-mer index (reads holding
                                  few of the 4^k k-mers), 2 k-mer count bitmaps with an
                                  exact sum for the pairs their bound leaves open, 3
-                                 per-k-mer tentative masks (short reads in a sparse
+                                 hashed k-mer counts or per-k-mer tentative masks, with
+                                 exact sums too (short reads in a sparse
                                  k-mer space) with the same exact sum */
     double filter_max_bytes;  /* with stage_timing only: input bytes of the filter launch
                                  that read the most, and its time (filter_max_ms) */
