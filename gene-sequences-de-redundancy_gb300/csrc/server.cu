@@ -14,7 +14,8 @@
 //   1. the scheduler thread gives a job a free slot (max_inflight); its worker
 //      counts the file's records and newlines and starts when an upper bound
 //      of the parse buffers (from those counts) fits the remaining budget, or
-//      no other job holds any of it;
+//      no other job holds any of it; a job that waits here is not passed by
+//      one that got its slot later (admission.h);
 //   2. once the worker knows the reads, the job's exact clustering footprint
 //      must fit too; the worker waits for it while the job's parse buffers
 //      are held.
@@ -48,6 +49,7 @@
 #include <thread>
 #include <vector>
 
+#include "admission.h"
 #include "gsdr.h"
 #include "gsdr_host.h"
 #include "job.h"
@@ -63,11 +65,12 @@ struct ServerJob {
     std::string error;
     std::vector<int32_t> cluster;
     std::vector<char> out;
-    int64_t parse_bytes = 0;  // step-1 reservation (held: in mem_used)
+    int64_t parse_bytes = 0;  // step-1 reservation (held: reserved)
     int64_t job_bytes = 0;    // step-2 reservation
     bool held = false;
     bool clustering = false;
     bool express = false;     // runs in the express slot
+    int64_t ticket = 0;       // order of the slots
 };
 
 }  // namespace gsdr
@@ -89,11 +92,8 @@ struct gsdr_server {
     bool workers_stop = false;
     int inflight = 0;
     int express = 0;                   // jobs in the express slot (0 or 1)
-    int holding = 0;                   // jobs past step 1
-    int clustering = 0;                // jobs past step 2
-    int64_t mem_used = 0;
-    int64_t next_id = 1;
-    bool stopping = false;
+    Admission adm;
+    int64_t next_id = 1, next_ticket = 1;
 };
 
 namespace {
@@ -118,13 +118,8 @@ int admit_parse(gsdr_server* s, ServerJob* j) {
     const int64_t newlines = (int64_t)std::count(b, b + n, '\n');
     j->parse_bytes = cluster_fasta_parse_bytes(n, records, newlines);
     std::unique_lock<std::mutex> lock(s->mu);
-    s->cv_sched.wait(lock, [&] {
-        return s->stopping || s->mem_used + j->parse_bytes <= s->so.mem_budget ||
-               s->holding == 0;
-    });
-    if (s->stopping) return fail(GSDR_EBUSY, "server stopped");
-    s->mem_used += j->parse_bytes;
-    s->holding++;
+    if (!s->adm.parse(lock, s->cv_sched, j->ticket, j->parse_bytes))
+        return fail(GSDR_EBUSY, "server stopped");
     j->held = true;
     return GSDR_OK;
 }
@@ -139,14 +134,9 @@ void run_job(gsdr_server* s, std::shared_ptr<ServerJob> j) {
     // step 2 of the admission: the job's own footprint, once its reads are known
     const std::function<int(int64_t)> admit = [s, j](int64_t need) -> int {
         std::unique_lock<std::mutex> lock(s->mu);
-        s->cv_sched.wait(lock, [&] {
-            return s->stopping || s->mem_used + need <= s->so.mem_budget || s->clustering == 0;
-        });
-        if (s->stopping) return fail(GSDR_EBUSY, "server stopped");
-        s->mem_used += need;
+        if (!s->adm.cluster(lock, s->cv_sched, need)) return fail(GSDR_EBUSY, "server stopped");
         j->job_bytes = need;
         j->clustering = true;
-        s->clustering++;
         return GSDR_OK;
     };
     int rc = admit_parse(s, j.get());
@@ -171,11 +161,7 @@ void run_job(gsdr_server* s, std::shared_ptr<ServerJob> j) {
     std::lock_guard<std::mutex> lock(s->mu);
     s->inflight--;
     if (j->express) s->express = 0;
-    if (j->held) {
-        s->mem_used -= j->parse_bytes + j->job_bytes;
-        s->holding--;
-    }
-    if (j->clustering) s->clustering--;
+    if (j->held) s->adm.release(j->parse_bytes + j->job_bytes, j->clustering);
     finish(s, j, rc);
     s->cv_sched.notify_all();
 }
@@ -219,10 +205,10 @@ void scheduler_loop(gsdr_server* s) {
     while (true) {
         std::unique_lock<std::mutex> lock(s->mu);
         // the choice is made when a slot is free, among the jobs queued then
-        s->cv_sched.wait(lock, [&] { return s->stopping || next_job(s) != s->queue.end(); });
-        if (s->stopping && s->queue.empty()) return;
+        s->cv_sched.wait(lock, [&] { return s->adm.stopping || next_job(s) != s->queue.end(); });
+        if (s->adm.stopping && s->queue.empty()) return;
         std::shared_ptr<ServerJob> j;
-        if (s->stopping) {
+        if (s->adm.stopping) {
             j = s->queue.front();
             s->queue.pop_front();
         } else {
@@ -231,12 +217,13 @@ void scheduler_loop(gsdr_server* s) {
             s->queue.erase(it);
             j->express = s->inflight - s->express >= s->so.max_inflight;
         }
-        if (s->stopping) {
+        if (s->adm.stopping) {
             j->error = "server stopped";
             finish(s, j, GSDR_EBUSY);
             continue;
         }
         s->inflight++;
+        j->ticket = s->next_ticket++;
         if (j->express) s->express = 1;
         s->ready.push_back(j);
         s->cv_work.notify_one();
@@ -283,6 +270,7 @@ int gsdr_server_create(const gsdr_server_opts* so, gsdr_server** out) {
         }
         s->so.mem_budget = (int64_t)(free_b / 10 * 8);
     }
+    s->adm.budget = s->so.mem_budget;
     // a worker per slot, the express slot included
     for (int w = 0; w <= s->so.max_inflight; w++) s->workers.emplace_back(worker_loop, s);
     s->scheduler = std::thread(scheduler_loop, s);
@@ -313,7 +301,7 @@ int gsdr_server_submit(gsdr_server* s, const char* fasta, int64_t n, float thres
         j->fasta.shrink_to_fit();
     }
     std::lock_guard<std::mutex> lock(s->mu);
-    if (s->stopping) return fail(GSDR_EBUSY, "server: stopping");
+    if (s->adm.stopping) return fail(GSDR_EBUSY, "server: stopping");
     j->id = s->next_id++;
     s->jobs[j->id] = j;
     *job = j->id;
@@ -395,7 +383,7 @@ void gsdr_server_destroy(gsdr_server* s) {
     if (!s) return;
     {
         std::lock_guard<std::mutex> lock(s->mu);
-        s->stopping = true;
+        s->adm.stopping = true;
         s->cv_sched.notify_all();
     }
     if (s->scheduler.joinable()) s->scheduler.join();
