@@ -125,7 +125,6 @@ int admit_parse(gsdr_server* s, ServerJob* j) {
 }
 
 void run_job(gsdr_server* s, std::shared_ptr<ServerJob> j) {
-    j->t_start = now_ms();
     gsdr_opts o;
     gsdr_default_opts(&o);
     o.threshold = j->threshold;
@@ -140,6 +139,7 @@ void run_job(gsdr_server* s, std::shared_ptr<ServerJob> j) {
         return GSDR_OK;
     };
     int rc = admit_parse(s, j.get());
+    if (!rc) j->t_start = now_ms();  // the wait for room is queueing
     std::unique_ptr<gsdr_result, void (*)(gsdr_result*)> r(new_result(), gsdr_result_free);
     if (!rc && !r) rc = fail(GSDR_ENOMEM, "server: out of host memory");
     if (!rc)

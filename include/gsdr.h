@@ -331,9 +331,9 @@ int gsdr_server_wait(gsdr_server* s, int64_t timeout_ms, int64_t* job, int32_t* 
  * receives the size) and the cluster array in sorted order (may be NULL). */
 int gsdr_server_result(gsdr_server* s, int64_t job, char* buf, int64_t cap, int64_t* need,
                        int32_t* cluster, int32_t* n_reads);
-/* Timing of a finished job: submission to the start of its run on a worker
- * (parse, sort, admission wait) and the run itself (device work and output
- * formatting), host wall clock.  The sum of run_ms over jobs divided by the
+/* Timing of a finished job: submission to the start of its run (the waits for a
+ * slot and for room on the device) and the run itself (parse, sort, device work
+ * and output formatting), host wall clock.  The sum of run_ms over jobs divided by the
  * stream's wall time is the number of jobs running at once on average. */
 int gsdr_server_times(gsdr_server* s, int64_t job, double* queued_ms, double* run_ms);
 int gsdr_server_release(gsdr_server* s, int64_t job);
