@@ -73,6 +73,7 @@ struct Plan {
     int64_t idx_cap = 0;    // > 0: batched word filter by inverted index, postings capacity
     bool idx_smem = false;  // that index fits the filter's shared memory (16-bit copy)
     bool bits = false;      // batched word filter by k-mer presence bitmaps
+    bool folds = true;      // ... with folded copies where the word length has them
     bool masks = false;     // batched word filter by tentative masks
     int hbuckets = 0;       // that form by hashed k-mer counts, their buckets
     int ents_max = 0;       // its longest k-mer list
@@ -251,7 +252,7 @@ size_t carve_all(char* base, int n, int64_t n_bytes, const Plan& P, bool drop, i
     R.kextra = bits ? c.take<int32_t>(n) : nullptr;
     R.kbits2 = P.bits ? c.take<uint32_t>((size_t)n * nbw) : nullptr;
     R.kextra3 = P.bits ? c.take<int32_t>(n) : nullptr;
-    const bool folds = P.bits && k >= kMinFoldK;
+    const bool folds = P.bits && P.folds && k >= kMinFoldK;
     R.kfold = folds ? c.take<uint32_t>((size_t)n * (nbw / 2 + nbw / 4)) : nullptr;
     R.kfextra = folds ? c.take<int32_t>(2 * (size_t)n) : nullptr;
     B.st = reinterpret_cast<RoundState*>(c.take<char>(sizeof(RoundState) + 4 * 64));
@@ -319,6 +320,22 @@ size_t carve_all(char* base, int n, int64_t n_bytes, const Plan& P, bool drop, i
     R.pig_cap = pig ? 4 * B.seg_cap : 0;
     R.pig_q = pig ? c.take<Pair>((size_t)R.pig_cap) : nullptr;
     return c.used + 256;
+}
+
+// The forms that take most memory per read, given up one after another when the
+// device has no room for them: the rows of hashed counts for the tentative
+// masks (150 bp: 768 bytes a read for 32), the folded bitmaps for the full ones
+// (3/4 of a bitmap).  The results are the same; false: nothing left to give up.
+bool shrink_plan(Plan& P, int k) {
+    if (P.hbuckets) {
+        P.hbuckets = 0;
+        return true;
+    }
+    if (P.bits && P.folds && k >= kMinFoldK) {
+        P.folds = false;
+        return true;
+    }
+    return false;
 }
 
 int validate(const gsdr_reads* reads, const gsdr_opts* opts_in, gsdr_opts& o) {
@@ -424,8 +441,19 @@ int Job::init(const gsdr_reads* reads, const gsdr_opts* opts_in, cudaStream_t s,
     if (!h_done_ || !h_state_) return fail(GSDR_ENOMEM, "pinned host memory");
     if (n == 0) return GSDR_OK;
     const double t_device = now_ms();
-    dbytes_ = carve_all(nullptr, n, n_bytes_, P, opts.drop == 1, opts.word_length, R_, B_);
-    JCUDA(dev_alloc(&dmem_, dbytes_, stream));
+    // (beside the job, gsdr_cluster_fasta still needs room for its output)
+    const size_t later = (size_t)n_bytes_ + 64 * (size_t)n;
+    while (true) {
+        dbytes_ = carve_all(nullptr, n, n_bytes_, P, opts.drop == 1, opts.word_length, R_, B_);
+        if (!dev_room(dbytes_ + later) && shrink_plan(P, opts.word_length)) continue;
+        const cudaError_t e = dev_alloc(&dmem_, dbytes_, stream);
+        if (e == cudaErrorMemoryAllocation && shrink_plan(P, opts.word_length)) {
+            cudaGetLastError();
+            continue;
+        }
+        JCUDA(e);
+        break;
+    }
     carve_all(reinterpret_cast<char*>(dmem_), n, n_bytes_, P, opts.drop == 1, opts.word_length,
               R_, B_);
     if (trace_)
@@ -992,6 +1020,19 @@ int Job::lcs_pairs(const int32_t* pat, const int32_t* txt, int n_pairs, int mapp
 }
 
 }  // namespace gsdr
+
+extern "C" int gsdr_set_alloc_limit(int64_t bytes) {
+    set_alloc_limit(bytes);
+    return GSDR_OK;
+}
+
+extern "C" int gsdr_job_filter_form(gsdr_job* j, int32_t* hash_buckets, int32_t* folded) {
+    if (!j || !hash_buckets || !folded)
+        return fail(GSDR_EINVAL, "gsdr_job_filter_form: null argument");
+    *hash_buckets = j->job.device_reads().hbuckets;
+    *folded = j->job.device_reads().kfold != nullptr;
+    return GSDR_OK;
+}
 
 extern "C" int gsdr_set_spin_limit(int32_t device, int32_t polls) {
     if (cudaSetDevice(device) != cudaSuccess) return fail(GSDR_EDEVICE, "no such CUDA device");

@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <vector>
@@ -19,6 +20,11 @@ constexpr size_t kPinnedArenaSlots = 64;
 std::mutex g_pool_mu;
 cudaMemPool_t g_pool[kMaxDevices] = {};
 bool g_pool_failed[kMaxDevices] = {};
+std::atomic<int64_t> g_alloc_limit{-1};
+
+// Requests below this size are not checked against the free memory (the query
+// takes longer than a small job's whole allocation).
+constexpr size_t kAskFrom = (size_t)16 << 30;
 
 // The pool of the current device, created on first use: memory freed into it
 // is kept for later jobs up to the retained size, and an allocation never
@@ -57,11 +63,30 @@ std::vector<void*> g_pin_free;
 cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t s) {
     *p = nullptr;
     if (bytes == 0) bytes = 256;
+    const int64_t limit = g_alloc_limit.load(std::memory_order_relaxed);
+    if (limit >= 0 && bytes > (size_t)limit) return cudaErrorMemoryAllocation;
     cudaMemPool_t pool = current_pool();
     // without a pool of its own (creation refused) the device's default pool
     // still keeps the allocation stream-ordered
     return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
 }
+
+bool dev_room(size_t bytes) {
+    const int64_t limit = g_alloc_limit.load(std::memory_order_relaxed);
+    if (limit >= 0) return bytes <= (size_t)limit;
+    if (bytes < kAskFrom) return true;
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return true;
+    // and what the pool keeps for later jobs
+    uint64_t reserved = 0, used = 0;
+    if (cudaMemPool_t pool = current_pool()) {
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved);
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used);
+    }
+    return bytes <= free_b + (size_t)(reserved > used ? reserved - used : 0);
+}
+
+void set_alloc_limit(int64_t bytes) { g_alloc_limit.store(bytes < 0 ? -1 : bytes); }
 
 void dev_free(void* p, cudaStream_t s) {
     if (p) cudaFreeAsync(p, s);

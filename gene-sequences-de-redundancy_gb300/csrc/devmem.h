@@ -20,6 +20,11 @@ namespace gsdr {
 
 // Device memory on the current device, ordered on stream s.
 cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t s);
+// Whether the current device seems to have room for `bytes`, the pool's kept
+// memory included.  Small requests are taken to fit.
+bool dev_room(size_t bytes);
+// Testing: requests above `bytes` fail as on a full device (< 0: no limit).
+void set_alloc_limit(int64_t bytes);
 // Returns p (from dev_alloc on the same device) to the pool after the work
 // queued on s so far; p == nullptr is a no-op.
 void dev_free(void* p, cudaStream_t s);

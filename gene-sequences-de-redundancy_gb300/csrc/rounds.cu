@@ -1606,6 +1606,8 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
     constexpr int NQ = (1 << (2 * K)) / 128;        // 16-byte words of one bitmap
     constexpr int GL = NQ >= 8 ? NQ / 8 : 1;        // groups of four stages per level
     constexpr int DEPTHS = K >= kMinFoldK ? kMaxDepth : K == 5 ? 1 : 0;
+    // (a job without room for the folded bitmaps takes none of them)
+    const int depths = R.kfold ? DEPTHS : min(DEPTHS, 1);
     extern __shared__ __align__(1024) uint8_t bsm_raw[];
     __shared__ uint64_t full[kBitsStages], empty[kBitsStages], tfull[2], tempty[2], drain;
     __shared__ uint32_t s_tmem;
@@ -1668,6 +1670,7 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
         const int kq = R.n_kmer[q] + xq, kr = R.n_kmer[rep] + xr;
 #pragma unroll
         for (int d = 1; d <= DEPTHS; d++) {
+            if (d > depths) break;
             const int eq = d == 1 ? xq : R.kfextra[(size_t)(d - 2) * R.n + q];
             const int er = d == 1 ? xr : R.kfextra[(size_t)(d - 2) * R.n + rep];
             const float w = 1.0f / (float)((1 << (2 * K)) >> (d - 1));
@@ -1690,7 +1693,8 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
     for (int d = 1; d <= DEPTHS; d++) {
         const float c = (float)(GL >> (d - 1)) +
                         kOpenCost * (float)s_open[d] * (1.0f / (65536.0f * kBitsThreads));
-        if ((st->bits_hold == 0 || d <= st->bits_cap) && c < cost) depth = d, cost = c;
+        if (d <= depths && (st->bits_hold == 0 || d <= st->bits_cap) && c < cost)
+            depth = d, cost = c;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) st->bits_depth = depth;
     // groups of two stages (1,024 bits) per tile (k = 4: half of them zeros)

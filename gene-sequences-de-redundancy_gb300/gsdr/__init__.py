@@ -181,6 +181,8 @@ def lib():
                                               C.c_int32, C.c_void_p, C.c_void_p, C.c_int32,
                                               C.c_float, C.c_void_p, C.c_void_p]
         L.gsdr_set_spin_limit.argtypes = [C.c_int32, C.c_int32]
+        L.gsdr_set_alloc_limit.argtypes = [C.c_int64]
+        L.gsdr_job_filter_form.argtypes = [C.c_void_p, P(C.c_int32), P(C.c_int32)]
         L.gsdr_job_resume.argtypes = [C.c_void_p, C.c_void_p, C.c_int32, P(Stats)]
         L.gsdr_autotune.argtypes = [P(Reads), P(Opts), C.c_int32, C.c_int32, C.c_char_p,
                                     P(Opts), C.c_char_p, C.c_int64, P(C.c_int64)]
@@ -424,6 +426,13 @@ class Job:
         _check(lib().gsdr_job_resume(self._h, cp.ctypes.data, max_passes, C.byref(st)))
         return st
 
+    def filter_form(self):
+        """(hash buckets, folded bitmaps) of the job's batched word filter
+        (gsdr_job_filter_form)."""
+        h, f = C.c_int32(), C.c_int32()
+        _check(lib().gsdr_job_filter_form(self._h, C.byref(h), C.byref(f)))
+        return h.value, bool(f.value)
+
     def cluster(self) -> np.ndarray:
         cl = np.empty(max(self.n, 1), dtype=np.int32)
         _check(lib().gsdr_job_cluster(self._h, cl.ctypes.data))
@@ -550,6 +559,11 @@ def lcs_decide_noalloc(d_packed, d_pack_off, d_len_raw, d_len_gf, n_seq, d_pat, 
     """gsdr_lcs_decide_noalloc on device pointers (integers); raises on error."""
     _check(lib().gsdr_lcs_decide_noalloc(d_packed, d_pack_off, d_len_raw, d_len_gf, n_seq,
                                          d_pat, d_txt, n_pairs, C.c_float(t), d_accept, stream))
+
+
+def set_alloc_limit(n_bytes):
+    """gsdr_set_alloc_limit: larger device allocations fail (None: no limit)."""
+    _check(lib().gsdr_set_alloc_limit(-1 if n_bytes is None else int(n_bytes)))
 
 
 def set_spin_limit(polls, device=0):

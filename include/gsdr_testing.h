@@ -34,6 +34,15 @@ int gsdr_lcs_decide(const char* bytes, int64_t n_bytes, const int64_t* off, cons
  * the early, full-size passes of a job (gsdr/autotune.py). */
 int gsdr_job_run_limited(gsdr_job* job, int32_t max_passes, gsdr_stats* stats);
 
+/* Device allocations of more than `bytes` fail as on a full device from now on
+ * (bytes < 0: no limit), so that a job's smaller forms can be tested. */
+int gsdr_set_alloc_limit(int64_t bytes);
+
+/* The form of a job's batched word filter beyond gsdr_stats.word_index:
+ * *hash_buckets the buckets of the hashed k-mer counts (0: tentative masks, or
+ * another form), *folded 1 where the bitmaps have folded copies. */
+int gsdr_job_filter_form(gsdr_job* job, int32_t* hash_buckets, int32_t* folded);
+
 /* Polls each bounded wait of the alignment kernels (a warp of a multi-warp
  * group waiting for its neighbour's carry words) makes on `device` before it
  * gives up, sets the error flag and returns; polls < 0 restores the default
