@@ -478,7 +478,9 @@ int Job::init(const gsdr_reads* reads, const gsdr_opts* opts_in, cudaStream_t s,
     if (opts.group_words == 0)
         if (const char* gw = std::getenv("GSDR_GROUP_MAXW"))
             R_.group_max_w = std::min(std::max(std::atoi(gw), 0), kSegMaxWords);
-    R_.band_few = R_.group_max_w > 0 ? kBandFew : 0;
+    // (a lane-banded pair's window, of rows T - c + q - c <= 32 x 8 - 63, in that kernel)
+    constexpr int kBandSegWords = (32 * kBandMaxWords - 62 + kSegSteps32) / 32 + 3;
+    R_.band_few = R_.group_max_w >= kBandSegWords ? kBandFew : 0;
     // a window holds at most the longest read's rows
     const int64_t widest = (P.max_len + 31) / 32;
     R_.wide = widest <= R_.group_max_w                                        ? 0
@@ -973,7 +975,7 @@ int Job::lcs_pairs(const int32_t* pat, const int32_t* txt, int n_pairs, int mapp
             // a narrow run first where the passes would take one
             const int T = gf[txt[k]], q = gf[pat[k]], cb = cut[pat[k]];
             if (T > 0 && cb > 0 && q >= cb && T >= cb &&
-                seg_narrow(T, q, cb, seg_words(T, q, cb, kSegSteps32)))
+                seg_narrow(T, q, cb, seg_words(T, q, cb, kSegSteps32), R_.group_max_w))
                 c = kNarrowClass;
         }
         cls[c].push_back(Pair{txt[k], pat[k]});

@@ -87,14 +87,17 @@ __host__ __device__ __forceinline__ float seg_accept_ratio(int q, int c) {
 __host__ __device__ __forceinline__ float seg_narrow_slope(int T, int q, int c) {
     return fminf((float)T / (float)q, seg_accept_ratio(q, c) + kSegSlopeMore);
 }
-// Whether a narrow run comes first (`words`: the full window): from that ratio
-// on, and where the strip is at most half the full window's words.  A wrong
-// guess costs the strip's run and changes no decision.
-__host__ __device__ __forceinline__ bool seg_narrow(int T, int q, int c, int words) {
+// Whether a narrow run comes first (`words`: the full window, max_words: the
+// widest window the kernel may take): from that ratio on, and where the strip's
+// widest window is at most half the full one's words.  A wrong guess costs the
+// strip's run and changes no decision.
+__host__ __device__ __forceinline__ bool seg_narrow(int T, int q, int c, int words,
+                                                    int max_words) {
     if (c >= q || T <= q) return false;
     const float s = seg_narrow_slope(T, q, c);
     if ((float)T < seg_accept_ratio(q, c) * (float)q) return false;
-    return words >= 2 * ((int)(kSegSteps8 * s + 2 * kSegStrip) / 32 + 2);
+    const int strip = (int)(kSegSteps8 * s + 2 * kSegStrip) / 32 + 2;
+    return words >= 2 * strip && strip <= max_words;
 }
 
 __device__ __forceinline__ int seg_vidx(int k) { return k + (k >> 4); }

@@ -136,7 +136,7 @@ __device__ __forceinline__ int pair_class(int T, int q, int c, int band_max_w,
             if ((long long)T * w <= band_serial) return kSysClasses + (w == 4 ? 0 : 1);
         }
         const int sw = seg_words(T, q, c, kSegSteps32);
-        if (seg_max_w > 0 && seg_narrow(T, q, c, sw)) return kNarrowClass;
+        if (seg_max_w > 0 && seg_narrow(T, q, c, sw, seg_max_w)) return kNarrowClass;
         return full_class(sw, q, seg_max_w);
     } else if (seg_max_w > 0) {
         return seg_class(1);
@@ -884,7 +884,7 @@ __global__ void __launch_bounds__(kAlignThreads, MODE == kSegWide ? 1 : 2) k_seg
             if (leader) done += (unsigned long long)steps * (32 * G * seg_tile(wl));
             if (d < 0) continue;
             if (BOTH && d == 0 && P.narrow &&
-                seg_words(P.T, P.q, P.c, kSegSteps32) <= kSegMaxWords) {
+                seg_words(P.T, P.q, P.c, kSegSteps32) <= R.group_max_w) {
                 seg_start(P, S, false);
                 continue;
             }
