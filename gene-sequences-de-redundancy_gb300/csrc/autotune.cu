@@ -13,8 +13,8 @@
 // descent in four stages (R_max x form, band tiles, block shape, staging
 // depth), each stage starting from the best setting so far.
 //
-// The result is kept in a text cache, one line per (GPU model, SM count,
-// workload bucket): a later job with batch = 0 whose bucket is in the cache
+// The result is kept in a text cache, one line per (GPU model, SM count, kernel
+// generation, workload bucket): a later job with batch = 0 whose bucket is in the cache
 // takes the tuned values for every knob it leaves automatic.  The bucket is
 // word length, drop mode, variant, pigeon filter, threshold (percent), and
 // log2 of the read count and of the mean read length, rounded.
@@ -65,6 +65,18 @@ std::string gpu_key(int device) {
     return known[device];
 }
 
+// The kernels that the knobs steer.  Raised when they change so much that a
+// setting measured on the old ones says nothing about the new: lines of another
+// generation are left alone and not applied.  (1, unmarked: the group-banded
+// alignment kernel and the word filters without tensor cores, where a window
+// of 64 words or R_max 256 could be the best; on the kernels after them the
+// same values send the wider windows to the systolic kernels and cap the
+// filters' products.)
+constexpr const char* kKernelGeneration = "g2";
+
+// First field of a cache line.
+std::string cache_key(int device) { return gpu_key(device) + "/" + kKernelGeneration; }
+
 int log2_round(double x) { return x > 1 ? (int)std::lround(std::log2(x)) : 0; }
 
 // The knobs a cache line sets, in file order.
@@ -114,7 +126,7 @@ bool apply_tuned(const gsdr_reads* reads, gsdr_opts& o) {
     if (o.batch != 0) return false;
     const std::string path = default_cache_path();
     if (path.empty()) return false;
-    const std::string gpu = gpu_key(o.device), bucket = tune_bucket(reads, o);
+    const std::string gpu = cache_key(o.device), bucket = tune_bucket(reads, o);
     std::lock_guard<std::mutex> lock(g_cache_mu);
     std::ifstream in(path);
     if (!in) return false;
@@ -155,7 +167,7 @@ int store_tuned(const std::string& path, const std::string& gpu, const std::stri
         }
     }
     if (keep.empty())
-        keep.push_back("# gsdr tuning cache: gpu, bucket, batch, word_filter, group_words, "
+        keep.push_back("# gsdr tuning cache: gpu and kernel generation, bucket, batch, word_filter, group_words, "
                        "band_serial, align_blocks, filter_blocks, graph_steps, us per "
                        "representative");
     char row[512];
@@ -345,7 +357,7 @@ int autotune(const gsdr_reads* reads, const gsdr_opts* base_in, int reps, int ru
     }
     const std::string path = cache_path ? std::string(cache_path) : default_cache_path();
     if (!path.empty()) {
-        rc = store_tuned(path, gpu_key(base.device), tune_bucket(reads, base), best,
+        rc = store_tuned(path, cache_key(base.device), tune_bucket(reads, base), best,
                          b->us_per_rep);
         if (rc) return rc;
     }
