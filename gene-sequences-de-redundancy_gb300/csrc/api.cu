@@ -96,7 +96,7 @@ int job_r_max(const gsdr_opts& o) {
 // kIndexDensity), where almost every table lookup of the table form would
 // read a zero, take the tentative masks when every read has at most
 // kMaskMaxEntries k-mer entries, else the inverted index of the tentatives'
-// k-mers.  GSDR_BFILTER=table|index|bits|masks forces a form.
+// k-mers.  GSDR_BFILTER=table|index|bits|masks|tmasks forces a form.
 constexpr int64_t kIndexDensity = 8;
 
 // Buckets of the hashed k-mer counts for reads of up to max_len bases, or 0:
@@ -177,13 +177,16 @@ int make_plan(const gsdr_reads* reads, const gsdr_opts& o, Plan& P, PlanPreset* 
         P.mask_planes = ents_max <= kMaskEntries8 ? 8 : 10;
         bool masks = index && masks_ok;
         // the caller's choice (word_filter), else GSDR_BFILTER=table|index|bits|masks
+        // (tmasks: the masks also where the hashed counts would be taken)
         int form = o.word_filter;
+        bool hashed = true;
         if (form == 0) {
             const char* f = std::getenv("GSDR_BFILTER");
             if (f && std::strcmp(f, "table") == 0) form = 1;
             if (f && std::strcmp(f, "index") == 0) form = 2;
             if (f && std::strcmp(f, "bits") == 0) form = 3;
             if (f && std::strcmp(f, "masks") == 0) form = 4;
+            if (f && std::strcmp(f, "tmasks") == 0) form = 4, hashed = false;
         }
         if (form == 1) index = false, bits = false, masks = false;
         if (form == 2) index = true, bits = false, masks = false;
@@ -193,7 +196,7 @@ int make_plan(const gsdr_reads* reads, const gsdr_opts& o, Plan& P, PlanPreset* 
         P.bits = bits;
         P.masks = masks;
         P.ents_max = (int)ents_max;
-        if (masks) P.hbuckets = hash_buckets(P.max_len, k, o.threshold);
+        if (masks && hashed) P.hbuckets = hash_buckets(P.max_len, k, o.threshold);
         // automatic R: the largest, except for the table form at k = 7, whose
         // tables hold only 4 tentatives per CTA (200k reads of 150-5,000 bp at
         // t = 0.90: 3.7 s at 256 against 4.4 s at 1024; the bitmap form, on
