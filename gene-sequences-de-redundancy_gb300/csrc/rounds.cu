@@ -1708,8 +1708,9 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const int limit = max(c_spin_limit, 1);
-    bool ok = true;  // this warp's waits all ended
+    const int limit = c_spin_limit;
+    bool ok = true;       // this warp's waits all ended
+    bool issued = false;  // this thread has MMAs in flight, or had
     if (warp == 0) {
         if (lane == 0) {
             const uint32_t idesc = tc_idesc_fp4(N);
@@ -1723,6 +1724,7 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
                     ok = mbar_wait(&full[s], ph, limit, &s_quit);
                     if (!ok) break;
                     tc_fence_after();
+                    issued = true;
                     const uint32_t a = tc_desc_lo(smem_u32(stage0 + s * kBitsStageBytes));
 #pragma unroll
                     for (int u = 0; u < 2; u++)
@@ -1943,7 +1945,7 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
-        if (s_quit && lane == 0) {
+        if (s_quit && issued) {
             // the MMAs in flight, before the accumulators are given back
             const int none = 0;
             tc_commit(&drain);
@@ -2675,8 +2677,9 @@ __global__ void __launch_bounds__(kHashThreads, 1) k_bfilter_hash(
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const int limit = max(c_spin_limit, 1);
-    bool ok = true;  // this warp's waits all ended
+    const int limit = c_spin_limit;
+    bool ok = true;       // this warp's waits all ended
+    bool issued = false;  // this thread has MMAs in flight, or had
     if (warp == 0) {
         if (lane == 0) {
             const uint32_t idesc = tc_idesc_fp4(N);
@@ -2691,6 +2694,7 @@ __global__ void __launch_bounds__(kHashThreads, 1) k_bfilter_hash(
                     ok = mbar_wait(&full[s], ph, limit, &s_quit);
                     if (!ok) break;
                     tc_fence_after();
+                    issued = true;
                     const uint32_t a = a0 + s * (kHashStageBytes / 16);
                     const uint32_t b = b0 + 2 * c * N * (kTcRowBytes / 16);
                     tc_mma_stage(tmem + buf * kTcMaxN, tmem, a, b, idesc, c == 0);
@@ -2848,7 +2852,7 @@ __global__ void __launch_bounds__(kHashThreads, 1) k_bfilter_hash(
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
-        if (s_quit && lane == 0) {
+        if (s_quit && issued) {
             // the MMAs in flight, before the accumulators are given back
             const int none = 0;
             tc_commit(&drain);

@@ -567,8 +567,8 @@ def set_alloc_limit(n_bytes):
 
 
 def set_spin_limit(polls, device=0):
-    """gsdr_set_spin_limit: polls each bounded device-side wait of the
-    alignment kernels makes before giving up (None or < 0: the default)."""
+    """gsdr_set_spin_limit: polls each bounded device-side wait of the alignment
+    and filter kernels makes before giving up (None or < 0: the default)."""
     _check(lib().gsdr_set_spin_limit(device, -1 if polls is None else int(polls)))
 
 

@@ -43,11 +43,13 @@ int gsdr_set_alloc_limit(int64_t bytes);
  * another form), *folded 1 where the bitmaps have folded copies. */
 int gsdr_job_filter_form(gsdr_job* job, int32_t* hash_buckets, int32_t* folded);
 
-/* Polls each bounded wait of the alignment kernels (a warp of a multi-warp
- * group waiting for its neighbour's carry words) makes on `device` before it
- * gives up, sets the error flag and returns; polls < 0 restores the default
- * (4,194,304).  With 0 every such wait gives up at once, so a call whose pairs
- * need a multi-warp group returns GSDR_ETIMEOUT: the way tests check that a
+/* Polls each bounded wait makes on `device` before it gives up, sets the error
+ * flag and returns: in the alignment kernels a warp of a multi-warp group
+ * waiting for its neighbour's carry words, in the tensor-core word filters the
+ * hand-overs between loading, multiplying and reading warps; polls < 0
+ * restores the default (4,194,304).  With 0 every such wait gives up at once,
+ * so a call whose pairs need a multi-warp group or whose passes run such a
+ * filter returns GSDR_ETIMEOUT: the way tests check that a
  * wait that runs out ends in a status and not in a hang.  The reference has no
  * device-side waits (its errors are read once by checkError,
  * cuda-version/func.cu:1118-1123). */
