@@ -102,8 +102,11 @@ constexpr int64_t kIndexDensity = 8;
 // Buckets of the hashed k-mer counts for reads of up to max_len bases, or 0:
 // the tentative masks.  Two unrelated reads of L k-mers each reach a product
 // sum of about L^2 / H, close to a Poisson variable; the fewest buckets that
-// leave the word cutoff five deviations above it (150 bp reads at t = 0.90:
-// 1,536, where about one unrelated pair in 1e5 stays open).  Longer reads would
+// leave the word cutoff five deviations above it.  (Pairs of unrelated
+// 150 bp reads of uniform bases, t = 0.90, that stay open behind the composition
+// bound: 8.8e-3 with 1,024 buckets, 4.4e-4 with 1,280, 2.8e-5 with the rule's
+// 1,536; of 100 bp reads, where it takes 2,048 because their cutoff is lower,
+// 1.6e-4 with 1,536.  24 million pairs each, on the CPU.)  Longer reads would
 // need more buckets, each of which costs as much as any other, while the masks
 // cost by the k-mers a read has: 2,048 buckets at 1.0e12 pairs/s break even
 // with the masks at about 100 k-mers.

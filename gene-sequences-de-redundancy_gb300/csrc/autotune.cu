@@ -167,9 +167,9 @@ int store_tuned(const std::string& path, const std::string& gpu, const std::stri
         }
     }
     if (keep.empty())
-        keep.push_back("# gsdr tuning cache: gpu and kernel generation, bucket, batch, word_filter, group_words, "
-                       "band_serial, align_blocks, filter_blocks, graph_steps, us per "
-                       "representative");
+        keep.push_back("# gsdr tuning cache: gpu and kernel generation, bucket, batch, "
+                       "word_filter, group_words, band_serial, align_blocks, filter_blocks, "
+                       "graph_steps, us per representative");
     char row[512];
     const Knobs k = knobs_of(best);
     std::snprintf(row, sizeof(row), "%s\t%s\t%d\t%d\t%d\t%d\t%d\t%d\t%d\t%.3f", gpu.c_str(),
@@ -290,7 +290,7 @@ int autotune(const gsdr_reads* reads, const gsdr_opts* base_in, int reps, int ru
         t.stage = stage;
         run_trial(reads, t, reps, runs);
         // a form the job could not take (bitmaps above word length 7, masks
-        // for reads above 255 k-mers) is not a setting
+        // for reads above 1,023 k-mers) is not a setting
         if (t.ok && o.word_filter == 3 && t.word_index != 2) return;
         if (t.ok && o.word_filter == 4 && t.word_index != 3) return;
         trials.push_back(t);

@@ -321,7 +321,8 @@ __global__ void __launch_bounds__(kFilterThreads, 6) k_filter(DevReads R, RoundS
                 // D = shared k-mers (non-zero counts) bounds S: D <= S <= D + min(excesses)
                 bytes += 4ull * NBW;
                 const int q_extra = R.kextra[q];
-                const uint4 cb = __ldcs(reinterpret_cast<const uint4*>(R.kbits + (size_t)q * NBW) + lane % (NBW / 4));
+                const uint4 cb = __ldcs(
+                    reinterpret_cast<const uint4*>(R.kbits + (size_t)q * NBW) + lane % (NBW / 4));
                 int d = 0;
                 if (lane < NBW / 4) {
                     const uint4 rb = reinterpret_cast<const uint4*>(rbits)[lane];
@@ -2569,10 +2570,10 @@ __global__ void __launch_bounds__(1024, 1) k_bfilter_idx(
 //
 // 990k candidates x 1,024 tentatives, H = 1,536: 0.75 ms (1.35e12 pairs/s; the
 // masks 1.5 ms); 1M reads of 100-150 bp at t = 0.90 spent 127 ms in the filter
-// stage instead of 211, and 108 since k_bexact_d and hash_even_r.  An MMA (64 buckets) takes N / 2 cycles, and the MMAs alone
-// would take 0.36 ms; the MMA thread's wait for a stage adds about 200 cycles
-// that nothing covers (issuing blocks while the tensor pipe is busy), so a stage
-// holds eight MMAs.  On the way there, average of the first 249 passes (0.39
+// stage instead of 211, and 108 since k_bexact_d and hash_even_r.  An MMA (64
+// buckets) takes N / 2 cycles, and the MMAs alone would take 0.36 ms; the MMA
+// thread's wait for a stage adds about 200 cycles that nothing covers (issuing
+// blocks while the tensor pipe is busy), so a stage holds eight MMAs.  On the way there, average of the first 249 passes (0.39
 // ms as it is): 16 KB stages with eight warps on each 0.43 ms; an arrival per copying
 // thread 0.43; rows by TMA gathers of four 1.07 (67 cycles a gather); two warps
 // owning each 16 KB stage 0.41; the next stage's wait in the middle of the MMAs
@@ -3471,7 +3472,8 @@ void launch_bfilter_tab_t(const DevReads& R, RoundBuffers& B, const int32_t* rem
         cudaFuncSetAttribute(k_bfilter_tab<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         grid = grid_for(k_bfilter_tab<K>, kTabThreads, smem, 2);
     }
-    k_bfilter_tab<K><<<shaped(grid, R.filter_blocks), kTabThreads, smem, s>>>(R, B.st, remain, B.tent, B.pairs, B.seg_cap);
+    k_bfilter_tab<K><<<shaped(grid, R.filter_blocks), kTabThreads, smem, s>>>(
+        R, B.st, remain, B.tent, B.pairs, B.seg_cap);
 }
 
 template <int K, bool DROP>
@@ -3481,7 +3483,8 @@ void launch_bfilter_t(const DevReads& R, RoundBuffers& B, const int32_t* remain,
     } else {
         static int grid = 0;
         if (!grid) grid = grid_for(k_bprefilter, kFilterThreads, 0, 8);
-        launch_next(B, k_bprefilter, shaped(grid, R.filter_blocks), kFilterThreads, 0, s, R, B.st, remain, B.tent, B.pairs, B.seg_cap);
+        launch_next(B, k_bprefilter, shaped(grid, R.filter_blocks), kFilterThreads, 0, s, R, B.st,
+                    remain, B.tent, B.pairs, B.seg_cap);
     }
 }
 
@@ -3534,8 +3537,10 @@ void launch_exact_t(const DevReads& R, RoundBuffers& B, cudaStream_t s) {
     const int ga = num_sms() * 2;
     launch_next(B, k_amb_count, ga, kAmbThreads, 0, s, B.st, B.amb, B.amb_cap, B.tidx, B.amb_idx);
     launch_next(B, k_amb_scan, 1, 1024, 0, s, B.st, B.amb_cap, B.amb_idx);
-    launch_next(B, k_amb_place, ga, kAmbThreads, 0, s, B.st, B.amb, B.amb_cap, B.tidx, B.amb_idx, B.amb2);
-    launch_next(B, k_bexact_t<K>, shaped(grid, R.filter_blocks), kAmbThreads, xsmem, s,  R, B.st, B.amb2, B.amb_idx, B.amb_cap, B.tent, B.pairs, B.seg_cap);
+    launch_next(B, k_amb_place, ga, kAmbThreads, 0, s, B.st, B.amb, B.amb_cap, B.tidx, B.amb_idx,
+                B.amb2);
+    launch_next(B, k_bexact_t<K>, shaped(grid, R.filter_blocks), kAmbThreads, xsmem, s, R, B.st,
+                B.amb2, B.amb_idx, B.amb_cap, B.tent, B.pairs, B.seg_cap);
 }
 
 template <int K>
@@ -3550,7 +3555,8 @@ void launch_bfilter_bits_t(const DevReads& R, RoundBuffers& B, const int32_t* re
                              kBitsSmem);
         grid = grid_for(k_bfilter_bits<K>, kBitsThreads, kBitsSmem, 1);
     }
-    launch_next(B, k_bfilter_bits<K>, grid, kBitsThreads, kBitsSmem, s, R, B.st, remain, B.tent, B.pairs, B.seg_cap, B.amb, B.amb_cap);
+    launch_next(B, k_bfilter_bits<K>, grid, kBitsThreads, kBitsSmem, s, R, B.st, remain, B.tent,
+                B.pairs, B.seg_cap, B.amb, B.amb_cap);
     launch_exact_t<K>(R, B, s);
 }
 
@@ -3564,11 +3570,13 @@ void launch_bfilter_hash(const DevReads& R, RoundBuffers& B, const int32_t* rema
                              kDirectWarps * kDirectMaxSlots * (int)sizeof(uint32_t));
         attr = true;
     }
-    launch_next(B, k_bfilter_hash, num_sms(), kHashThreads, kHashSmem, s, R, B.st, remain, B.tent, B.amb, B.amb_cap);
+    launch_next(B, k_bfilter_hash, num_sms(), kHashThreads, kHashSmem, s, R, B.st, remain, B.tent,
+                B.amb, B.amb_cap);
     const int words = std::max(R.hslots, (1 << (2 * R.k)) / 32);  // as direct_words()
     const int smem = kDirectWarps * words * (int)sizeof(uint32_t);
     const int grid = num_sms() * std::min(8, 220 * 1024 / (smem + 1024));
-    launch_next(B, k_bexact_d, shaped(grid, R.filter_blocks), 32 * kDirectWarps, smem, s, R, B.st, B.amb, B.amb_cap, B.pairs, B.seg_cap);
+    launch_next(B, k_bexact_d, shaped(grid, R.filter_blocks), 32 * kDirectWarps, smem, s, R, B.st,
+                B.amb, B.amb_cap, B.pairs, B.seg_cap);
 }
 
 template <int K>
@@ -3605,7 +3613,8 @@ void launch_filter_any(const DevReads& R, RoundBuffers& B, const int32_t* remain
         static int grid = 0;
         if (!grid) grid = grid_for(k_filter_g, kFilterThreads, 0, 8);
         k_gtab<<<64, 256, 0, s>>>(R, B.st, 0);
-        k_filter_g<<<shaped(grid, R.filter_blocks), kFilterThreads, 0, s>>>(R, B.st, remain, B.pairs, B.seg_cap);
+        k_filter_g<<<shaped(grid, R.filter_blocks), kFilterThreads, 0, s>>>(
+            R, B.st, remain, B.pairs, B.seg_cap);
         k_gtab<<<64, 256, 0, s>>>(R, B.st, 1);
         return;
     }
@@ -3684,7 +3693,8 @@ void launch_align_t(const DevReads& R, RoundBuffers& B, int cls, cudaStream_t s)
                              smem);
         grid = grid_for(k_align<G, W, BATCH>, kAlignThreads, smem, 8);
     }
-    k_align<G, W, BATCH><<<shaped(grid, R.align_blocks), kAlignThreads, smem, s>>>(R, B.st, align_args(B), cls);
+    k_align<G, W, BATCH><<<shaped(grid, R.align_blocks), kAlignThreads, smem, s>>>(
+        R, B.st, align_args(B), cls);
 }
 
 template <bool BATCH, int MODE>
@@ -3696,14 +3706,16 @@ void launch_seg_t(const DevReads& R, RoundBuffers& B, cudaStream_t s) {
                              smem);
         grid = grid_for(k_seg<BATCH, MODE>, kAlignThreads, smem, 8);
     }
-    launch_next(B, k_seg<BATCH, MODE>, shaped(grid, R.align_blocks), kAlignThreads, smem, s, R, B.st, align_args(B));
+    launch_next(B, k_seg<BATCH, MODE>, shaped(grid, R.align_blocks), kAlignThreads, smem, s, R,
+                B.st, align_args(B));
 }
 
 template <bool BATCH>
 void launch_band_t(const DevReads& R, RoundBuffers& B, cudaStream_t s) {
     static int grid = 0;
     if (!grid) grid = grid_for(k_band<BATCH>, kAlignThreads, 0, 8);
-    launch_next(B, k_band<BATCH>, shaped(grid, R.align_blocks), kAlignThreads, 0, s, R, B.st, align_args(B));
+    launch_next(B, k_band<BATCH>, shaped(grid, R.align_blocks), kAlignThreads, 0, s, R, B.st,
+                align_args(B));
 }
 
 template <bool BATCH>
@@ -3807,11 +3819,13 @@ void launch_plain_round(const DevReads& R, RoundBuffers& B, int drop, int parity
     B.chained = ev4 == nullptr;
     if (ev4) cudaEventRecordWithFlags(ev4[0], s, cudaEventRecordExternal);
     launch_filter_any<false>(R, B, rin, drop, s);
-    if (R.pig_q && !drop) k_pigeon<false><<<num_sms() * 8, 256, 0, s>>>(R, B.st, B.pairs, B.seg_cap);
+    if (R.pig_q && !drop)
+        k_pigeon<false><<<num_sms() * 8, 256, 0, s>>>(R, B.st, B.pairs, B.seg_cap);
     if (ev4) cudaEventRecordWithFlags(ev4[1], s, cudaEventRecordExternal);
     launch_align_classes<false>(R, B, s);
     if (ev4) cudaEventRecordWithFlags(ev4[2], s, cudaEventRecordExternal);
-    launch_next(B, k_compact<false>, num_sms() * 4, 256, 0, s,  B.st, rin, rout, CompactArgs{B.cluster, align_work_of(B.st), nullptr, nullptr, 0, 0, 0, 0});
+    launch_next(B, k_compact<false>, num_sms() * 4, 256, 0, s, B.st, rin, rout,
+                CompactArgs{B.cluster, align_work_of(B.st), nullptr, nullptr, 0, 0, 0, 0});
     if (ev4) cudaEventRecordWithFlags(ev4[3], s, cudaEventRecordExternal);
     if (count)
         *count += 2 + align_launches<false>(R, B) + (R.pig_q && !drop ? 1 : 0) +
@@ -3835,7 +3849,8 @@ void launch_batch_pass(const DevReads& R, RoundBuffers& B, int drop, int parity,
     const int32_t* rin = B.remain[parity];
     int32_t* rout = B.remain[parity ^ 1];
     B.chained = ev4 == nullptr;
-    launch_next(B, k_bselect, 1, 1024, 0, s, B.st, B.cluster, R.n, B.tent, B.tidx, B.tt, B.ttrow, align_work_of(B.st));
+    launch_next(B, k_bselect, 1, 1024, 0, s, B.st, B.cluster, R.n, B.tent, B.tidx, B.tt, B.ttrow,
+                align_work_of(B.st));
     if (ev4) cudaEventRecordWithFlags(ev4[0], s, cudaEventRecordExternal);
     launch_filter_any<true>(R, B, rin, drop, s);
     if (R.pig_q && !drop) k_pigeon<true><<<num_sms() * 8, 256, 0, s>>>(R, B.st, B.pairs, B.seg_cap);
@@ -3843,8 +3858,11 @@ void launch_batch_pass(const DevReads& R, RoundBuffers& B, int drop, int parity,
     launch_align_classes<true>(R, B, s);
     if (ev4) cudaEventRecordWithFlags(ev4[2], s, cudaEventRecordExternal);
     const int r_even = B.r_auto && R.hbuckets && !drop ? hash_even_r(R.hbuckets, B.r_max) : 0;
-    launch_next(B, k_bclaim, num_sms(), kMaxBatch, 0, s, B.st, B.tent, B.tt, B.ttrow, B.acc, B.tidx, B.best, B.cluster);
-    launch_next(B, k_compact<true>, num_sms() * 4, 256, 0, s,  B.st, rin, rout, CompactArgs{B.cluster, align_work_of(B.st), B.best, B.tent, B.seg_cap, B.acc_cap, B.amb_cap, drop, r_even});
+    launch_next(B, k_bclaim, num_sms(), kMaxBatch, 0, s, B.st, B.tent, B.tt, B.ttrow, B.acc, B.tidx,
+                B.best, B.cluster);
+    launch_next(B, k_compact<true>, num_sms() * 4, 256, 0, s, B.st, rin, rout,
+                CompactArgs{B.cluster, align_work_of(B.st), B.best, B.tent, B.seg_cap, B.acc_cap,
+                            B.amb_cap, drop, r_even});
     if (ev4) cudaEventRecordWithFlags(ev4[3], s, cudaEventRecordExternal);
     if (count)
         *count += 4 + align_launches<true>(R, B) + (!drop ? 1 : 0) +

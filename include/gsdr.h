@@ -68,9 +68,10 @@ typedef struct {
                              takes; 0 = automatic (16,384), -1 = none (those pairs go to
                              the other alignment kernels); the result is the same */
     int32_t group_words;  /* window of the segment alignment kernel (a group of lanes per
-                             pair): the widest (32-bit words, 1..128) it takes; 0 =
-                             automatic (512), -1 = none (those pairs go to the systolic
-                             kernels); the result is the same */
+                             pair): 0 = automatic (all that fit: 512 32-bit words, 768 in
+                             its wide form), 1..128 = windows of at most that many words,
+                             -1 = none; the other pairs go to the systolic kernels; the
+                             result is the same */
     int32_t align_blocks; /* block shape: resident CTAs per SM the alignment kernels are
                              launched with (1..8, capped by what fits; 0 = automatic: as
                              many as fit); the result is the same */
