@@ -1595,6 +1595,14 @@ constexpr int kBitsSmem = 1024 + kBitsStages * kBitsStageBytes + kTentPad * (16 
 static_assert(128 % 8 == 0 && kTcMaxN % 16 == 0, "whole groups of eight rows");
 constexpr int kBitsRows = (128 + kTcMaxN + 4 * kBitsProducers - 1) / (4 * kBitsProducers);
 
+// A limit of 0 polls (set_spin_limit) asks the tensor-core filters to give up:
+// their stages then wait for one arrival more than there are, so that every
+// warp's waits run out at their first poll and no product is issued.  In the
+// waits themselves (a limit of 0 as it is, or a note of the first product) this
+// took 0.4 to 1.4% of the hashed filter's time.
+__device__ __forceinline__ int never_full() { return c_spin_limit <= 0 ? 1 : 0; }
+constexpr int kDrainLimit = 1 << 14;  // polls for the products in flight (microseconds)
+
 __device__ __forceinline__ uint2 comp_halves(const int4 c) {
     return make_uint2((uint32_t)min(c.x, 0xffff) | (uint32_t)min(c.y, 0xffff) << 16,
                       (uint32_t)min(c.z, 0xffff) | (uint32_t)min(c.w, 0xffff) << 16);
@@ -1643,7 +1651,7 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
     const int warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
         for (int i = 0; i < kBitsStages; i++) {
-            mbar_init(&full[i], kBitsProducers);
+            mbar_init(&full[i], kBitsProducers + never_full());
             mbar_init(&empty[i], 1);
         }
         for (int i = 0; i < 2; i++) {
@@ -1709,9 +1717,8 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const int limit = c_spin_limit;
-    bool ok = true;       // this warp's waits all ended
-    bool issued = false;  // this thread has MMAs in flight, or had
+    const int limit = max(c_spin_limit, 1);
+    bool ok = true;  // this warp's waits all ended
     if (warp == 0) {
         if (lane == 0) {
             const uint32_t idesc = tc_idesc_fp4(N);
@@ -1725,7 +1732,6 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
                     ok = mbar_wait(&full[s], ph, limit, &s_quit);
                     if (!ok) break;
                     tc_fence_after();
-                    issued = true;
                     const uint32_t a = tc_desc_lo(smem_u32(stage0 + s * kBitsStageBytes));
 #pragma unroll
                     for (int u = 0; u < 2; u++)
@@ -1946,11 +1952,11 @@ __global__ void __launch_bounds__(kBitsThreads, 1) k_bfilter_bits(
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
-        if (s_quit && issued) {
+        if (s_quit && lane == 0 && !never_full()) {
             // the MMAs in flight, before the accumulators are given back
             const int none = 0;
             tc_commit(&drain);
-            mbar_wait(&drain, 0, kSpinLimit, &none);
+            mbar_wait(&drain, 0, kDrainLimit, &none);
         }
         __syncwarp();
         tmem_free_all(tmem);
@@ -2573,11 +2579,12 @@ __global__ void __launch_bounds__(1024, 1) k_bfilter_idx(
 // stage instead of 211, and 108 since k_bexact_d and hash_even_r.  An MMA (64
 // buckets) takes N / 2 cycles, and the MMAs alone would take 0.36 ms; the MMA
 // thread's wait for a stage adds about 200 cycles that nothing covers (issuing
-// blocks while the tensor pipe is busy), so a stage holds eight MMAs.  On the way there, average of the first 249 passes (0.39
-// ms as it is): 16 KB stages with eight warps on each 0.43 ms; an arrival per copying
-// thread 0.43; rows by TMA gathers of four 1.07 (67 cycles a gather); two warps
-// owning each 16 KB stage 0.41; the next stage's wait in the middle of the MMAs
-// 0.43; one team of four on the sums 0.43.
+// blocks while the tensor pipe is busy), so a stage holds eight MMAs.  On the
+// way there, average of the first 249 passes (0.39 ms as it is): 16 KB stages
+// with eight warps on each 0.43 ms; an arrival per copying thread 0.43; rows by
+// TMA gathers of four 1.07 (67 cycles a gather); two warps owning each 16 KB
+// stage 0.41; the next stage's wait in the middle of the MMAs 0.43; one team of
+// four on the sums 0.43.
 constexpr int kHashEpilogue = 8;  // two teams of four, one per accumulator
 constexpr int kHashStages = 3;
 constexpr int kHashStepBuckets = 512;  // buckets per stage
@@ -2646,7 +2653,7 @@ __global__ void __launch_bounds__(kHashThreads, 1) k_bfilter_hash(
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int i = 0; i < kHashStages; i++) {
-            mbar_init(&full[i], kHashProducers / kHashStages);
+            mbar_init(&full[i], kHashProducers / kHashStages + never_full());
             mbar_init(&empty[i], 1);
         }
         for (int i = 0; i < 2; i++) {
@@ -2678,9 +2685,8 @@ __global__ void __launch_bounds__(kHashThreads, 1) k_bfilter_hash(
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const int limit = c_spin_limit;
-    bool ok = true;       // this warp's waits all ended
-    bool issued = false;  // this thread has MMAs in flight, or had
+    const int limit = max(c_spin_limit, 1);
+    bool ok = true;  // this warp's waits all ended
     if (warp == 0) {
         if (lane == 0) {
             const uint32_t idesc = tc_idesc_fp4(N);
@@ -2695,7 +2701,6 @@ __global__ void __launch_bounds__(kHashThreads, 1) k_bfilter_hash(
                     ok = mbar_wait(&full[s], ph, limit, &s_quit);
                     if (!ok) break;
                     tc_fence_after();
-                    issued = true;
                     const uint32_t a = a0 + s * (kHashStageBytes / 16);
                     const uint32_t b = b0 + 2 * c * N * (kTcRowBytes / 16);
                     tc_mma_stage(tmem + buf * kTcMaxN, tmem, a, b, idesc, c == 0);
@@ -2853,11 +2858,11 @@ __global__ void __launch_bounds__(kHashThreads, 1) k_bfilter_hash(
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
-        if (s_quit && issued) {
+        if (s_quit && lane == 0 && !never_full()) {
             // the MMAs in flight, before the accumulators are given back
             const int none = 0;
             tc_commit(&drain);
-            mbar_wait(&drain, 0, kSpinLimit, &none);
+            mbar_wait(&drain, 0, kDrainLimit, &none);
         }
         __syncwarp();
         tmem_free_all(tmem);
