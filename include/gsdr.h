@@ -333,8 +333,9 @@ int gsdr_server_wait(gsdr_server* s, int64_t timeout_ms, int64_t* job, int32_t* 
 int gsdr_server_result(gsdr_server* s, int64_t job, char* buf, int64_t cap, int64_t* need,
                        int32_t* cluster, int32_t* n_reads);
 /* Timing of a finished job: submission to the start of its run (the waits for a
- * slot and for room on the device) and the run itself (parse, sort, device work
- * and output formatting), host wall clock.  The sum of run_ms over jobs divided by the
+ * slot and for room on the device, and between them the count of the file's
+ * records that sizes it) and the run itself (parse, sort, device work and output
+ * formatting), host wall clock.  The sum of run_ms over jobs divided by the
  * stream's wall time is the number of jobs running at once on average. */
 int gsdr_server_times(gsdr_server* s, int64_t job, double* queued_ms, double* run_ms);
 int gsdr_server_release(gsdr_server* s, int64_t job);
