@@ -16,7 +16,6 @@
 #include <condition_variable>
 #include <cstdint>
 #include <mutex>
-#include <set>
 
 namespace gsdr {
 
@@ -28,17 +27,37 @@ struct Admission {
     int holding = 0;              // jobs past step 1
     int clustering = 0;           // jobs past step 2
     bool stopping = false;        // waiters give up
-    std::set<int64_t> waiting;    // tickets waiting at step 1
+
+    // Jobs waiting at step 1, one per slot at most: a list through the waiting
+    // calls' own frames, so that waiting needs no memory.
+    struct Waiter {
+        int64_t ticket;
+        Waiter* next;
+    };
+    Waiter* waiting = nullptr;
+
+    bool is_waiting(int64_t ticket) const {
+        for (const Waiter* w = waiting; w; w = w->next)
+            if (w->ticket == ticket) return true;
+        return false;
+    }
+    bool is_first(int64_t ticket) const {
+        for (const Waiter* w = waiting; w; w = w->next)
+            if (w->ticket < ticket) return false;
+        return true;
+    }
 
     // False when the server stops.
     bool parse(std::unique_lock<std::mutex>& lock, std::condition_variable& cv, int64_t ticket,
                int64_t bytes) {
-        waiting.insert(ticket);
+        Waiter me{ticket, waiting};
+        waiting = &me;
         cv.wait(lock, [&] {
-            return stopping || (*waiting.begin() == ticket &&
-                                (used + bytes <= budget || holding == 0));
+            return stopping || (is_first(ticket) && (used + bytes <= budget || holding == 0));
         });
-        waiting.erase(ticket);
+        Waiter** at = &waiting;
+        while (*at != &me) at = &(*at)->next;
+        *at = me.next;
         cv.notify_all();  // the next ticket may fit as well
         if (stopping) return false;
         used += bytes;

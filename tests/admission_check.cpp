@@ -34,9 +34,10 @@ struct Bench {
             state[ticket] = ok ? 1 : -1;
             cv.notify_all();
         });
+        // (a job that begins to wait notifies nobody)
         std::unique_lock<std::mutex> lock(mu);
-        cv.wait_for(lock, std::chrono::seconds(10),
-                    [&] { return state.count(ticket) || a.waiting.count(ticket); });
+        for (int i = 0; i < 10000 && !state.count(ticket) && !a.is_waiting(ticket); i++)
+            cv.wait_for(lock, std::chrono::milliseconds(1));
     }
     void leave(int64_t bytes) {
         std::lock_guard<std::mutex> lock(mu);
